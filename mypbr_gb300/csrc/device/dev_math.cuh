@@ -38,6 +38,13 @@ MYPBR_HD float3 cross(float3 a, float3 b) {
 MYPBR_HD float len2(float3 a) { return dot(a, a); }
 MYPBR_DEV float length(float3 a) { return sqrtf(dot(a, a)); }
 MYPBR_DEV float3 normalize(float3 a) { return a * rsqrtf(dot(a, a)); }
+// Sums of two products leave the compiler a choice of which product to fuse,
+// and it takes it by the code around: these fix the order where a last bit
+// decides (x first, or y first).
+MYPBR_DEV float dot_x(float3 a, float3 b) { return fmaf(a.z, b.z, fmaf(a.x, b.x, a.y * b.y)); }
+MYPBR_DEV float dot_y(float3 a, float3 b) { return fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x)); }
+MYPBR_DEV float3 normalize_x(float3 a) { return a * rsqrtf(dot_x(a, a)); }
+MYPBR_DEV float3 normalize_y(float3 a) { return a * rsqrtf(dot_y(a, a)); }
 MYPBR_HD float comp(float3 a, int i) { return i == 0 ? a.x : (i == 1 ? a.y : a.z); }
 MYPBR_HD float comp4(float4 a, int i) { return i == 0 ? a.x : (i == 1 ? a.y : (i == 2 ? a.z : a.w)); }
 MYPBR_HD void set_comp(float3& a, int i, float v) {

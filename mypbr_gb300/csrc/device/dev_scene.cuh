@@ -1347,9 +1347,13 @@ MYPBR_DEV float spawn_tmin(float3 o, float3 d) {
     return m * 9.5367431640625e-7f * rsqrtf(dot(d, d));
 }
 
-// Where a ray leaving surface s in direction w starts.
+// Where a ray leaving surface s in direction w starts. Y_FIRST: which product
+// of the offset's length is fused (in one case in 10^5 the origin's last bit
+// depends on it; feature guides and guided renders have always taken the other
+// one, and a render's paths stay the same to the last bit).
+template <bool Y_FIRST = true>
 MYPBR_DEV float3 spawn_origin(const Surface& s, float3 w) {
-    float dist = fabsf(s.ng.x) * s.perr.x + fabsf(s.ng.y) * s.perr.y + fabsf(s.ng.z) * s.perr.z;
+    float dist = Y_FIRST ? dot_y(abs3(s.ng), s.perr) : dot_x(abs3(s.ng), s.perr);
     float3 off = dist * s.ng;
     if (dot(w, s.ng) < 0.0f)
         off = -1.0f * off;

@@ -306,9 +306,10 @@ struct Lobe {
     float3 n;   // frame axis
     float3 wo;  // GGX / glass: wo in the local frame
     float alpha, eta;
-    MYPBR_DEV float value(float3 dir) const {
+    // unit: dir normalised (callers have it at hand)
+    MYPBR_DEV float value(float3 dir, float3 unit) const {
         if (kind == kLobeCosine)
-            return fmaxf(0.0f, dot(normalize(dir), normalize(n)) * kInvPi);
+            return fmaxf(0.0f, dot(unit, normalize(n)) * kInvPi);
         if (kind == kLobeGgx) {
             if (dot(dir, dir) == 0.0f)
                 return 0.0f;
@@ -326,7 +327,7 @@ struct Lobe {
             return p;
         }
         float g = alpha;
-        float c = dot(normalize(dir), normalize(n));
+        float c = dot(unit, normalize(n));
         float den = 1.0f + g * g - 2.0f * g * c;
         return (1.0f - g * g) / (4.0f * kPi * den * sqrtf(den));
     }
@@ -393,12 +394,12 @@ struct Pdf {
     float prob[3];
     // Loops with a constant trip count and static indices keep the lobes in
     // registers (a dynamically indexed array would live in local memory).
-    MYPBR_DEV float value(float3 dir) const {
+    MYPBR_DEV float value(float3 dir, float3 unit) const {
         float s = 0.0f;
 #pragma unroll
         for (int k = 0; k < 3; k++)
             if (k < n && prob[k] > 0.0f)
-                s += prob[k] * lobe[k].value(dir);
+                s += prob[k] * lobe[k].value(dir, unit);
         return s;
     }
     MYPBR_DEV float3 generate(Rng& g) const {
@@ -520,16 +521,55 @@ MYPBR_DEV float3 base_eval(const DeviceScene& S, const DevMaterial& m, const Pri
     return spec + ((1.0f - a.metallic) * tr * wi.z * kInvPi) * a.base;
 }
 
+// What a material's textures and normal maps give at one vertex. A vertex
+// scatters once and is evaluated towards two directions (the light sample and
+// the scattered ray); each class kernel looks the textures up once for all
+// three. (On the 2 M-triangle room's principled kernel the nine lookups, loops
+// over wrapper chains, took the larger part of its instructions.)
+template <int TYPE>
+struct MatPoint {};
+template <>
+struct MatPoint<kLambertian> {
+    float3 albedo;
+};
+template <>
+struct MatPoint<kPrincipled> {
+    PrincipledAt at;
+    float3 nb, nc;  // the base's and (with a coat) the coat's normal
+};
+template <int TYPE>
+MYPBR_DEV MatPoint<TYPE> mat_point(const DeviceScene& S, const DevMaterial& m, float3 r_dir, const Surface& rec) {
+    MatPoint<TYPE> pt;
+    if constexpr (TYPE == kLambertian) {
+        pt.albedo = tex_value(S, m.tex[0], rec.u, rec.v, rec.p);
+    } else if constexpr (TYPE == kPrincipled) {
+        pt.at = principled_at(S, m, rec);
+        pt.nb = m.tex[3] >= 0 ? normal_from_map(S, r_dir, rec, m.tex[3]) : rec.normal;
+        pt.nc = pt.at.coat > 0.0f && m.tex[6] >= 0 ? normal_from_map(S, r_dir, rec, m.tex[6]) : rec.normal;
+    }
+    return pt;
+}
+// The point of type TYPE inside scatter_inner / eval_inner<ONLY>: the caller's
+// when the type is fixed, else looked up here.
+template <int ONLY, int TYPE>
+MYPBR_DEV MatPoint<TYPE> mat_point_for(const DeviceScene& S, const DevMaterial& m, float3 r_dir, const Surface& rec,
+                                       const MatPoint<ONLY>& given) {
+    if constexpr (ONLY == TYPE)
+        return given;
+    else
+        return mat_point<TYPE>(S, m, r_dir, rec);
+}
+
 // scatter() of the material itself (no normal-map wrapper). ONLY >= 0 names
 // the material type at compile time, which leaves only that case in the code.
 template <int ONLY = -1>
 MYPBR_DEV bool scatter_inner(const DeviceScene& S, const DevMaterial& m, float3 r_dir, const Surface& rec,
-                             ScatterRec& sr, Rng& g) {
+                             ScatterRec& sr, Rng& g, const MatPoint<ONLY>& given = {}) {
     sr.skip_pdf = false;
     sr.pdf.n = 0;
     switch (ONLY >= 0 ? ONLY : m.type) {
         case kLambertian:  // material.h:79-85
-            sr.attenuation = tex_value(S, m.tex[0], rec.u, rec.v, rec.p);
+            sr.attenuation = mat_point_for<ONLY, kLambertian>(S, m, r_dir, rec, given).albedo;
             sr.pdf.n = 1;
             sr.pdf.lobe[0] = cosine_lobe(rec.normal);
             sr.pdf.prob[0] = 1.0f;
@@ -602,9 +642,10 @@ MYPBR_DEV bool scatter_inner(const DeviceScene& S, const DevMaterial& m, float3 
             return true;
         }
         case kPrincipled: {  // material.h:387-421
-            PrincipledAt a = principled_at(S, m, rec);
+            const MatPoint<kPrincipled> pt = mat_point_for<ONLY, kPrincipled>(S, m, r_dir, rec, given);
+            const PrincipledAt& a = pt.at;
+            const float3 nb = pt.nb;
             float3 wo = normalize(-r_dir);
-            float3 nb = m.tex[3] >= 0 ? normal_from_map(S, r_dir, rec, m.tex[3]) : rec.normal;
             float co = fmaxf(0.0f, dot(nb, wo));
             float sw = avg3(spec_fresnel(m, co, a.base, a.metallic));
             float dw = (1.0f - a.metallic) * avg3(a.base) * (1.0f - schlick(co, m.p[0]));
@@ -613,7 +654,7 @@ MYPBR_DEV bool scatter_inner(const DeviceScene& S, const DevMaterial& m, float3 
             ps = clampf(ps, 0.1f, 1.0f);
             sr.attenuation = a.base;
             if (a.coat > 0.0f) {
-                float3 nc = m.tex[6] >= 0 ? normal_from_map(S, r_dir, rec, m.tex[6]) : rec.normal;
+                const float3 nc = pt.nc;
                 float cw = a.coat * schlick(dot(nc, wo), 0.04f);
                 float below = (1.0f - cw) * (sw + dw) * avg3(coat_transmittance(m, a.coat, 1.0f, 1.0f));
                 float pc = clampf(cw / (cw + below), 0.1f, 0.9f);
@@ -652,11 +693,12 @@ MYPBR_DEV bool scatter_inner(const DeviceScene& S, const DevMaterial& m, float3 
 }
 
 template <int ONLY = -1>
-MYPBR_DEV float3 eval_inner(const DeviceScene& S, const DevMaterial& m, float3 r_dir, const Surface& rec, float3 dir) {
+MYPBR_DEV float3 eval_inner(const DeviceScene& S, const DevMaterial& m, float3 r_dir, const Surface& rec, float3 dir,
+                            float3 unit, const MatPoint<ONLY>& given = {}) {
     switch (ONLY >= 0 ? ONLY : m.type) {
         case kLambertian: {  // material.h:88-97
-            float c = dot(rec.normal, normalize(dir));
-            return tex_value(S, m.tex[0], rec.u, rec.v, rec.p) * (c < 0.0f ? 0.0f : c * kInvPi);
+            float c = dot(rec.normal, unit);
+            return mat_point_for<ONLY, kLambertian>(S, m, r_dir, rec, given).albedo * (c < 0.0f ? 0.0f : c * kInvPi);
         }
         case kMetal: {  // material.h:154-164
             float alpha = rough_to_alpha(m.p[3]);
@@ -684,13 +726,14 @@ MYPBR_DEV float3 eval_inner(const DeviceScene& S, const DevMaterial& m, float3 r
         case kPrincipled: {  // material.h:423-453
             if (dot(dir, rec.normal) <= 0.0f)
                 return f3(0.0f);
-            PrincipledAt a = principled_at(S, m, rec);
-            float3 wo = normalize(-r_dir), wi = normalize(dir);
-            float3 nb = m.tex[3] >= 0 ? normal_from_map(S, r_dir, rec, m.tex[3]) : rec.normal;
+            const MatPoint<kPrincipled> pt = mat_point_for<ONLY, kPrincipled>(S, m, r_dir, rec, given);
+            const PrincipledAt& a = pt.at;
+            const float3 nb = pt.nb;
+            float3 wo = normalize(-r_dir), wi = unit;
             float3 below = base_eval(S, m, a, nb, wo, wi);
             if (a.coat <= 0.0f)
                 return below;
-            float3 nc = m.tex[6] >= 0 ? normal_from_map(S, r_dir, rec, m.tex[6]) : rec.normal;
+            const float3 nc = pt.nc;
             float co = dot(nc, wo), ci = dot(nc, wi);
             float through = (1.0f - a.coat * schlick(co, 0.04f)) * (1.0f - a.coat * schlick(ci, 0.04f));
             float3 result = through * coat_transmittance(m, a.coat, co, ci) * below;
@@ -706,7 +749,7 @@ MYPBR_DEV float3 eval_inner(const DeviceScene& S, const DevMaterial& m, float3 r
             return result;
         }
         case kPhase: {  // medium.h:265-269
-            float c = dot(normalize(r_dir), normalize(dir)), g = m.p[3];
+            float c = dot(normalize(r_dir), unit), g = m.p[3];
             float den = 1.0f + g * g - 2.0f * g * c;
             return mat_vec(m, 0) * ((1.0f - g * g) / (4.0f * kPi * den * sqrtf(den)));
         }
@@ -732,15 +775,15 @@ MYPBR_DEV bool scatter(const DeviceScene& S, int mi, float3 r_dir, const Surface
     return true;
 }
 
-MYPBR_DEV float3 eval(const DeviceScene& S, int mi, float3 r_dir, const Surface& rec, float3 dir) {
+MYPBR_DEV float3 eval(const DeviceScene& S, int mi, float3 r_dir, const Surface& rec, float3 dir, float3 unit) {
     const DevMaterial& m = S.materials[mi];
     if (m.normal_map < 0 || m.type == kPrincipled)
-        return eval_inner(S, m, r_dir, rec, dir);
+        return eval_inner(S, m, r_dir, rec, dir, unit);
     if (dot(dir, rec.normal) <= 0.0f)
         return f3(0.0f);
     Surface sh = rec;
     sh.normal = normal_from_map(S, r_dir, rec, m.normal_map);
-    return eval_inner(S, m, r_dir, sh, dir);
+    return eval_inner(S, m, r_dir, sh, dir, unit);
 }
 
 // material.h:578-598 (diffuse_light) and :731-736 (emissive_surface)
@@ -784,7 +827,8 @@ MYPBR_DEV bool is_volume(const DeviceScene& S, int mi) { return S.materials[mi].
 MYPBR_DEV void env_angles(const DeviceScene& S, float3 dir, float& u, float& theta) {
     float3 d = normalize(dir);
     theta = acosf(clampf(d.y, -1.0f, 1.0f));
-    u = 0.5f + atan2f(d.x, -d.z) * (0.5f * kInvPi) + S.env_rotation;
+    // fused by hand: left to the compiler, whether it fuses depends on the code around
+    u = fmaf(atan2f(d.x, -d.z), 0.5f * kInvPi, 0.5f) + S.env_rotation;
     u -= floorf(u);
 }
 

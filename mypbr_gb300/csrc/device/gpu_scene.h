@@ -14,24 +14,25 @@ namespace mypbr_dev {
 
 struct BatchGraphCache;  // render.cu
 
-// Scratch memory of one render: path state in slots, queues of slot indices,
-// the FP64 film. Kept on the scene handle and grown on demand.
+// Scratch memory of one render: path records in queue order, the FP64 film.
+// Kept on the scene handle and grown on demand.
+//
+// A path's record moves with it: bounce d reads it at the path's place in
+// extension queue d (buffer d & 1) and writes it at its place in queue d + 1,
+// so every kernel reads neighbouring records, whatever paths have ended. An
+// entry's ray and throughput are dead once it is shaded; its shadow ray takes
+// their place.
 struct RenderBuffers {
-    size_t capacity = 0;   // path slots
+    size_t capacity = 0;   // paths of a wave
     size_t pixels = 0;     // film pixels
     int depth_slots = 0;   // per-bounce queue counters
-    // path state (slot-indexed, 64 B)
-    float4* ray_o = nullptr;     // origin, path flags (bits)
-    float4* ray_d = nullptr;     // direction, scatter pdf of the direction
-    float4* beta = nullptr;      // throughput, pass (bits)
-    float4* radiance = nullptr;  // path radiance so far, pixel (bits)
-    float4* hit = nullptr;       // t, b1, b2, prim (bits)
-    float4* sh_o = nullptr;      // shadow ray: origin, -
-    float4* sh_d = nullptr;      // direction, final flag
-    float4* sh_c = nullptr;      // contribution rgb, -
-    uint32_t* queue[2] = {nullptr, nullptr};  // extension queues (ping-pong)
-    uint32_t* class_queue = nullptr;          // one queue per shading class, capacity each
-    uint32_t* shadow_queue = nullptr;
+    float4* ray[2] = {nullptr, nullptr};    // 2 per entry: (origin, flags), (direction, scatter pdf)
+    float4* state[2] = {nullptr, nullptr};  // 2 per entry: (throughput, slot), (radiance so far, -)
+    float4* hit = nullptr;                  // per entry: t, b1, b2, prim (bits)
+    uint8_t* cls = nullptr;                 // per entry: shading class of the hit
+    uint32_t* class_queue = nullptr;        // entries by shading class, two classes to an array of `capacity`
+    uint2* shadow_queue = nullptr;          // (entry holding the shadow ray, where its light goes)
+    float4* out = nullptr;                  // per slot: radiance of the ended path
     uint32_t* counters = nullptr;
     int* wave_state = nullptr;   // (first pass, passes) of the wave a captured graph replays; null: kernel arguments
     // film (pixel-indexed, FP64 sums)
@@ -73,7 +74,7 @@ struct GuideState {
     // recording buffers (slot-indexed, grown with the render buffers)
     GuideRecords rec{};
     size_t rec_slots = 0;
-    __half* packed = nullptr;        // per slot: the vertex's decoded mixture (GuidePacked)
+    __half* packed = nullptr;        // per queue entry: the vertex's decoded mixture (GuidePacked)
     size_t packed_slots = 0;
 };
 

@@ -54,14 +54,14 @@ __global__ void k_bsdf(DeviceScene S, int material, const float* rec, const floa
         s.material = material;
         float3 d = f3(r_in[3 * k], r_in[3 * k + 1], r_in[3 * k + 2]);
         float3 w = f3(wi[3 * k], wi[3 * k + 1], wi[3 * k + 2]);
-        float3 e = eval(S, material, d, s, w);
+        float3 e = eval(S, material, d, s, w, normalize(w));
         Rng g = make_rng(1, uint64_t(k), 0);
         ScatterRec sr;
         bool sc = scatter(S, material, d, s, sr, g);
         out[4 * k] = e.x;
         out[4 * k + 1] = e.y;
         out[4 * k + 2] = e.z;
-        out[4 * k + 3] = (sc && !sr.skip_pdf) ? sr.pdf.value(w) : 0.0f;
+        out[4 * k + 3] = (sc && !sr.skip_pdf) ? sr.pdf.value(w, normalize(w)) : 0.0f;
     }
 }
 

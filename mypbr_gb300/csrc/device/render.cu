@@ -1,17 +1,20 @@
 // The wavefront path tracer: camera::render / ray_color of the reference
 // (include/camera.h:79-461) as kernels over queues in HBM.
 //
-// A wave holds every pixel times `npass` passes, one path per slot. Each
-// bounce runs three kernels:
+// A wave holds every pixel times `npass` passes, one path per slot; the passes
+// of a pixel are neighbours, so a warp's camera rays start alike. Each bounce
+// runs three kinds of kernels:
 //   extend  closest hit of every ray in the extension queue (BVH walk);
 //   shade   per path: sky or emission with MIS, Beer-Lambert, scatter();
 //           for non-specular vertices next-event estimation writes a shadow
-//           ray into the shadow queue; the BSDF sample, Russian roulette, and
-//           the surviving path goes to the next extension queue;
-//   shadow  closest hit of every shadow ray; adds f L w / pdf to its path and,
-//           for a path that ended at this bounce, writes it to the film.
-// Queues hold slot indices and are appended with warp-aggregated atomics; the
-// per-bounce counters live in device memory, so the host never waits on them.
+//           ray; the BSDF sample, Russian roulette, and the surviving path
+//           goes to the next extension queue;
+//   shadow  closest hit of every shadow ray; adds f L w / pdf to its path.
+// A path that ends leaves its radiance in its slot; once the wave is done one
+// kernel sums every pixel's slots into the FP64 film.
+// Path records move through the queues (RenderBuffers) and are appended with one
+// atomic per warp; the per-bounce counters live in device memory, so the host
+// never waits on them.
 // Kernels are persistent-style (grid = SMs x resident blocks, grid-stride over
 // the queue length they read on the device).
 #include <algorithm>
@@ -34,6 +37,10 @@ namespace mypbr_dev {
 // shadow ray, then the diffuse / specular / scatter bounce counts (8 bits each).
 constexpr uint32_t kFlagSpecular = 1u;
 constexpr uint32_t kFlagSeen = 2u;
+
+// A shadow ray's light goes to an entry of the next extension queue, or, with
+// this bit, to the slot of a path that ended (a wave has at most 2^30 slots).
+constexpr uint32_t kShadowEnds = 0x80000000u;
 
 // Shading classes: each has its own queue and kernel, so a warp shades one
 // kind of material and each kernel carries only that material's code.
@@ -59,29 +66,53 @@ struct WaveParams {
     int pass0, npass;
     int first_row, band_rows;  // the rows rendered: [first_row, first_row + band_rows)
     unsigned long long* totals;  // extension rays, shadow rays, bounces run by a replayed wave graph
+    int moments;                 // sum squares too (the per-channel variance was asked for)
     // path guiding
     int guided;                // mixtures were computed for this wave's guidable vertices
     float guide_alpha;         // probability of sampling the mixture there (one-sample MIS), first bounce
     float guide_alpha_deep;    // the same at later bounces
     int guide_depths;          // bounces below this sample the mixture
     int record;                // write training records
-    GuideRecords rec;          // slots below rec_slots record their first rec.depth vertices
-    uint32_t rec_slots;
-    GuidePacked* guide_mix;    // per slot
+    GuideRecords rec;          // the first rec_passes paths of a pixel record their first rec.depth vertices
+    int rec_passes;
+    GuidePacked* guide_mix;    // per queue entry
     float3 guide_lo, guide_inv;
 };
 
 // Counters: extension queue length entering bounce d; shadow queue length of
-// bounce d; length of shading class c's queue at bounce d.
+// bounce d; rays of the extension queue handed out so far (the persistent
+// extend kernel); length of shading class c's queue at bounce d.
 MYPBR_DEV uint32_t* ext_counter(const WaveParams& P, int d) { return P.B.counters + d; }
 MYPBR_DEV uint32_t* sh_counter(const WaveParams& P, int d) { return P.B.counters + P.B.depth_slots + d; }
+MYPBR_DEV uint32_t* fetch_counter(const WaveParams& P, int d) { return P.B.counters + 2 * P.B.depth_slots + d; }
 MYPBR_DEV uint32_t* class_counter(const WaveParams& P, int d, int c) {
-    return P.B.counters + 2 * P.B.depth_slots + d * kShadeClasses + c;
+    return P.B.counters + 3 * P.B.depth_slots + d * kShadeClasses + c;
 }
-MYPBR_DEV uint32_t* class_queue(const WaveParams& P, int c) { return P.B.class_queue + size_t(c) * P.B.capacity; }
-// Rays of bounce d's extension queue handed out so far (the persistent extend kernel).
-MYPBR_DEV uint32_t* fetch_counter(const WaveParams& P, int d) {
-    return P.B.counters + (2 + kShadeClasses) * P.B.depth_slots + d;
+constexpr int kCounterRows = 3 + kShadeClasses;
+// Place i of class c's queue: two classes share an array, one from its front,
+// the other from its back (together they hold a wave's paths at most).
+MYPBR_DEV uint32_t* class_entry(const WaveParams& P, int c, uint32_t i) {
+    return P.B.class_queue + size_t(c >> 1) * P.B.capacity + ((c & 1) ? uint32_t(P.B.capacity) - 1 - i : i);
+}
+
+// 32-byte records, one 256-bit access each (a sector of L2, so that a gather
+// of records wastes none of what it fetches).
+struct Pair {
+    float4 a, b;
+};
+MYPBR_DEV Pair load_pair(const float4* base, uint32_t k) {
+    Pair p;
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(p.a.x), "=f"(p.a.y), "=f"(p.a.z), "=f"(p.a.w), "=f"(p.b.x), "=f"(p.b.y), "=f"(p.b.z),
+                   "=f"(p.b.w)
+                 : "l"(base + 2 * size_t(k))
+                 : "memory");
+    return p;
+}
+MYPBR_DEV void store_pair(float4* base, uint32_t k, float4 a, float4 b) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(base + 2 * size_t(k)), "f"(a.x),
+                 "f"(a.y), "f"(a.z), "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+                 : "memory");
 }
 
 // One atomic per warp: the active lanes that push get consecutive slots.
@@ -94,37 +125,6 @@ MYPBR_DEV uint32_t warp_push(uint32_t* counter) {
         base = atomicAdd(counter, uint32_t(__popc(mask)));
     base = __shfl_sync(mask, base, leader);
     return base + uint32_t(__popc(mask & ((1u << lane) - 1u)));
-}
-
-// The same for lanes pushing to different counters: one atomic per distinct counter.
-MYPBR_DEV uint32_t warp_push_keyed(uint32_t* counter) {
-    unsigned mask = __activemask();
-    unsigned peers = __match_any_sync(mask, reinterpret_cast<unsigned long long>(counter));
-    int lane = threadIdx.x & 31;
-    int leader = __ffs(peers) - 1;
-    uint32_t base = 0;
-    if (lane == leader)
-        base = atomicAdd(counter, uint32_t(__popc(peers)));
-    base = __shfl_sync(peers, base, leader);
-    return base + uint32_t(__popc(peers & ((1u << lane) - 1u)));
-}
-
-MYPBR_DEV void film_add(const WaveParams& P, uint32_t pixel, float3 c) {
-    // NaN or infinite estimates count as black (camera.h:281-287)
-    if (!isfinite(c.x) || !isfinite(c.y) || !isfinite(c.z))
-        c = f3(0.0f);
-    double* f = P.B.film + 3 * size_t(pixel);
-    double* f2 = P.B.film2 + 3 * size_t(pixel);
-    atomicAdd(f, double(c.x));
-    atomicAdd(f + 1, double(c.y));
-    atomicAdd(f + 2, double(c.z));
-    atomicAdd(f2, double(c.x) * c.x);
-    atomicAdd(f2 + 1, double(c.y) * c.y);
-    atomicAdd(f2 + 2, double(c.z) * c.z);
-    if (P.collect_features) {
-        double l = luminance(c);
-        atomicAdd(P.B.feat + 7 * size_t(pixel) + 6, l * l);
-    }
 }
 
 // Keys of the random numbers: everything random in a path depends only on
@@ -193,6 +193,26 @@ MYPBR_DEV int2 wave_of(const WaveParams& P) {
 // counter in device memory.
 MYPBR_DEV int bounce_of(const WaveParams& P, int depth) { return depth >= 0 ? depth : P.B.wave_state[2]; }
 
+// A slot's pixel (of the whole image) and pass: the passes of one pixel are
+// neighbouring slots.
+struct SlotPath {
+    uint32_t pixel, pass, band_pixel, band_pass;
+};
+MYPBR_DEV SlotPath slot_path(const WaveParams& P, int2 wave, uint32_t slot) {
+    SlotPath s;
+    const uint32_t passes = uint32_t(wave.y);
+    s.band_pixel = slot / passes;
+    s.band_pass = slot - s.band_pixel * passes;
+    s.pixel = uint32_t(P.first_row) * uint32_t(P.cam.width) + s.band_pixel;
+    s.pass = uint32_t(wave.x) + s.band_pass;
+    return s;
+}
+// The slot of entry k of bounce `depth`'s queue. Camera rays lie in slot
+// order and have no throughput record yet.
+MYPBR_DEV uint32_t entry_slot(const WaveParams& P, int depth, uint32_t k) {
+    return depth == 0 ? k : f_bits(P.B.state[depth & 1][2 * size_t(k)].w);
+}
+
 __global__ void k_set_wave(int* state, int pass0, int npass) {
     state[0] = pass0;
     state[1] = npass;
@@ -257,6 +277,12 @@ __global__ void k_job_step(WaveParams P, cudaGraphConditionalHandle loop, int pe
             P.B.counters[k] = 0;
 }
 
+// Whether this bounce is its wave's last one (a job's device-side loop).
+MYPBR_DEV bool wave_ending(const WaveParams& P) {
+    const int next = P.B.wave_state[2] + 1;
+    return !(next < P.max_depth && *ext_counter(P, next) > 0);
+}
+
 // gated: only when the wave state says a wave starts (a job's device-side
 // loop in a batch graph runs this kernel every iteration).
 MYPBR_DEV bool wave_starting(const WaveParams& P, int gated) { return !gated || P.B.wave_state[3] != 0; }
@@ -265,37 +291,33 @@ __global__ void k_generate(WaveParams P, int gated) {
     if (!wave_starting(P, gated))
         return;
     const int2 wv = wave_of(P);
-    size_t npix = size_t(P.cam.width) * P.band_rows;
-    size_t n = npix * size_t(wv.y);
-    size_t stride = size_t(gridDim.x) * blockDim.x;
-    size_t first_pixel = size_t(P.first_row) * P.cam.width;
-    for (size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x; t < n; t += stride) {
-        uint32_t pixel = uint32_t(first_pixel + t % npix);
-        uint32_t pass = uint32_t(wv.x + int(t / npix));
-        int i = int(pixel % uint32_t(P.cam.width)), j = int(pixel / uint32_t(P.cam.width));
-        Rng g = make_rng(P.seed, pixel, pass);
+    const uint32_t n = uint32_t(P.cam.width) * uint32_t(P.band_rows) * uint32_t(wv.y);  // at most 2^30
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += stride) {
+        const SlotPath sp = slot_path(P, wv, t);
+        int i = int(sp.pixel % uint32_t(P.cam.width)), j = int(sp.pixel / uint32_t(P.cam.width));
+        Rng g = make_rng(P.seed, sp.pixel, sp.pass);
         float3 o, d;
-        camera_ray(P.cam, i, j, int(pass), g, o, d);
-        P.B.ray_o[t] = make_float4(o.x, o.y, o.z, bits_f(kFlagSpecular));
-        P.B.ray_d[t] = make_float4(d.x, d.y, d.z, 0.0f);
-        P.B.beta[t] = make_float4(1.0f, 1.0f, 1.0f, bits_f(pass));
-        P.B.radiance[t] = make_float4(0.0f, 0.0f, 0.0f, bits_f(pixel));
-        P.B.queue[0][t] = uint32_t(t);
+        camera_ray(P.cam, i, j, int(sp.pass), g, o, d);
+        store_pair(P.B.ray[0], t, make_float4(o.x, o.y, o.z, bits_f(kFlagSpecular)),
+                   make_float4(d.x, d.y, d.z, 0.0f));
     }
     if (blockIdx.x == 0 && threadIdx.x == 0)
-        *ext_counter(P, 0) = uint32_t(n);
+        *ext_counter(P, 0) = n;
 }
 
 // camera.h:253-277: albedo and normal of the first non-specular surface
 __global__ void k_features(WaveParams P, int gated) {
     if (!wave_starting(P, gated))
         return;
-    size_t n = size_t(P.cam.width) * P.band_rows * size_t(wave_of(P).y);
-    size_t stride = size_t(gridDim.x) * blockDim.x;
-    for (size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x; t < n; t += stride) {
-        float4 ro = P.B.ray_o[t], rd = P.B.ray_d[t];
-        uint32_t pixel = f_bits(P.B.radiance[t].w), pass = f_bits(P.B.beta[t].w);
-        float3 o = f3(ro), d = f3(rd);
+    const int2 wv = wave_of(P);
+    const uint32_t n = uint32_t(P.cam.width) * uint32_t(P.band_rows) * uint32_t(wv.y);
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += stride) {
+        const Pair ray = load_pair(P.B.ray[0], t);
+        const SlotPath path = slot_path(P, wv, t);
+        const uint32_t pixel = path.pixel, pass = path.pass;
+        float3 o = f3(ray.a), d = f3(ray.b);
         Rng g = make_rng(P.seed ^ 0x5bd1e995ull, pixel, pass);
         float3 tint = f3(1.0f), albedo = f3(1.0f), normal = f3(0.0f);
         bool done = false;
@@ -317,7 +339,7 @@ __global__ void k_features(WaveParams P, int gated) {
             } else {
                 tint *= sr.attenuation;
                 d = sr.skip_dir;
-                o = spawn_origin(s, d);
+                o = spawn_origin<false>(s, d);
             }
         }
         if (!done) {
@@ -347,28 +369,33 @@ MYPBR_DEV int hit_material(const DeviceScene& S, const HitInfo& h) {
     }
 }
 
-// Closest hits of the extension queue; each ray then joins its shading class's queue.
+// The hit of entry k and the shading class it gives its path.
+MYPBR_DEV void put_hit(const WaveParams& P, uint32_t k, const HitInfo& h) {
+    P.B.hit[k] = make_float4(h.t, h.b1, h.b2, __uint_as_float(h.prim));
+    P.B.cls[k] = h.prim == kMiss ? uint8_t(kClassMiss) : P.S.mat_class[hit_material(P.S, h)];
+}
+
+MYPBR_DEV uint64_t extend_key(const WaveParams& P, int2 wave, int depth, uint32_t k) {
+    if (!P.keyed)
+        return 0;
+    const SlotPath sp = slot_path(P, wave, entry_slot(P, depth, k));
+    return media_key(P, sp.pixel, sp.pass, uint32_t(depth), 0);
+}
+
+// Closest hits of the extension queue.
 template <bool VOX, int WALK>
 __global__ void __launch_bounds__(256, 3) k_extend(WaveParams P, int depth) {
     depth = bounce_of(P, depth);
     uint32_t n = *ext_counter(P, depth);
     if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0)
         atomicAdd(&P.totals[0], (unsigned long long)n);
-    const uint32_t* q = P.B.queue[depth & 1];
+    const float4* rays = P.B.ray[depth & 1];
+    const int2 wave = wave_of(P);
     uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += stride) {
-        uint32_t slot = q[k];
-        float4 ro = P.B.ray_o[slot], rd = P.B.ray_d[slot];
-        uint64_t key = 0;
-        if (P.keyed) {
-            uint32_t pixel = f_bits(P.B.radiance[slot].w), pass = f_bits(P.B.beta[slot].w);
-            key = media_key(P, pixel, pass, uint32_t(depth), 0);
-        }
-        HitInfo h = closest_hit<VOX, WALK>(P.S, f3(ro), f3(rd), spawn_tmin(f3(ro), f3(rd)), 3.0e38f, key);
-        P.B.hit[slot] = make_float4(h.t, h.b1, h.b2, __uint_as_float(h.prim));
-        int c = h.prim == kMiss ? kClassMiss : int(P.S.mat_class[hit_material(P.S, h)]);
-        uint32_t* counter = class_counter(P, depth, c);
-        class_queue(P, c)[warp_push_keyed(counter)] = slot;
+        const Pair r = load_pair(rays, k);
+        const float3 o = f3(r.a), d = f3(r.b);
+        put_hit(P, k, closest_hit<VOX, WALK>(P.S, o, d, spawn_tmin(o, d), 3.0e38f, extend_key(P, wave, depth, k)));
     }
 }
 
@@ -384,13 +411,14 @@ __global__ void __launch_bounds__(256, 3) k_extend_pt(WaveParams P, int depth) {
     const uint32_t n = *ext_counter(P, depth);
     if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0)
         atomicAdd(&P.totals[0], (unsigned long long)n);
-    const uint32_t* q = P.B.queue[depth & 1];
+    const float4* rays = P.B.ray[depth & 1];
+    const int2 wave = wave_of(P);
     uint32_t* fetch = fetch_counter(P, depth);
     const int lane = threadIdx.x & 31;
     const unsigned lanes_below = (1u << lane) - 1u;
     WalkState W;
     int stack[kBvhStack];
-    uint32_t slot = 0;
+    uint32_t entry = 0;
     bool active = false, exhausted = false;
     // every lane's walk is bounded (node visits); this bounds the warp's steps
     // by the rays one warp could ever be given, were it given all of them
@@ -405,16 +433,11 @@ __global__ void __launch_bounds__(256, 3) k_extend_pt(WaveParams P, int depth) {
                 base = atomicAdd(fetch, uint32_t(__popc(idle)));
             base = __shfl_sync(0xffffffffu, base, leader);
             if (!active && !exhausted) {
-                uint32_t k = base + uint32_t(__popc(idle & lanes_below));
-                if (k < n) {
-                    slot = q[k];
-                    float4 ro = P.B.ray_o[slot], rd = P.B.ray_d[slot];
-                    uint64_t key = 0;
-                    if (P.keyed) {
-                        uint32_t pixel = f_bits(P.B.radiance[slot].w), pass = f_bits(P.B.beta[slot].w);
-                        key = media_key(P, pixel, pass, uint32_t(depth), 0);
-                    }
-                    walk_init(P.S, W, f3(ro), f3(rd), spawn_tmin(f3(ro), f3(rd)), 3.0e38f, key);
+                entry = base + uint32_t(__popc(idle & lanes_below));
+                if (entry < n) {
+                    const Pair r = load_pair(rays, entry);
+                    walk_init(P.S, W, f3(r.a), f3(r.b), spawn_tmin(f3(r.a), f3(r.b)), 3.0e38f,
+                              extend_key(P, wave, depth, entry));
                     active = true;
                 } else {
                     exhausted = true;
@@ -425,10 +448,7 @@ __global__ void __launch_bounds__(256, 3) k_extend_pt(WaveParams P, int depth) {
             break;
         if (active && !walk_node<false, VOX>(P.S, W, stack)) {
             walk_unbounded<false>(P.S, W);
-            const HitInfo& h = W.h;
-            P.B.hit[slot] = make_float4(h.t, h.b1, h.b2, __uint_as_float(h.prim));
-            int c = h.prim == kMiss ? kClassMiss : int(P.S.mat_class[hit_material(P.S, h)]);
-            class_queue(P, c)[warp_push_keyed(class_counter(P, depth, c))] = slot;
+            put_hit(P, entry, W.h);
             active = false;
         }
     }
@@ -443,18 +463,20 @@ constexpr int class_type() {
          : C == kClassPrincipled ? kPrincipled : -1;
 }
 template <int C>
-MYPBR_DEV bool class_scatter(const DeviceScene& S, int mi, float3 d, const Surface& s, ScatterRec& sr, Rng& g) {
+MYPBR_DEV bool class_scatter(const DeviceScene& S, int mi, float3 d, const Surface& s, ScatterRec& sr, Rng& g,
+                             const MatPoint<class_type<C>()>& pt) {
     if constexpr (C == kClassGeneric)
         return scatter(S, mi, d, s, sr, g);
     else
-        return scatter_inner<class_type<C>()>(S, S.materials[mi], d, s, sr, g);
+        return scatter_inner<class_type<C>()>(S, S.materials[mi], d, s, sr, g, pt);
 }
 template <int C>
-MYPBR_DEV float3 class_eval(const DeviceScene& S, int mi, float3 d, const Surface& s, float3 dir) {
+MYPBR_DEV float3 class_eval(const DeviceScene& S, int mi, float3 d, const Surface& s, float3 dir,
+                            float3 unit, const MatPoint<class_type<C>()>& pt) {
     if constexpr (C == kClassGeneric)
-        return eval(S, mi, d, s, dir);
+        return eval(S, mi, d, s, dir, unit);
     else
-        return eval_inner<class_type<C>()>(S, S.materials[mi], d, s, dir);
+        return eval_inner<class_type<C>()>(S, S.materials[mi], d, s, dir, unit, pt);
 }
 
 // Classes whose non-specular vertices the guiding network serves.
@@ -463,34 +485,117 @@ constexpr bool kGuidable() {
     return C == kClassLambert || C == kClassMetal || C == kClassPrincipled || C == kClassGeneric;
 }
 
+// Entries of the extension queue into their shading classes' queues, in queue
+// order: a block reads the class bytes of a tile (8 a thread), counts, takes
+// its places with one atomic per class and writes them. Neighbours stay
+// neighbours, so the shading kernels' reads of rays, hits and throughputs
+// share cache lines; queues appended by the walks' warps themselves, in the
+// order they finish, cost an atomic per warp and class on words of one L2
+// line, and scatter.
+__global__ void __launch_bounds__(256) k_classify(WaveParams P, int depth) {
+    __shared__ uint32_t sums[kShadeClasses][8], base[kShadeClasses];
+    depth = bounce_of(P, depth);
+    const uint32_t n = *ext_counter(P, depth);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // small queues are cut finer, so that every block has a tile
+    const uint32_t share = (n + gridDim.x - 1) / gridDim.x;
+    const uint32_t tile = share >= 2048 ? 2048 : (share + 7) / 8 * 8;
+    for (uint32_t at = blockIdx.x * tile; at < n; at += gridDim.x * tile) {
+        const uint32_t first = at + 8 * threadIdx.x;
+        const uint32_t mine = 8 * threadIdx.x < tile && first < n ? min(8u, n - first) : 0u;
+        uint2 b = make_uint2(0u, 0u);
+        if (mine > 0)
+            b = *reinterpret_cast<const uint2*>(P.B.cls + first);
+        // counts per class, 10 bits each: at most 8 a thread, 256 a warp
+        uint32_t c012 = 0, c345 = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < 8; j++) {
+            const uint32_t c = ((j < 4 ? b.x : b.y) >> (8 * (j & 3))) & 0xffu;
+            if (j < mine) {
+                c012 += c < 3 ? 1u << (10 * c) : 0u;
+                c345 += c >= 3 ? 1u << (10 * (c - 3)) : 0u;
+            }
+        }
+        uint32_t s012 = c012, s345 = c345;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t u0 = __shfl_up_sync(0xffffffffu, s012, o), u1 = __shfl_up_sync(0xffffffffu, s345, o);
+            s012 += lane >= o ? u0 : 0u;
+            s345 += lane >= o ? u1 : 0u;
+        }
+        if (lane == 31)
+#pragma unroll
+            for (int c = 0; c < kShadeClasses; c++)
+                sums[c][warp] = ((c < 3 ? s012 : s345) >> (10 * (c % 3))) & 0x3ffu;
+        __syncthreads();
+        if (threadIdx.x < kShadeClasses) {
+            uint32_t total = 0;
+            for (int w = 0; w < 8; w++) {
+                const uint32_t v = sums[threadIdx.x][w];
+                sums[threadIdx.x][w] = total;
+                total += v;
+            }
+            base[threadIdx.x] = total > 0 ? atomicAdd(class_counter(P, depth, threadIdx.x), total) : 0u;
+        }
+        __syncthreads();
+        s012 -= c012;
+        s345 -= c345;
+#pragma unroll
+        for (uint32_t j = 0; j < 8; j++) {
+            if (j >= mine)
+                break;
+            const uint32_t c = ((j < 4 ? b.x : b.y) >> (8 * (j & 3))) & 0xffu;
+            uint32_t& s = c < 3 ? s012 : s345;
+            const uint32_t shift = 10 * (c < 3 ? c : c - 3);
+            *class_entry(P, c, base[c] + sums[c][warp] + ((s >> shift) & 0x3ffu)) = first + j;
+            s += 1u << shift;
+        }
+        __syncthreads();
+    }
+}
+
 // One bounce of ray_color (camera.h:370-457) for the paths of shading class C.
 // GUIDED: the variant of guided renders, which reads the learned mixtures and
 // writes training records (plain renders keep the leaner code).
 template <int C, bool GUIDED>
 __device__ __forceinline__ void shade_body(const WaveParams& P, int depth) {
-    uint32_t n = *class_counter(P, depth, C);
-    const uint32_t* q = class_queue(P, C);
-    uint32_t* q_next = P.B.queue[(depth + 1) & 1];
+    const uint32_t n = *class_counter(P, depth, C);
     const DeviceScene& S = P.S;
-    uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += stride) {
-        uint32_t slot = q[k];
-        float4 ro = P.B.ray_o[slot], rd = P.B.ray_d[slot];
-        float4 bt = P.B.beta[slot], rad4 = P.B.radiance[slot];
-        uint32_t pixel = f_bits(rad4.w), pass = f_bits(bt.w), flags = f_bits(ro.w);
-        float3 o = f3(ro), d = f3(rd), beta = f3(bt), rad = f3(rad4);
-        float scatter_pdf = rd.w;
+    float4* const rays = P.B.ray[depth & 1];
+    float4* const states = P.B.state[depth & 1];
+    const int2 wave = wave_of(P);
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        const uint32_t k = *class_entry(P, C, i);
+        const Pair ray = load_pair(rays, k);
+        float3 beta = f3(1.0f), rad = f3(0.0f);
+        uint32_t slot = k;
+        if (depth > 0) {
+            const Pair st = load_pair(states, k);
+            beta = f3(st.a);
+            rad = f3(st.b);
+            slot = f_bits(st.a.w);
+        }
+        const SlotPath path = slot_path(P, wave, slot);
+        const uint32_t pixel = path.pixel, pass = path.pass, flags = f_bits(ray.a.w);
+        const float3 o = f3(ray.a), d = f3(ray.b);
+        float scatter_pdf = ray.b.w;
         bool specular = flags & kFlagSpecular, seen = flags & kFlagSeen;
         uint32_t diffuse_count = (flags >> 8) & 0xff, specular_count = (flags >> 16) & 0xff;
         uint32_t scatter_count = flags >> 24;
         bool terminate = false, pushed_shadow = false;
         float3 new_o = o, new_d = d;
         int rec_at = -1;  // record written at this vertex (index), listed if the path goes on
-        if (GUIDED && P.record && slot < P.rec_slots && depth >= 1 && depth - 1 < P.rec.depth) {
-            // what the previous vertex's record needs: radiance and throughput on arrival here
-            uint32_t r = slot * uint32_t(P.rec.depth) + uint32_t(depth - 1);
-            P.rec.mark[r] = make_float4(rad.x, rad.y, rad.z, 0.0f);
-            P.rec.bnext[r] = make_float4(beta.x, beta.y, beta.z, 0.0f);
+        uint32_t rec_slot = 0;
+        bool recorded = false;
+        if (GUIDED && P.record && path.band_pass < uint32_t(P.rec_passes)) {
+            recorded = true;
+            rec_slot = path.band_pixel * uint32_t(P.rec_passes) + path.band_pass;
+            if (depth >= 1 && depth - 1 < P.rec.depth) {
+                // what the previous vertex's record needs: radiance and throughput on arrival here
+                uint32_t r = rec_slot * uint32_t(P.rec.depth) + uint32_t(depth - 1);
+                P.rec.mark[r] = make_float4(rad.x, rad.y, rad.z, 0.0f);
+                P.rec.bnext[r] = make_float4(beta.x, beta.y, beta.z, 0.0f);
+            }
         }
         if constexpr (C == kClassMiss) {
             // camera.h:373-387: the sky is a light, weighted like emission
@@ -511,7 +616,7 @@ __device__ __forceinline__ void shade_body(const WaveParams& P, int depth) {
             terminate = true;
         } else {
             Rng g = bounce_rng(P, pixel, pass, depth, 0);
-            float4 hb = P.B.hit[slot];
+            float4 hb = P.B.hit[k];
             HitInfo h;
             h.t = hb.x;
             h.b1 = hb.y;
@@ -533,7 +638,8 @@ __device__ __forceinline__ void shade_body(const WaveParams& P, int depth) {
                 }
             }
             ScatterRec sr;
-            if (!class_scatter<C>(S, mat, d, s, sr, g)) {
+            const MatPoint<class_type<C>()> pt = mat_point<class_type<C>()>(S, S.materials[mat], d, s);
+            if (!class_scatter<C>(S, mat, d, s, sr, g, pt)) {
                 terminate = true;
             } else if (sr.skip_pdf) {  // camera.h:413-423
                 if (P.max_specular > 0 && ++specular_count > uint32_t(P.max_specular)) {
@@ -541,7 +647,7 @@ __device__ __forceinline__ void shade_body(const WaveParams& P, int depth) {
                 } else {
                     beta *= sr.attenuation;
                     new_d = sr.skip_dir;
-                    new_o = spawn_origin(s, new_d);
+                    new_o = spawn_origin<!GUIDED>(s, new_d);
                     if (P.transparent_shadows && lets_shadows_through(S, mat) && P.has_lights && depth > 0 && !specular)
                         seen = true;
                     specular = true;
@@ -561,13 +667,13 @@ __device__ __forceinline__ void shade_body(const WaveParams& P, int depth) {
                 const float ga = depth == 0 ? P.guide_alpha : P.guide_alpha_deep;
                 if constexpr (GUIDED && kGuidable<C>()) {
                     if (P.guided && ga > 0.0f && !vol && depth < P.guide_depths) {
-                        guide_unpack(P.guide_mix[slot], gm);
+                        guide_unpack(P.guide_mix[k], gm);
                         use_guide = true;
                     }
                 }
-                auto mis_pdf = [&](float3 dir) {
-                    float pb = sr.pdf.value(dir);
-                    return use_guide ? ga * guide_pdf(gm, normalize(dir)) + (1.0f - ga) * pb : pb;
+                auto mis_pdf = [&](float3 dir, float3 unit) {
+                    float pb = sr.pdf.value(dir, unit);
+                    return use_guide ? ga * guide_pdf(gm, unit) + (1.0f - ga) * pb : pb;
                 };
                 if (P.has_lights) {  // camera.h:466-506; the shadow ray is traced by k_shadow
                     // With the sky as the only light, the sample carries its own
@@ -582,16 +688,18 @@ __device__ __forceinline__ void shade_body(const WaveParams& P, int depth) {
                         lp = lights_pdf(S, s.p, to_light);
                     }
                     if (lp > 0.0f) {
-                        float3 f = class_eval<C>(S, mat, d, s, to_light);
+                        const float3 light_unit = normalize_y(to_light);
+                        float3 f = class_eval<C>(S, mat, d, s, to_light, light_unit, pt);
                         if (f.x > 0.0f || f.y > 0.0f || f.z > 0.0f) {
-                            float w = last ? 1.0f : power_heuristic(lp, mis_pdf(to_light));
+                            float w = last ? 1.0f : power_heuristic(lp, mis_pdf(to_light, light_unit));
                             float3 c = beta * f * sky * (w / lp);
-                            float3 sd = normalize(to_light);
-                            float3 so = spawn_origin(s, sd);
-                            P.B.sh_o[slot] = make_float4(so.x, so.y, so.z, 0.0f);
-                            P.B.sh_d[slot] = make_float4(sd.x, sd.y, sd.z, 0.0f);
-                            P.B.sh_c[slot] = make_float4(c.x, c.y, c.z, sky_only ? 1.0f : 0.0f);
-                            P.B.shadow_queue[warp_push(sh_counter(P, depth))] = slot;
+                            float3 sd = light_unit;
+                            float3 so = spawn_origin<!GUIDED>(s, sd);
+                            // the entry's own ray and throughput were read above: the shadow
+                            // ray takes their place
+                            store_pair(rays, k, make_float4(so.x, so.y, so.z, bits_f(slot)),
+                                       make_float4(sd.x, sd.y, sd.z, sky_only ? 1.0f : 0.0f));
+                            states[2 * size_t(k)] = make_float4(c.x, c.y, c.z, 0.0f);
                             pushed_shadow = true;
                         }
                     }
@@ -606,22 +714,23 @@ __device__ __forceinline__ void shade_body(const WaveParams& P, int depth) {
                     } else {
                         dir = sr.pdf.generate(g);
                     }
-                    float spdf = mis_pdf(dir);
+                    const float3 unit = normalize_x(dir);
+                    float spdf = mis_pdf(dir, unit);
                     if (!(spdf > 0.0f)) {
                         terminate = true;
                     } else {
-                        float3 factor = class_eval<C>(S, mat, d, s, dir) / spdf;
+                        float3 factor = class_eval<C>(S, mat, d, s, dir, unit, pt) / spdf;
                         beta *= factor;
                         scatter_pdf = spdf;
                         new_d = dir;
-                        new_o = spawn_origin(s, new_d);
+                        new_o = spawn_origin<!GUIDED>(s, new_d);
                         specular = false;
                         if constexpr (GUIDED && kGuidable<C>()) {
-                            if (P.record && !vol && slot < P.rec_slots && depth < P.rec.depth) {
+                            if (recorded && !vol && depth < P.rec.depth) {
                                 float sc[7];
                                 guide_scalars(s.p, s.normal, normalize(-1.0f * d), P.guide_lo, P.guide_inv, sc);
-                                float3 wd = normalize(dir);
-                                uint32_t r = slot * uint32_t(P.rec.depth) + uint32_t(depth);
+                                float3 wd = unit;
+                                uint32_t r = rec_slot * uint32_t(P.rec.depth) + uint32_t(depth);
                                 P.rec.in0[r] = make_float4(sc[0], sc[1], sc[2], sc[3]);
                                 P.rec.in1[r] = make_float4(sc[4], sc[5], sc[6], 0.0f);
                                 P.rec.dir[r] = make_float4(wd.x, wd.y, wd.z, 0.0f);
@@ -643,36 +752,41 @@ __device__ __forceinline__ void shade_body(const WaveParams& P, int depth) {
             if (!terminate && depth + 1 >= P.max_depth)
                 terminate = true;
         }
-        if (terminate) {
-            if (pushed_shadow) {
-                P.B.radiance[slot] = make_float4(rad.x, rad.y, rad.z, rad4.w);
-                P.B.sh_d[slot].w = 1.0f;  // the shadow kernel finishes this path
-            } else {
-                film_add(P, pixel, rad);
-                if (GUIDED && P.record && slot < P.rec_slots)
-                    P.rec.fin[slot] = make_float4(rad.x, rad.y, rad.z, 0.0f);
-            }
-            continue;
+        uint32_t at_next = 0;
+        if (terminate) {  // the shadow kernel adds to it, if a shadow ray is under way
+            P.B.out[slot] = make_float4(rad.x, rad.y, rad.z, 0.0f);
+            if (GUIDED && recorded && !pushed_shadow)
+                P.rec.fin[rec_slot] = make_float4(rad.x, rad.y, rad.z, 0.0f);
+        } else {
+            if (GUIDED && rec_at >= 0)  // the path goes on: the next vertex completes the record
+                P.rec.list[warp_push(P.rec.count)] = uint32_t(rec_at);
+            const uint32_t nflags = (specular ? kFlagSpecular : 0u) | (seen ? kFlagSeen : 0u) | (diffuse_count << 8) |
+                                    (specular_count << 16) | (scatter_count << 24);
+            at_next = warp_push(ext_counter(P, depth + 1));
+            store_pair(P.B.ray[(depth + 1) & 1], at_next, make_float4(new_o.x, new_o.y, new_o.z, bits_f(nflags)),
+                       make_float4(new_d.x, new_d.y, new_d.z, scatter_pdf));
+            store_pair(P.B.state[(depth + 1) & 1], at_next, make_float4(beta.x, beta.y, beta.z, bits_f(slot)),
+                       make_float4(rad.x, rad.y, rad.z, 0.0f));
         }
-        if (GUIDED && rec_at >= 0)  // the path goes on: the next vertex completes the record
-            P.rec.list[warp_push(P.rec.count)] = uint32_t(rec_at);
-        uint32_t nflags = (specular ? kFlagSpecular : 0u) | (seen ? kFlagSeen : 0u) | (diffuse_count << 8) |
-                          (specular_count << 16) | (scatter_count << 24);
-        P.B.ray_o[slot] = make_float4(new_o.x, new_o.y, new_o.z, bits_f(nflags));
-        P.B.ray_d[slot] = make_float4(new_d.x, new_d.y, new_d.z, scatter_pdf);
-        P.B.beta[slot] = make_float4(beta.x, beta.y, beta.z, bt.w);
-        P.B.radiance[slot] = make_float4(rad.x, rad.y, rad.z, rad4.w);
-        q_next[warp_push(ext_counter(P, depth + 1))] = slot;
+        if (pushed_shadow)
+            P.B.shadow_queue[warp_push(sh_counter(P, depth))] =
+                make_uint2(k, terminate ? kShadowEnds | slot : at_next);
     }
 }
 
-// The shading kernels. The plain ones leave registers to the compiler
-// (requiring one or three resident blocks instead, with more registers or a
-// few spills, measured 2.5 % slower on the sphere field); the guided ones
-// would take up to 211 registers, one block of 256 per multiprocessor, and
-// are held to two (a guided render 19 % faster).
+// The shading kernels. Resident blocks asked for, by class: measured on one
+// box, two blocks of 256 for the lambertian, metal and dielectric kernels
+// (sphere field at 64 spp: shading 22.2 ms against 24.9 with the compiler's
+// choice and 32.9 with one block), the compiler's choice for the principled
+// and generic ones, which spill less gainfully when bound (300 k-triangle
+// room: 12.8 ms against 14.2 with two and 17.5 with one). The guided ones would
+// take up to 211 registers, one block per multiprocessor, and are held to two
+// (a guided render 19 % faster).
+constexpr int shade_blocks(int c) {
+    return c == kClassMiss ? 4 : c == kClassPrincipled || c == kClassGeneric ? 0 : 2;
+}
 template <int C>
-__global__ void __launch_bounds__(256) k_shade(WaveParams P, int depth) {
+__global__ void __launch_bounds__(256, shade_blocks(C)) k_shade(WaveParams P, int depth) {
     shade_body<C, false>(P, bounce_of(P, depth));
 }
 template <int C>
@@ -688,25 +802,29 @@ __global__ void __launch_bounds__(256, 3) k_shadow(WaveParams P, int depth) {
         atomicAdd(&P.totals[1], (unsigned long long)n);
     const DeviceScene& S = P.S;
     uint32_t stride = gridDim.x * blockDim.x;
+    const float4* rays = P.B.ray[depth & 1];
+    const float4* states = P.B.state[depth & 1];
+    const int2 wave = wave_of(P);
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += stride) {
-        uint32_t slot = P.B.shadow_queue[k];
-        float4 so = P.B.sh_o[slot], sd = P.B.sh_d[slot], sc = P.B.sh_c[slot];
-        float3 o = f3(so), d = f3(sd);
+        const uint2 entry = P.B.shadow_queue[k];
+        const Pair ray = load_pair(rays, entry.x);
+        float3 o = f3(ray.a), d = f3(ray.b);
         uint64_t key = 0;
         uint32_t pixel = 0, pass = 0;
         if (P.keyed) {
-            pixel = f_bits(P.B.radiance[slot].w);
-            pass = f_bits(P.B.beta[slot].w);
+            const SlotPath sp = slot_path(P, wave, f_bits(ray.a.w));
+            pixel = sp.pixel;
+            pass = sp.pass;
         }
         float3 through = f3(1.0f), emission = f3(0.0f);
         if (!S.has_emitters && !(P.transparent_shadows && S.has_clear_glass)) {
             // Nothing the ray can reach emits, and nothing lets it through:
             // only whether it escapes matters (camera.h:488-503). A sky-only
-            // sample already holds the sky's radiance (sc.w = 1).
+            // sample already holds the sky's radiance (marked beside the direction).
             if (P.keyed)
                 key = media_key(P, pixel, pass, uint32_t(depth), 1);
             if (!any_hit<VOX, WALK>(S, o, d, spawn_tmin(o, d), 3.0e38f, key))
-                emission = sc.w != 0.0f ? f3(1.0f) : escaped_radiance(S, d, false);
+                emission = ray.b.w != 0.0f ? f3(1.0f) : escaped_radiance(S, d, false);
         } else
         for (int hop = 0; hop <= 16; hop++) {
             if (P.keyed)
@@ -731,14 +849,112 @@ __global__ void __launch_bounds__(256, 3) k_shadow(WaveParams P, int depth) {
             emission = emitted(S, mat, d, s);
             break;
         }
-        float4 r4 = P.B.radiance[slot];
-        float3 rad = f3(r4) + f3(sc) * through * emission;
-        if (sd.w != 0.0f) {
-            film_add(P, f_bits(r4.w), rad);
-            if (P.record && slot < P.rec_slots)
-                P.rec.fin[slot] = make_float4(rad.x, rad.y, rad.z, 0.0f);
-        } else
-            P.B.radiance[slot] = make_float4(rad.x, rad.y, rad.z, r4.w);
+        const float4 sc = states[2 * size_t(entry.x)];
+        const bool ends = entry.y & kShadowEnds;
+        float4* to = ends ? P.B.out + (entry.y & ~kShadowEnds) : P.B.state[(depth + 1) & 1] + 2 * size_t(entry.y) + 1;
+        float3 rad = f3(*to) + f3(sc) * through * emission;
+        *to = make_float4(rad.x, rad.y, rad.z, 0.0f);
+        if (P.record && ends) {
+            const SlotPath sp = slot_path(P, wave, entry.y & ~kShadowEnds);
+            if (sp.band_pass < uint32_t(P.rec_passes))
+                P.rec.fin[sp.band_pixel * uint32_t(P.rec_passes) + sp.band_pass] =
+                    make_float4(rad.x, rad.y, rad.z, 0.0f);
+        }
+    }
+}
+
+// A finite FP32 value in FP64, by its bits: the FP64 pipe, which converts two
+// values a clock on an SM, is left to the sums. FP32 results here are never
+// denormal (they flush to zero).
+MYPBR_DEV double widen(float x) {
+    const uint32_t u = __float_as_uint(x), m = u & 0x7fffffffu;
+    if (m < 0x00800000u)
+        return 0.0;
+    return __hiloint2double(int((u & 0x80000000u) | ((m >> 3) + 0x38000000u)), int(u << 29));
+}
+
+// A finished wave's radiance into the film: `lanes` lanes (a power of two)
+// share a pixel, whose slots are neighbours, and the first adds their FP64
+// sums to the film. No two threads touch a pixel, so nothing is atomic, and a
+// frame's last bits do not depend on the order in which paths end. moments:
+// the squares too (the per-channel variance), which only some calls ask for.
+// The FP64 atomics this replaces cost each path six read-modify-writes in L2.
+__global__ void __launch_bounds__(256) k_accumulate(WaveParams P, int gated) {
+    if (gated && !wave_ending(P))
+        return;
+    const int2 wv = wave_of(P);
+    const uint32_t passes = uint32_t(wv.y), npix = uint32_t(P.cam.width) * uint32_t(P.band_rows);
+    // Four lanes a pixel read 64 bytes at a time and leave two levels of
+    // cross-lane sums; a whole warp would spend more FP64 additions on those
+    // than on the radiances (an SM carries out two a clock). More lanes only
+    // where the pixels alone do not fill the GPU.
+    uint32_t lanes = 1;
+    while (lanes < 32 && lanes < passes && (lanes < 4 || npix * lanes < 131072u))
+        lanes *= 2;
+    const uint32_t sub = threadIdx.x & (lanes - 1);
+    const uint32_t stride = gridDim.x * blockDim.x / lanes;
+    const uint32_t rounds = (npix + stride - 1) / stride;
+    uint32_t band_pixel = (blockIdx.x * blockDim.x + threadIdx.x) / lanes;
+    for (uint32_t round = 0; round < rounds; round++, band_pixel += stride) {
+        double s0 = 0.0, s1 = 0.0, s2 = 0.0, q0 = 0.0, q1 = 0.0, q2 = 0.0, ql = 0.0;
+        if (band_pixel < npix) {
+            const float4* out = P.B.out + size_t(band_pixel) * passes;
+            auto add = [&](float4 c4) {
+                float3 c = f3(c4);
+                // NaN or infinite estimates count as black (camera.h:281-287)
+                if (!isfinite(c.x) || !isfinite(c.y) || !isfinite(c.z))
+                    c = f3(0.0f);
+                s0 += widen(c.x);
+                s1 += widen(c.y);
+                s2 += widen(c.z);
+                if (P.moments) {
+                    q0 += double(c.x) * c.x;
+                    q1 += double(c.y) * c.y;
+                    q2 += double(c.z) * c.z;
+                }
+                if (P.collect_features) {
+                    const double l = luminance(c);
+                    ql += l * l;
+                }
+            };
+            uint32_t p = sub;
+            for (; p + 3 * lanes < passes; p += 4 * lanes) {  // four reads under way
+                const float4 a = out[p], b = out[p + lanes], c = out[p + 2 * lanes], e = out[p + 3 * lanes];
+                add(a);
+                add(b);
+                add(c);
+                add(e);
+            }
+            for (; p < passes; p += lanes)
+                add(out[p]);
+        }
+        for (uint32_t m = lanes / 2; m > 0; m >>= 1) {
+            s0 += __shfl_xor_sync(0xffffffffu, s0, m);
+            s1 += __shfl_xor_sync(0xffffffffu, s1, m);
+            s2 += __shfl_xor_sync(0xffffffffu, s2, m);
+            if (P.moments) {
+                q0 += __shfl_xor_sync(0xffffffffu, q0, m);
+                q1 += __shfl_xor_sync(0xffffffffu, q1, m);
+                q2 += __shfl_xor_sync(0xffffffffu, q2, m);
+            }
+            if (P.collect_features)
+                ql += __shfl_xor_sync(0xffffffffu, ql, m);
+        }
+        if (sub != 0 || band_pixel >= npix)
+            continue;
+        const size_t pixel = size_t(P.first_row) * P.cam.width + band_pixel;
+        double* f = P.B.film + 3 * pixel;
+        f[0] += s0;
+        f[1] += s1;
+        f[2] += s2;
+        if (P.moments) {
+            double* f2 = P.B.film2 + 3 * pixel;
+            f2[0] += q0;
+            f2[1] += q1;
+            f2[2] += q2;
+        }
+        if (P.collect_features)
+            P.B.feat[7 * pixel + 6] += ql;
     }
 }
 
@@ -793,9 +1009,8 @@ __global__ void k_channel_variance(WaveParams P, int samples, double* out) {
 // ------------------------------------------------------------ host side
 
 int release_buffers(RenderBuffers& rb) {
-    void* ptrs[] = {rb.ray_o, rb.ray_d, rb.beta, rb.radiance, rb.hit, rb.sh_o, rb.sh_d, rb.sh_c, rb.queue[0],
-                    rb.queue[1], rb.class_queue, rb.shadow_queue, rb.counters, rb.wave_state, rb.film, rb.film2,
-                    rb.feat};
+    void* ptrs[] = {rb.ray[0], rb.ray[1], rb.state[0], rb.state[1], rb.hit, rb.cls, rb.class_queue, rb.shadow_queue, rb.out,
+                    rb.counters, rb.wave_state, rb.film, rb.film2, rb.feat};
     for (void* p : ptrs)
         if (p)
             cudaFree(p);
@@ -809,19 +1024,19 @@ MYPBR_HD constexpr int guided_class(int c) {
     return c == 0 ? kClassLambert : c == 1 ? kClassMetal : c == 2 ? kClassPrincipled : kClassGeneric;
 }
 
-MYPBR_DEV uint32_t guided_slot(const WaveParams& P, int depth, long long i) {
+MYPBR_DEV uint32_t guided_entry(const WaveParams& P, int depth, long long i) {
 #pragma unroll
     for (int c = 0; c < 4; c++) {
         long long n = *class_counter(P, depth, guided_class(c));
         if (i < n)
-            return class_queue(P, guided_class(c))[i];
+            return *class_entry(P, guided_class(c), uint32_t(i));
         i -= n;
     }
     return 0;  // not reached: i < count()
 }
 
 // The guidable vertices of a bounce (depth -1: the bounce in device memory),
-// none past the guided depths. A row is the vertex's path slot and, once
+// none past the guided depths. A row is the vertex's queue entry and, once
 // finished, its 7 network scalars; load starts the reads of the ray and hit
 // records, finish turns them into the surface point and its scalars.
 struct GuideQueueSource {
@@ -830,7 +1045,7 @@ struct GuideQueueSource {
     struct Row {
         float4 ro, rd, hb;
         float s[kGuideScalars];
-        uint32_t slot;
+        uint32_t entry;
         bool valid;
     };
     MYPBR_DEV long long count(long long) const {
@@ -847,10 +1062,12 @@ struct GuideQueueSource {
         r.valid = i >= 0;
         if (!r.valid)
             return;
-        r.slot = guided_slot(P, bounce_of(P, depth), i);
-        r.ro = P.B.ray_o[r.slot];
-        r.rd = P.B.ray_d[r.slot];
-        r.hb = P.B.hit[r.slot];
+        const int d = bounce_of(P, depth);
+        r.entry = guided_entry(P, d, i);
+        const Pair ray = load_pair(P.B.ray[d & 1], r.entry);
+        r.ro = ray.a;
+        r.rd = ray.b;
+        r.hb = P.B.hit[r.entry];
     }
     MYPBR_DEV void finish(Row& r) const {
         if (!r.valid) {  // a padding row: its outputs are never used
@@ -875,11 +1092,11 @@ struct GuidePackSink {
     MYPBR_DEV void put(long long, const GuideQueueSource::Row& r, const float* v) const {
         GuidePacked pk;
         guide_pack(v, pk);
-        P.guide_mix[r.slot] = pk;
+        P.guide_mix[r.entry] = pk;
     }
 };
 
-size_t counter_words(int depth_slots) { return size_t(depth_slots) * (3 + kShadeClasses) + 8; }
+size_t counter_words(int depth_slots) { return size_t(depth_slots) * kCounterRows + 8; }
 
 namespace {
 
@@ -899,18 +1116,15 @@ int ensure_buffers(RenderBuffers& rb, size_t capacity, size_t pixels, int depth_
     int s = MYPBR_OK;
 #define A(ptr, n) \
     if (s == MYPBR_OK) s = alloc(ptr, n)
-    A(rb.ray_o, capacity);
-    A(rb.ray_d, capacity);
-    A(rb.beta, capacity);
-    A(rb.radiance, capacity);
+    for (int k = 0; k < 2; k++) {
+        A(rb.ray[k], 2 * capacity);
+        A(rb.state[k], 2 * capacity);
+    }
     A(rb.hit, capacity);
-    A(rb.sh_o, capacity);
-    A(rb.sh_d, capacity);
-    A(rb.sh_c, capacity);
-    A(rb.queue[0], capacity);
-    A(rb.queue[1], capacity);
-    A(rb.class_queue, capacity * kShadeClasses);
+    A(rb.cls, (capacity + 7) / 8 * 8);  // read eight at a time
+    A(rb.class_queue, capacity * (kShadeClasses / 2));
     A(rb.shadow_queue, capacity);
+    A(rb.out, capacity);
     A(rb.counters, counter_words(depth_slots));
     A(rb.wave_state, 4);
     A(rb.film, 3 * pixels);
@@ -1165,6 +1379,14 @@ int run_prefix(WaveParams& P, const Launch& L, cudaStream_t st, uint64_t& launch
     return MYPBR_OK;
 }
 
+// A wave's end: its paths' radiance into the film.
+int run_suffix(WaveParams& P, const Launch& L, cudaStream_t st, uint64_t& launches, KernelTimer& T) {
+    TIMED(4, (k_accumulate<<<L.grid_stream, 256, 0, st>>>(P, 0)));
+    launches++;
+    MYPBR_CUDA(cudaGetLastError());
+    return MYPBR_OK;
+}
+
 // One bounce: extend, the guiding network's mixtures (guided renders), the
 // shading classes, shadow rays. depth -1: the bounce counter in device memory.
 int run_bounce(WaveParams& P, const Launch& L, cudaStream_t st, uint64_t& launches, KernelTimer& T, int depth) {
@@ -1174,6 +1396,7 @@ int run_bounce(WaveParams& P, const Launch& L, cudaStream_t st, uint64_t& launch
         TIMED(1, (k_extend_pt<false><<<L.grid_extend, L.block, 0, st>>>(P, depth)));
     else
         TIMED(1, (launch_bounce_kernel(extend_kernel(P.S.has_voxels, L.walk), L.grid_extend, L.block, st, P, depth)));
+    TIMED(2, (k_classify<<<L.grid_stream, 256, 0, st>>>(P, depth)));
     if (P.guided && (depth < 0 || depth < P.guide_depths)) {  // the mixtures of this bounce's guidable vertices
         TIMED(4, (k_guide_forward<GuideQueueSource, GuidePackSink><<<L.grid_guide, 128 * kGuideGroups, L.guide_smem, st>>>(
                      L.net, GuideQueueSource{P, depth}, GuidePackSink{P}, 0)));
@@ -1195,7 +1418,7 @@ int run_bounce(WaveParams& P, const Launch& L, cudaStream_t st, uint64_t& launch
         TIMED(2, (k_shade<kClassGeneric><<<L.grid_shade, L.block, 0, st>>>(P, depth)));
     }
     TIMED(3, (launch_bounce_kernel(shadow_kernel(P.S.has_voxels, L.walk), L.grid_shadow, L.block, st, P, depth)));
-    launches += 2 + kShadeClasses;
+    launches += 3 + kShadeClasses;
     return MYPBR_OK;
 }
 
@@ -1207,8 +1430,7 @@ int run_wave(WaveParams& P, const Launch& L, cudaStream_t st, uint64_t& launches
         s = run_bounce(P, L, st, launches, T, depth);
     if (s != MYPBR_OK)
         return s;
-    MYPBR_CUDA(cudaGetLastError());
-    return MYPBR_OK;
+    return run_suffix(P, L, st, launches, T);
 }
 
 // A wave's bounces as a CUDA graph replayed for every wave with the same
@@ -1293,7 +1515,7 @@ int launch_wave(WaveParams& P, const Launch& L, cudaStream_t st, uint64_t& launc
     if (s != MYPBR_OK)
         return s;
     MYPBR_CUDA(cudaGraphLaunch(graph->exec, st));
-    return MYPBR_OK;
+    return run_suffix(P, L, st, launches, T);
 }
 
 // Whether waves on stream st may be captured: not the legacy default stream,
@@ -1399,7 +1621,7 @@ int prepare(mypbr_gpu_scene* G, const mypbr_camera* cam, const mypbr_render_opts
             return s;
         GuideState& g = G->guide;
         P.rec = g.rec;
-        P.rec_slots = uint32_t(g.rec_slots);
+        P.rec_passes = int(g.rec_slots / std::max<size_t>(R.npix, 1));
         P.guide_mix = reinterpret_cast<GuidePacked*>(g.packed);
         P.guide_lo = g.box_lo;
         P.guide_inv = g.box_inv;
@@ -1484,9 +1706,11 @@ int render_all(mypbr_gpu_scene* G, RenderSetup& R, cudaStream_t st, double* d_ra
     MYPBR_CUDA(cudaMalloc(&tot.d, 3 * sizeof(unsigned long long)));
     MYPBR_CUDA(cudaMemsetAsync(tot.d, 0, 3 * sizeof(unsigned long long), st));
     P.totals = tot.d;
+    P.moments = d_chvar != nullptr;
     size_t full = size_t(P.cam.width) * P.cam.height;
     MYPBR_CUDA(cudaMemsetAsync(P.B.film, 0, 3 * full * sizeof(double), st));
-    MYPBR_CUDA(cudaMemsetAsync(P.B.film2, 0, 3 * full * sizeof(double), st));
+    if (P.moments)
+        MYPBR_CUDA(cudaMemsetAsync(P.B.film2, 0, 3 * full * sizeof(double), st));
     if (P.collect_features)
         MYPBR_CUDA(cudaMemsetAsync(P.B.feat, 0, 7 * full * sizeof(double), st));
     uint64_t launches = 0;
@@ -1671,7 +1895,6 @@ int job_start(mypbr_batch_job& jb, BatchJob& j) {
     P.totals = j.tot.d;
     size_t full = size_t(P.cam.width) * P.cam.height;
     MYPBR_CUDA(cudaMemsetAsync(P.B.film, 0, 3 * full * sizeof(double), st));
-    MYPBR_CUDA(cudaMemsetAsync(P.B.film2, 0, 3 * full * sizeof(double), st));
     if (P.collect_features)
         MYPBR_CUDA(cudaMemsetAsync(P.B.feat, 0, 7 * full * sizeof(double), st));
     P.B.wave_state = G->rb.wave_state;
@@ -1697,7 +1920,6 @@ int capture_job(const mypbr_batch_job& jb, RenderSetup& R, cudaStream_t st, cuda
     size_t full = size_t(P.cam.width) * P.cam.height;
     MYPBR_CUDA(cudaMemsetAsync(P.totals, 0, 3 * sizeof(unsigned long long), st));
     MYPBR_CUDA(cudaMemsetAsync(P.B.film, 0, 3 * full * sizeof(double), st));
-    MYPBR_CUDA(cudaMemsetAsync(P.B.film2, 0, 3 * full * sizeof(double), st));
     if (P.collect_features)
         MYPBR_CUDA(cudaMemsetAsync(P.B.feat, 0, 7 * full * sizeof(double), st));
     const int words = int(counter_words(P.B.depth_slots));
@@ -1725,6 +1947,7 @@ int capture_job(const mypbr_batch_job& jb, RenderSetup& R, cudaStream_t st, cuda
     if (P.collect_features)
         k_features<<<R.L.grid_shade, 256, 0, side>>>(P, 1);
     int s = run_bounce(P, R.L, side, n, off, -1);
+    k_accumulate<<<R.L.grid_stream, 256, 0, side>>>(P, 1);
     if (s == MYPBR_OK)
         k_job_step<<<1, 256, 0, side>>>(P, loop, R.per_wave, R.spp, words);
     cudaGraph_t body = nullptr;
@@ -2076,9 +2299,9 @@ constexpr int kNoAllocMaxDepth = 1024;
 constexpr size_t kNoAllocAlign = 256;
 
 constexpr size_t align_up(size_t x) { return (x + kNoAllocAlign - 1) / kNoAllocAlign * kNoAllocAlign; }
-constexpr size_t kSlotBytes = 8 * sizeof(float4) + (3 + kShadeClasses) * sizeof(uint32_t);
+constexpr size_t kSlotBytes = 10 * sizeof(float4) + sizeof(uint2) + kShadeClasses / 2 * sizeof(uint32_t) + 1;
 constexpr size_t kPixelBytes = (3 + 3 + 7) * sizeof(double);
-constexpr size_t kCounterBytes = ((3 + kShadeClasses) * (kNoAllocMaxDepth + 1) + 8) * sizeof(uint32_t);
+constexpr size_t kCounterBytes = (kCounterRows * (kNoAllocMaxDepth + 1) + 8) * sizeof(uint32_t);
 constexpr size_t kNoAllocNeed = 16 * kNoAllocAlign + kNoAllocMaxPixels * (kSlotBytes + kPixelBytes) + kCounterBytes +
                                 2 * sizeof(unsigned long long);
 constexpr size_t kNoAllocBytes = size_t(18) << 20;
@@ -2116,18 +2339,15 @@ RenderBuffers carve(unsigned char* base, unsigned long long** totals) {
         return p;
     };
     const size_t n = kNoAllocMaxPixels;
-    rb.ray_o = reinterpret_cast<float4*>(take(n * sizeof(float4)));
-    rb.ray_d = reinterpret_cast<float4*>(take(n * sizeof(float4)));
-    rb.beta = reinterpret_cast<float4*>(take(n * sizeof(float4)));
-    rb.radiance = reinterpret_cast<float4*>(take(n * sizeof(float4)));
+    for (int k = 0; k < 2; k++) {
+        rb.ray[k] = reinterpret_cast<float4*>(take(2 * n * sizeof(float4)));
+        rb.state[k] = reinterpret_cast<float4*>(take(2 * n * sizeof(float4)));
+    }
     rb.hit = reinterpret_cast<float4*>(take(n * sizeof(float4)));
-    rb.sh_o = reinterpret_cast<float4*>(take(n * sizeof(float4)));
-    rb.sh_d = reinterpret_cast<float4*>(take(n * sizeof(float4)));
-    rb.sh_c = reinterpret_cast<float4*>(take(n * sizeof(float4)));
-    rb.queue[0] = reinterpret_cast<uint32_t*>(take(n * sizeof(uint32_t)));
-    rb.queue[1] = reinterpret_cast<uint32_t*>(take(n * sizeof(uint32_t)));
-    rb.class_queue = reinterpret_cast<uint32_t*>(take(kShadeClasses * n * sizeof(uint32_t)));
-    rb.shadow_queue = reinterpret_cast<uint32_t*>(take(n * sizeof(uint32_t)));
+    rb.out = reinterpret_cast<float4*>(take(n * sizeof(float4)));
+    rb.shadow_queue = reinterpret_cast<uint2*>(take(n * sizeof(uint2)));
+    rb.class_queue = reinterpret_cast<uint32_t*>(take(kShadeClasses / 2 * n * sizeof(uint32_t)));
+    rb.cls = take(n);
     rb.counters = reinterpret_cast<uint32_t*>(take(kCounterBytes));
     rb.film = reinterpret_cast<double*>(take(3 * n * sizeof(double)));
     rb.film2 = reinterpret_cast<double*>(take(3 * n * sizeof(double)));
@@ -2193,7 +2413,6 @@ extern "C" int mypbr_gpu_render_noalloc(mypbr_gpu_scene* G, const mypbr_camera* 
     // The array keeps the last call's contents: clear what accumulates (the
     // band's film only, which starts at the array's film buffers)
     MYPBR_CUDA(cudaMemsetAsync(P.B.film, 0, 3 * npix * sizeof(double), st));
-    MYPBR_CUDA(cudaMemsetAsync(P.B.film2, 0, 3 * npix * sizeof(double), st));
     if (P.collect_features)
         MYPBR_CUDA(cudaMemsetAsync(P.B.feat, 0, 7 * npix * sizeof(double), st));
     MYPBR_CUDA(cudaMemsetAsync(P.totals, 0, 2 * sizeof(unsigned long long), st));
