@@ -43,6 +43,10 @@ MYPBR_DEV float3 normalize(float3 a) { return a * rsqrtf(dot(a, a)); }
 // decides (x first, or y first).
 MYPBR_DEV float dot_x(float3 a, float3 b) { return fmaf(a.z, b.z, fmaf(a.x, b.x, a.y * b.y)); }
 MYPBR_DEV float dot_y(float3 a, float3 b) { return fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x)); }
+// a s + b t with the first product fused.
+MYPBR_DEV float3 weigh(float3 a, float s, float3 b, float t) {
+    return f3(fmaf(a.x, s, b.x * t), fmaf(a.y, s, b.y * t), fmaf(a.z, s, b.z * t));
+}
 MYPBR_DEV float3 normalize_x(float3 a) { return a * rsqrtf(dot_x(a, a)); }
 MYPBR_DEV float3 normalize_y(float3 a) { return a * rsqrtf(dot_y(a, a)); }
 MYPBR_HD float comp(float3 a, int i) { return i == 0 ? a.x : (i == 1 ? a.y : a.z); }

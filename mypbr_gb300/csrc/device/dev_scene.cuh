@@ -8,6 +8,9 @@
 //               references. Boxes are rounded outwards to FP32. Loaded with
 //               128-bit loads through the read-only path.
 //   leaf_refs   (kind << 29 | index) per leaf slot.
+//   leaves      64 bytes per leaf slot: its reference and what the walk's
+//               intersection test reads of its primitive (pack_leaf), so that
+//               a leaf costs one dependent read instead of two or three.
 //   spheres     float4 (centre, radius) + int2 (material, xform).
 //   quads       5 float4: (Q | material), u, v, unit normal n, w = (u x v) / |u x v|^2.
 //   triangles   3 float4 (v0 | material), (v1 | flags), (v2 | mesh); shading
@@ -71,6 +74,8 @@ struct DeviceScene {
     // geometry
     const float4* bvh;
     const uint32_t* leaf_refs;
+    const float4* leaves;  // 4 per leaf slot
+    int leaf_tails;        // some leaf slot uses more than its first 32 bytes (triangles, quads)
     const float4* bvh4;  // the same tree collapsed to 4 children per node (nullptr: not built)
     int bvh4_node_count;
     const uint4* bvh8;   // collapsed to 8 children with quantised boxes (nullptr: not built)
@@ -130,6 +135,21 @@ struct DeviceScene {
 
 MYPBR_DEV float4 ldg4(const float4* p) { return __ldg(p); }
 
+// 32 bytes in one read through the read-only path. Lanes of a divergent walk
+// read different lines, and L1 looks lines up per instruction: a node of 64
+// bytes in two reads costs half the lookups of four 128-bit ones (they bound
+// the walks of the triangle room: L1 at 65 to 81 % of its throughput).
+struct Float8 {
+    float4 a, b;
+};
+MYPBR_DEV Float8 ldg8(const float4* p) {
+    Float8 r;
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(r.a.x), "=f"(r.a.y), "=f"(r.a.z), "=f"(r.a.w), "=f"(r.b.x), "=f"(r.b.y), "=f"(r.b.z), "=f"(r.b.w)
+        : "l"(p));
+    return r;
+}
+
 // ------------------------------------------------------------- transforms
 
 struct XformRef {
@@ -177,12 +197,13 @@ MYPBR_DEV bool sphere_root(float3 c, float r, float3 o, float3 d, float tmin, fl
     float3 f = o - c;
     float b = -dot(f, d);  // = dot(d, c - o)
     float3 l = f + (b / a) * d;  // offset of the closest point of the line from the centre
-    float disc = a * (r * r - dot(l, l));
+    const float r2 = __fmul_rn(r, r);  // rounded once, for both differences below
+    float disc = a * (r2 - dot_x(l, l));
     if (disc < 0.0f)
         return false;
     float sq = sqrtf(disc);
     float q = b + copysignf(sq, b);
-    float cc = dot(f, f) - r * r;
+    float cc = dot_x(f, f) - r2;
     float r0 = cc / q, r1 = q / a;
     if (q == 0.0f) {
         r0 = r1 = b / a;
@@ -199,30 +220,26 @@ MYPBR_DEV bool sphere_root(float3 c, float r, float3 o, float3 d, float tmin, fl
     return false;
 }
 
-MYPBR_DEV bool hit_sphere(const DeviceScene& S, int i, float3 o, float3 d, float tmin, float tmax, float& t) {
-    float4 s = ldg4(S.spheres + i);
-    int xf = __ldg(&S.sphere_info[i].y);
+// A sphere (centre, radius) under transform xf (below 0: none).
+MYPBR_DEV bool hit_sphere(const DeviceScene& S, float3 c, float r, int xf, float3 o, float3 d, float tmin, float tmax,
+                          float& t) {
     if (xf < 0)
-        return sphere_root(f3(s), s.w, o, d, tmin, tmax, t);
+        return sphere_root(c, r, o, d, tmin, tmax, t);
     XformRef X;
     load_xform(S, xf, X);
-    return sphere_root(f3(s), s.w, xf_ipoint(X, o), xf_ivec(X, d), tmin, tmax, t);
+    return sphere_root(c, r, xf_ipoint(X, o), xf_ivec(X, d), tmin, tmax, t);
 }
 
 // Plane t, then the parallelogram test 0 <= a, b <= 1 (quad.h:30-62).
-MYPBR_DEV bool hit_quad(const DeviceScene& S, int i, float3 o, float3 d, float tmin, float tmax, float& t, float& a,
-                        float& b) {
-    const float4* q = S.quads + 5 * i;
-    float4 Q = ldg4(q), n = ldg4(q + 3);
-    float3 N = f3(n);
+MYPBR_DEV bool hit_quad(float3 Q, float3 N, float3 u, float3 v, float3 w, float3 o, float3 d, float tmin, float tmax,
+                        float& t, float& a, float& b) {
     float denom = dot(N, d);
     if (fabsf(denom) < 1e-8f)
         return false;
-    float tt = dot(N, f3(Q) - o) / denom;
+    float tt = dot(N, Q - o) / denom;
     if (!(tt >= tmin && tt <= tmax))
         return false;
-    float3 hp = (o - f3(Q)) + tt * d;
-    float3 u = f3(ldg4(q + 1)), v = f3(ldg4(q + 2)), w = f3(ldg4(q + 4));
+    float3 hp = (o - Q) + tt * d;
     float al = dot(w, cross(hp, v)), be = dot(w, cross(u, hp));
     if (al < 0.0f || al > 1.0f || be < 0.0f || be > 1.0f)
         return false;
@@ -230,6 +247,13 @@ MYPBR_DEV bool hit_quad(const DeviceScene& S, int i, float3 o, float3 d, float t
     a = al;
     b = be;
     return true;
+}
+// Quad i of the scene.
+MYPBR_DEV bool hit_quad(const DeviceScene& S, int i, float3 o, float3 d, float tmin, float tmax, float& t, float& a,
+                        float& b) {
+    const float4* q = S.quads + 5 * i;
+    return hit_quad(f3(ldg4(q)), f3(ldg4(q + 3)), f3(ldg4(q + 1)), f3(ldg4(q + 2)), f3(ldg4(q + 4)), o, d, tmin, tmax,
+                    t, a, b);
 }
 
 // Per-ray constants of the watertight ray/triangle test (Woop, Benthin and
@@ -309,10 +333,9 @@ MYPBR_DEV float err_gamma(int n) {
 }
 
 template <bool MASKED = true>
-MYPBR_DEV bool hit_triangle(const DeviceScene& S, int i, float3 o, const TriRay& R, float tmin, float tmax, float& t,
-                            float& b1, float& b2, uint64_t key = 0) {
-    const float4* tp = S.tris + 3 * i;
-    float3 A = f3(ldg4(tp)) - o, B = f3(ldg4(tp + 1)) - o, C = f3(ldg4(tp + 2)) - o;
+MYPBR_DEV bool hit_triangle(const DeviceScene& S, int i, float3 v0, float3 v1, float3 v2, float3 o, const TriRay& R,
+                            float tmin, float tmax, float& t, float& b1, float& b2, uint64_t key = 0) {
+    float3 A = v0 - o, B = v1 - o, C = v2 - o;
     float Az = comp(A, R.kz), Bz = comp(B, R.kz), Cz = comp(C, R.kz);
     float Ax = comp(A, R.kx) - R.sx * Az, Ay = comp(A, R.ky) - R.sy * Az;
     float Bx = comp(B, R.kx) - R.sx * Bz, By = comp(B, R.ky) - R.sy * Bz;
@@ -488,15 +511,14 @@ MYPBR_DEV int voxel_crossing(int kf, int kt) {
     return voxel_face_visible(kf, kt) ? 2 : 0;
 }
 
-// Block i of a placed voxel model, walked cell by cell with a 3D DDA
+// A block of a placed voxel model ((model, lo), (hi, -)), walked cell by cell with a 3D DDA
 // (Amanatides and Woo 1987) in the model's space, as voxel_grid::hit
 // (voxel.h:193-268). A surface is a crossing between cells of different kind.
 // On a hit: t, the material and face = axis | (outward normal positive) << 2.
 // The walk keeps its cell, step and next-plane distances in scalars (no
 // dynamically indexed arrays, which would live in local memory).
-MYPBR_DEV bool hit_voxel_block(const DeviceScene& S, int i, float3 ow, float3 dw, float tmin, float tmax, float& t_out,
-                               int& mat_out, int& face_out) {
-    int4 b0 = __ldg(S.voxel_blocks + 2 * i), b1 = __ldg(S.voxel_blocks + 2 * i + 1);
+MYPBR_DEV bool hit_voxel_block(const DeviceScene& S, int4 b0, int4 b1, float3 ow, float3 dw, float tmin, float tmax,
+                               float& t_out, int& mat_out, int& face_out) {
     const DevVoxelModel m = S.voxel_models[b0.x];
     XformRef X;
     load_xform(S, m.xform, X);
@@ -623,6 +645,79 @@ struct HitInfo {
 };
 constexpr uint32_t kMiss = 0xffffffffu;
 
+// What a leaf slot holds of its primitive: word 3 the reference; a sphere's
+// centre, radius and transform; a quad's corner, normal, edges and w; a
+// triangle's corners (the third one's y and z in the second half); a voxel
+// block's corners and model. Media are looked up by their index.
+MYPBR_DEV void pack_leaf(const DeviceScene& S, uint32_t ref, float4* out) {
+    const int kind = int(ref >> kKindShift), i = int(ref & kIndexMask);
+    const float r = __uint_as_float(ref);
+    float4 q[4];
+    for (int k = 0; k < 4; k++)
+        q[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    q[0].w = r;
+    if (kind == kSphere) {
+        const float4 c = S.spheres[i];
+        q[0] = make_float4(c.x, c.y, c.z, r);
+        q[1] = make_float4(c.w, __int_as_float(S.sphere_info[i].y), 0.0f, 0.0f);
+    } else if (kind == kQuad) {
+        const float4 Q = S.quads[5 * i], u = S.quads[5 * i + 1], v = S.quads[5 * i + 2], n = S.quads[5 * i + 3],
+                     w = S.quads[5 * i + 4];
+        q[0] = make_float4(Q.x, Q.y, Q.z, r);
+        q[1] = make_float4(n.x, n.y, n.z, w.x);
+        q[2] = make_float4(u.x, u.y, u.z, w.y);
+        q[3] = make_float4(v.x, v.y, v.z, w.z);
+    } else if (kind == kTriangle) {
+        const float4 a = S.tris[3 * i], b = S.tris[3 * i + 1], c = S.tris[3 * i + 2];
+        q[0] = make_float4(a.x, a.y, a.z, r);
+        q[1] = make_float4(b.x, b.y, b.z, c.x);
+        q[2] = make_float4(c.y, c.z, 0.0f, 0.0f);
+    } else if (kind == kVoxel) {
+        const int4 b0 = S.voxel_blocks[2 * i], b1 = S.voxel_blocks[2 * i + 1];
+        q[0] = make_float4(__int_as_float(b0.y), __int_as_float(b0.z), __int_as_float(b0.w), r);
+        q[1] = make_float4(__int_as_float(b1.x), __int_as_float(b1.y), __int_as_float(b1.z), __int_as_float(b0.x));
+    }
+    for (int k = 0; k < 4; k++)
+        out[k] = q[k];
+}
+
+// The primitive of leaf slot `slot` against the ray; on a hit nearer than
+// tmax its t, coordinates and reference.
+template <bool VOX>
+MYPBR_DEV bool hit_leaf(const DeviceScene& S, int slot, float3 o, float3 d, const TriRay& tr, float tmin, float tmax,
+                        uint64_t media_key, float& t, float& b1, float& b2, uint32_t& ref) {
+    const float4* p = S.leaves + 4 * size_t(slot);
+    const Float8 q = ldg8(p);
+    float2 tail = make_float2(0.0f, 0.0f);
+    if (S.leaf_tails)  // under way together with the first half
+        tail = __ldg(reinterpret_cast<const float2*>(p + 2));
+    ref = __float_as_uint(q.a.w);
+    const int kind = int(ref >> kKindShift), idx = int(ref & kIndexMask);
+    b1 = b2 = 0.0f;
+    if (kind == kTriangle)
+        return hit_triangle(S, idx, f3(q.a), f3(q.b), f3(q.b.w, tail.x, tail.y), o, tr, tmin, tmax, t, b1, b2,
+                            media_key);
+    if (kind == kSphere)
+        return hit_sphere(S, f3(q.a), q.b.x, __float_as_int(q.b.y), o, d, tmin, tmax, t);
+    if (kind == kQuad) {
+        const Float8 e = ldg8(p + 2);
+        return hit_quad(f3(q.a), f3(q.b), f3(e.a), f3(e.b), f3(q.b.w, e.a.w, e.b.w), o, d, tmin, tmax, t, b1, b2);
+    }
+    if (kind == kMedium)
+        return media_key != 0 && hit_medium(S, idx, o, d, tmin, tmax, hash_uniform(media_key, uint32_t(idx)), t);
+    if (VOX && kind == kVoxel) {
+        int mat, face;
+        const int4 lo = make_int4(__float_as_int(q.b.w), __float_as_int(q.a.x), __float_as_int(q.a.y),
+                                  __float_as_int(q.a.z));
+        const int4 hi = make_int4(__float_as_int(q.b.x), __float_as_int(q.b.y), __float_as_int(q.b.z), 0);
+        const bool got = hit_voxel_block(S, lo, hi, o, d, tmin, tmax, t, mat, face);
+        b1 = __int_as_float(mat);
+        b2 = __int_as_float(face);
+        return got;
+    }
+    return false;
+}
+
 MYPBR_DEV float safe_inv(float x) { return fabsf(x) > 1e-30f ? 1.0f / x : copysignf(1e30f, x); }
 
 // The closest hit along o + t d, t in (tmin, tmax): the BVH, then the
@@ -700,7 +795,8 @@ MYPBR_DEV bool walk_node(const DeviceScene& S, WalkState& W, int* stack) {
     const float tmin = W.tmin;
     HitInfo& h = W.h;
     const float4* n = S.bvh + 4 * W.node;
-    float4 a0 = ldg4(n), a1 = ldg4(n + 1), c0 = ldg4(n + 2), c1 = ldg4(n + 3);
+    const Float8 na = ldg8(n), nc = ldg8(n + 2);
+    const float4 a0 = na.a, a1 = na.b, c0 = nc.a, c1 = nc.b;
     // slab tests of both children against (tmin, best)
     float lx0 = fmaf(a0.x, inv.x, oi.x), hx0 = fmaf(a1.x, inv.x, oi.x);
     float ly0 = fmaf(a0.y, inv.y, oi.y), hy0 = fmaf(a1.y, inv.y, oi.y);
@@ -725,25 +821,9 @@ MYPBR_DEV bool walk_node(const DeviceScene& S, WalkState& W, int* stack) {
         if (!(hit && cnt > 0))
             continue;
         for (int k = 0; k < cnt; k++) {
-            uint32_t ref = __ldg(S.leaf_refs + first + k);
-            int kind = int(ref >> kKindShift), idx = int(ref & kIndexMask);
-            float t, b1 = 0.0f, b2 = 0.0f;
-            bool got = false;
-            if (kind == kTriangle) {
-                got = hit_triangle(S, idx, o, W.tr, tmin, h.t, t, b1, b2, W.media_key);
-            } else if (kind == kSphere) {
-                got = hit_sphere(S, idx, o, d, tmin, h.t, t);
-            } else if (kind == kQuad) {
-                got = hit_quad(S, idx, o, d, tmin, h.t, t, b1, b2);
-            } else if (kind == kMedium && W.media_key != 0) {
-                got = hit_medium(S, idx, o, d, tmin, h.t, hash_uniform(W.media_key, uint32_t(idx)), t);
-            } else if (VOX && kind == kVoxel) {
-                int mat, face;
-                got = hit_voxel_block(S, idx, o, d, tmin, h.t, t, mat, face);
-                b1 = __int_as_float(mat);
-                b2 = __int_as_float(face);
-            }
-            if (got) {
+            float t, b1, b2;
+            uint32_t ref;
+            if (hit_leaf<VOX>(S, first + k, o, d, W.tr, tmin, h.t, W.media_key, t, b1, b2, ref)) {
                 h.t = t;
                 h.b1 = b1;
                 h.b2 = b2;
@@ -834,25 +914,9 @@ template <bool ANY, bool VOX>
 MYPBR_DEV bool test_leaf(const DeviceScene& S, int first, int count, float3 o, float3 d, const TriRay& tr, float tmin,
                          uint64_t media_key, HitInfo& h) {
     for (int k = 0; k < count; k++) {
-        uint32_t ref = __ldg(S.leaf_refs + first + k);
-        int kind = int(ref >> kKindShift), idx = int(ref & kIndexMask);
-        float t, b1 = 0.0f, b2 = 0.0f;
-        bool got = false;
-        if (kind == kTriangle) {
-            got = hit_triangle(S, idx, o, tr, tmin, h.t, t, b1, b2, media_key);
-        } else if (kind == kSphere) {
-            got = hit_sphere(S, idx, o, d, tmin, h.t, t);
-        } else if (kind == kQuad) {
-            got = hit_quad(S, idx, o, d, tmin, h.t, t, b1, b2);
-        } else if (kind == kMedium && media_key != 0) {
-            got = hit_medium(S, idx, o, d, tmin, h.t, hash_uniform(media_key, uint32_t(idx)), t);
-        } else if (VOX && kind == kVoxel) {
-            int mat, face;
-            got = hit_voxel_block(S, idx, o, d, tmin, h.t, t, mat, face);
-            b1 = __int_as_float(mat);
-            b2 = __int_as_float(face);
-        }
-        if (got) {
+        float t, b1, b2;
+        uint32_t ref;
+        if (hit_leaf<VOX>(S, first + k, o, d, tr, tmin, h.t, media_key, t, b1, b2, ref)) {
             h.t = t;
             h.b1 = b1;
             h.b2 = b2;
@@ -986,7 +1050,8 @@ MYPBR_DEV bool walk_postponed(const DeviceScene& S, float3 o, float3 d, float tm
                 return false;
             }
             const float4* n = S.bvh + 4 * node;
-            float4 a0 = ldg4(n), a1 = ldg4(n + 1), c0 = ldg4(n + 2), c1 = ldg4(n + 3);
+            const Float8 na = ldg8(n), nc = ldg8(n + 2);
+            const float4 a0 = na.a, a1 = na.b, c0 = nc.a, c1 = nc.b;
             float lx0 = fmaf(a0.x, inv.x, oi.x), hx0 = fmaf(a1.x, inv.x, oi.x);
             float ly0 = fmaf(a0.y, inv.y, oi.y), hy0 = fmaf(a1.y, inv.y, oi.y);
             float lz0 = fmaf(a0.z, inv.z, oi.z), hz0 = fmaf(a1.z, inv.z, oi.z);
@@ -1177,7 +1242,8 @@ MYPBR_DEV HitInfo walk(const DeviceScene& S, float3 o, float3 d, float tmin, flo
                 break;
             }
             const float4* n = S.bvh + 4 * node;
-            float4 a0 = ldg4(n), a1 = ldg4(n + 1), c0 = ldg4(n + 2), c1 = ldg4(n + 3);
+            const Float8 na = ldg8(n), nc = ldg8(n + 2);
+            const float4 a0 = na.a, a1 = na.b, c0 = nc.a, c1 = nc.b;
             // slab tests of both children against (tmin, best)
             float lx0 = fmaf(a0.x, inv.x, oi.x), hx0 = fmaf(a1.x, inv.x, oi.x);
             float ly0 = fmaf(a0.y, inv.y, oi.y), hy0 = fmaf(a1.y, inv.y, oi.y);
@@ -1202,25 +1268,9 @@ MYPBR_DEV HitInfo walk(const DeviceScene& S, float3 o, float3 d, float tmin, flo
                 if (!(hit && cnt > 0))
                     continue;
                 for (int k = 0; k < cnt; k++) {
-                    uint32_t ref = __ldg(S.leaf_refs + first + k);
-                    int kind = int(ref >> kKindShift), idx = int(ref & kIndexMask);
-                    float t, b1 = 0.0f, b2 = 0.0f;
-                    bool got = false;
-                    if (kind == kTriangle) {
-                        got = hit_triangle(S, idx, o, tr, tmin, h.t, t, b1, b2, media_key);
-                    } else if (kind == kSphere) {
-                        got = hit_sphere(S, idx, o, d, tmin, h.t, t);
-                    } else if (kind == kQuad) {
-                        got = hit_quad(S, idx, o, d, tmin, h.t, t, b1, b2);
-                    } else if (kind == kMedium && media_key != 0) {
-                        got = hit_medium(S, idx, o, d, tmin, h.t, hash_uniform(media_key, uint32_t(idx)), t);
-                    } else if (VOX && kind == kVoxel) {
-                        int mat, face;
-                        got = hit_voxel_block(S, idx, o, d, tmin, h.t, t, mat, face);
-                        b1 = __int_as_float(mat);
-                        b2 = __int_as_float(face);
-                    }
-                    if (got) {
+                    float t, b1, b2;
+                    uint32_t ref;
+                    if (hit_leaf<VOX>(S, first + k, o, d, tr, tmin, h.t, media_key, t, b1, b2, ref)) {
                         h.t = t;
                         h.b1 = b1;
                         h.b2 = b2;

@@ -198,16 +198,16 @@ MYPBR_DEV float table_one_minus_E(const DeviceScene& S, float c, float alpha) {
     int i = min(int(x), 30), j = min(int(y), 30);
     float tx = x - i, ty = y - j;
     const float* e = S.ggx_e;
-    float lo = (1.0f - tx) * e[j * 32 + i] + tx * e[j * 32 + i + 1];
-    float hi = (1.0f - tx) * e[(j + 1) * 32 + i] + tx * e[(j + 1) * 32 + i + 1];
-    return (1.0f - ty) * lo + ty * hi;
+    float lo = fmaf(1.0f - tx, e[j * 32 + i], tx * e[j * 32 + i + 1]);
+    float hi = fmaf(1.0f - tx, e[(j + 1) * 32 + i], tx * e[(j + 1) * 32 + i + 1]);
+    return fmaf(1.0f - ty, lo, ty * hi);
 }
 MYPBR_DEV float table_E(const DeviceScene& S, float c, float alpha) { return 1.0f - table_one_minus_E(S, c, alpha); }
 MYPBR_DEV float table_one_minus_Eavg(const DeviceScene& S, float alpha) {
     float y = clampf(sqrtf(alpha), 0.0f, 1.0f) * 31.0f;
     int j = min(int(y), 30);
     float ty = y - j;
-    return (1.0f - ty) * S.ggx_eavg[j] + ty * S.ggx_eavg[j + 1];
+    return fmaf(ty, S.ggx_eavg[j + 1], (1.0f - ty) * S.ggx_eavg[j]);
 }
 MYPBR_DEV float table_Eavg(const DeviceScene& S, float alpha) { return 1.0f - table_one_minus_Eavg(S, alpha); }
 // microfacet.h:341-373
@@ -399,7 +399,7 @@ struct Pdf {
 #pragma unroll
         for (int k = 0; k < 3; k++)
             if (k < n && prob[k] > 0.0f)
-                s += prob[k] * lobe[k].value(dir, unit);
+                s = fmaf(prob[k], lobe[k].value(dir, unit), s);
         return s;
     }
     MYPBR_DEV float3 generate(Rng& g) const {
@@ -708,8 +708,8 @@ MYPBR_DEV float3 eval_inner(const DeviceScene& S, const DevMaterial& m, float3 r
                 return f3(0.0f);
             float3 h = normalize(wo + wi);
             Ggx d{alpha};
-            return metal_fresnel_at(m, dot(wi, h)) * (d.D(h) * d.G(wo, wi) / (4.0f * wo.z)) +
-                   ms_fresnel_avg(S, mat_vec(m, 10), alpha) * ms_eval(S, wo.z, wi.z, alpha);
+            return weigh(ms_fresnel_avg(S, mat_vec(m, 10), alpha), ms_eval(S, wo.z, wi.z, alpha),
+                         metal_fresnel_at(m, dot(wi, h)), d.D(h) * d.G(wo, wi) / (4.0f * wo.z));
         }
         case kDielectric: {  // material.h:244-249
             if (m.p[1] == 0.0f)
@@ -964,11 +964,11 @@ MYPBR_DEV float member_pdf(const DeviceScene& S, const DevMember& mb, float3 o, 
     // triangle
     TriRay tr = make_tri_ray(d);
     float t, b1, b2;
-    if (!hit_triangle<false>(S, mb.index, o, tr, 0.001f, 3.0e38f, t, b1, b2))
-        return 0.0f;
     const float4* tp = S.tris + 3 * mb.index;
-    float3 v0 = f3(ldg4(tp));
-    float3 c = cross(f3(ldg4(tp + 1)) - v0, f3(ldg4(tp + 2)) - v0);
+    const float3 v0 = f3(ldg4(tp)), v1 = f3(ldg4(tp + 1)), v2 = f3(ldg4(tp + 2));
+    if (!hit_triangle<false>(S, mb.index, v0, v1, v2, o, tr, 0.001f, 3.0e38f, t, b1, b2))
+        return 0.0f;
+    float3 c = cross(v1 - v0, v2 - v0);
     float area = 0.5f * length(c);
     float d2 = t * t * len2(d);
     float cosine = fabsf(dot(d, normalize(c))) * rsqrtf(len2(d));

@@ -130,6 +130,8 @@ int guide_train(mypbr_gpu_scene* G, int steps, int batch_tiles, float lr, cudaSt
 // (1st to 99th percentile per axis, plus a margin) and re-expresses the
 // records in it. Synchronises the stream once.
 int guide_fit_box(mypbr_gpu_scene* G, cudaStream_t st);
+// The walk's leaf records (dev_scene.cuh's pack_leaf) for the scene's leaf references, on the device.
+int build_leaves(mypbr_gpu_scene* G);
 // The binary tree's device nodes collapsed to four children per node (walk_tree4's layout); depth: deepest level.
 void collapse_to_4(const std::vector<float4>& bin, std::vector<float4>& out, int& depth);
 // The binary tree collapsed to 8 children per node with quantised child boxes

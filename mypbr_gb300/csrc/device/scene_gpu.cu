@@ -737,6 +737,9 @@ int create_scene(const mypbr_flat_scene* Fp, mypbr_gpu_scene** out) {
         D.sun_radiance = make_float3(float(F.sun.irradiance[0] / omega), float(F.sun.irradiance[1] / omega),
                                      float(F.sun.irradiance[2] / omega));
     }
+    D.leaf_tails = F.triangle_count > 0 || F.quad_count > 0;
+    if (int st = build_leaves(&G); st != MYPBR_OK)
+        return fail_cleanup(st);
     G.material_count = F.material_count;
     D.use_sky = F.use_sky;
     D.background = make_float3(float(F.background[0]), float(F.background[1]), float(F.background[2]));
