@@ -287,28 +287,33 @@ struct DevArr {
     }
 };
 
-__global__ void k_pack_leaves(DeviceScene S, int n, float4* out) {
+__global__ void k_pack_leaves(DeviceScene S, const uint32_t* refs, int n, float4* out) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
-        pack_leaf(S, S.leaf_refs[k], out + 4 * size_t(k));
+        pack_leaf(S, refs[k], out + 4 * size_t(k));
 }
 
 }  // namespace
 
-int build_leaves(mypbr_gpu_scene* G) {
-    const int n = int(G->leaf_ref_count);
-    G->dev.leaves = nullptr;
-    if (n == 0)
-        return MYPBR_OK;
+int pack_leaves(mypbr_gpu_scene* G, const uint32_t* refs, int n, float4*& out) {
     DevArr<float4> leaves;
     int s = leaves.alloc(4 * size_t(n));
     if (s != MYPBR_OK)
         return s;
-    k_pack_leaves<<<std::min((n + 255) / 256, G->sm_count * 16), 256>>>(G->dev, n, leaves.p);
+    k_pack_leaves<<<std::max(1, std::min((n + 255) / 256, G->sm_count * 16)), 256>>>(G->dev, refs, n, leaves.p);
     MYPBR_CUDA(cudaGetLastError());
     MYPBR_CUDA(cudaStreamSynchronize(nullptr));
     G->allocations.push_back(leaves.p);
-    G->dev.leaves = leaves.p;
+    out = leaves.p;
     leaves.p = nullptr;
+    return MYPBR_OK;
+}
+
+int build_leaves(mypbr_gpu_scene* G) {
+    float4* leaves = nullptr;
+    if (G->leaf_ref_count > 0)
+        if (int s = pack_leaves(G, G->dev.leaf_refs, int(G->leaf_ref_count), leaves); s != MYPBR_OK)
+            return s;
+    G->dev.leaves = leaves;
     return MYPBR_OK;
 }
 
@@ -406,11 +411,9 @@ extern "C" int mypbr_gpu_scene_rebuild_bvh(mypbr_gpu_scene* G, int32_t method, m
         G->allocations.push_back(wide8_p);
     }
     const uint32_t* host_refs = D.leaf_refs;
-    const float4* host_leaves = D.leaves;
     D.leaf_refs = sorted_refs.p;
     if ((s = build_leaves(G)) != MYPBR_OK) {  // the host tree stays
         D.leaf_refs = host_refs;
-        D.leaves = host_leaves;
         nodes.p = nullptr;  // freed with the handle
         sorted_refs.p = nullptr;
         return s;

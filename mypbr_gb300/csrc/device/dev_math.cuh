@@ -64,6 +64,7 @@ MYPBR_HD float avg3(float3 a) { return (a.x + a.y + a.z) * (1.0f / 3.0f); }
 MYPBR_HD float luminance(float3 c) { return 0.2126f * c.x + 0.7152f * c.y + 0.0722f * c.z; }
 MYPBR_HD float clampf(float x, float a, float b) { return fminf(fmaxf(x, a), b); }
 MYPBR_HD bool nonzero(float3 c) { return c.x > 0.0f || c.y > 0.0f || c.z > 0.0f; }
+MYPBR_HD bool is_zero(float3 c) { return c.x == 0.0f && c.y == 0.0f && c.z == 0.0f; }
 MYPBR_DEV float3 reflect(float3 v, float3 n) { return v - 2.0f * dot(v, n) * n; }
 // Refraction of unit uv through unit normal n with ratio eta_i / eta_t (vec3.h:324-329).
 MYPBR_DEV float3 refract(float3 uv, float3 n, float ratio) {

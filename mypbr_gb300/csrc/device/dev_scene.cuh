@@ -40,6 +40,7 @@ struct DevVoxelModel {
 
 constexpr int kBvhStack = 64;
 constexpr int kVoxelBlockMax = 64;  // cells along each side of a voxel block, at most
+constexpr size_t kFewEmitters = 16;  // shadow rays test up to so many emitting surfaces one by one
 constexpr uint32_t kKindShift = 29;
 constexpr uint32_t kIndexMask = (1u << kKindShift) - 1;
 
@@ -102,6 +103,9 @@ struct DeviceScene {
     int has_media;       // media or height fog present (free-flight sampling needs keys)
     int has_alpha;       // some triangle carries an alpha mask (its coverage test needs keys)
     int has_voxels;      // voxel blocks among the BVH's primitives
+    const float4* emitters;  // leaf records of every surface that can emit, where they are few (else emitter_count is -1)
+    int emitter_count;
+    int dark_sky;        // a ray that escapes meets no light at all
     int has_emitters;    // some hittable surface can emit (diffuse light or emissive texture)
     int has_clear_glass; // some hittable surface lets shadows through (smooth dielectric)
     const uint8_t* mat_class;  // shading class of each material
@@ -192,10 +196,13 @@ MYPBR_DEV float3 xf_normal(const XformRef& X, float3 n) {
 // Improvements for Ray/Sphere Intersection", Ray Tracing Gems 2019, ch. 7),
 // which keeps FP32 accurate for large spheres such as a ground of radius 1000.
 // Returns the nearest root in (tmin, tmax), the reference's rule (sphere.h:23-52).
+// FIXED: every sum of products in a stated order (the walks of LaneWalk, whose
+// results must be those of the other walks to the last bit).
+template <bool FIXED = false>
 MYPBR_DEV bool sphere_root(float3 c, float r, float3 o, float3 d, float tmin, float tmax, float& t) {
-    float a = dot(d, d);
+    float a = FIXED ? dot_x(d, d) : dot(d, d);
     float3 f = o - c;
-    float b = -dot(f, d);  // = dot(d, c - o)
+    float b = -(FIXED ? dot_x(f, d) : dot(f, d));  // = dot(d, c - o)
     float3 l = f + (b / a) * d;  // offset of the closest point of the line from the centre
     const float r2 = __fmul_rn(r, r);  // rounded once, for both differences below
     float disc = a * (r2 - dot_x(l, l));
@@ -221,13 +228,14 @@ MYPBR_DEV bool sphere_root(float3 c, float r, float3 o, float3 d, float tmin, fl
 }
 
 // A sphere (centre, radius) under transform xf (below 0: none).
+template <bool FIXED>
 MYPBR_DEV bool hit_sphere(const DeviceScene& S, float3 c, float r, int xf, float3 o, float3 d, float tmin, float tmax,
                           float& t) {
     if (xf < 0)
-        return sphere_root(c, r, o, d, tmin, tmax, t);
+        return sphere_root<FIXED>(c, r, o, d, tmin, tmax, t);
     XformRef X;
     load_xform(S, xf, X);
-    return sphere_root(c, r, xf_ipoint(X, o), xf_ivec(X, d), tmin, tmax, t);
+    return sphere_root<FIXED>(c, r, xf_ipoint(X, o), xf_ivec(X, d), tmin, tmax, t);
 }
 
 // Plane t, then the parallelogram test 0 <= a, b <= 1 (quad.h:30-62).
@@ -259,6 +267,7 @@ MYPBR_DEV bool hit_quad(const DeviceScene& S, int i, float3 o, float3 d, float t
 // Per-ray constants of the watertight ray/triangle test (Woop, Benthin and
 // Wald, "Watertight Ray/Triangle Intersection", JCGT 2013).
 struct TriRay {
+    static constexpr bool kFixed = false;
     int kx, ky, kz;
     float sx, sy, sz;
 };
@@ -279,6 +288,15 @@ MYPBR_DEV TriRay make_tri_ray(float3 d) {
     r.sz = 1.0f / dz;
     return r;
 }
+
+// The same made anew for each triangle met: for walks that hold too much in
+// registers already to keep six more for rays that may meet none.
+struct LazyTriRay {
+    static constexpr bool kFixed = true;
+    float3 d;
+};
+MYPBR_DEV const TriRay& tri_ray(const TriRay& r) { return r; }
+MYPBR_DEV TriRay tri_ray(const LazyTriRay& r) { return make_tri_ray(r.d); }
 
 // Barycentrics b1, b2 are the weights of v1 and v2, the reference's (u, v)
 // without texture coordinates (mesh.h:72-79).
@@ -442,7 +460,7 @@ MYPBR_DEV bool hit_medium(const DeviceScene& S, int i, float3 o, float3 d, float
     float t0 = fmaxf(a, tmin), t1 = fminf(b, tmax);
     if (t0 >= t1)
         return false;
-    float len = length(d);
+    float len = sqrtf(dot_x(d, d));
     float dist = -logf(1.0f - xi) / density;
     if (dist > (t1 - t0) * len)
         return false;
@@ -681,12 +699,11 @@ MYPBR_DEV void pack_leaf(const DeviceScene& S, uint32_t ref, float4* out) {
         out[k] = q[k];
 }
 
-// The primitive of leaf slot `slot` against the ray; on a hit nearer than
+// The primitive of the leaf record at p against the ray; on a hit nearer than
 // tmax its t, coordinates and reference.
-template <bool VOX>
-MYPBR_DEV bool hit_leaf(const DeviceScene& S, int slot, float3 o, float3 d, const TriRay& tr, float tmin, float tmax,
+template <bool VOX, class Tri>
+MYPBR_DEV bool hit_record(const DeviceScene& S, const float4* p, float3 o, float3 d, const Tri& tr, float tmin, float tmax,
                         uint64_t media_key, float& t, float& b1, float& b2, uint32_t& ref) {
-    const float4* p = S.leaves + 4 * size_t(slot);
     const Float8 q = ldg8(p);
     float2 tail = make_float2(0.0f, 0.0f);
     if (S.leaf_tails)  // under way together with the first half
@@ -695,10 +712,10 @@ MYPBR_DEV bool hit_leaf(const DeviceScene& S, int slot, float3 o, float3 d, cons
     const int kind = int(ref >> kKindShift), idx = int(ref & kIndexMask);
     b1 = b2 = 0.0f;
     if (kind == kTriangle)
-        return hit_triangle(S, idx, f3(q.a), f3(q.b), f3(q.b.w, tail.x, tail.y), o, tr, tmin, tmax, t, b1, b2,
+        return hit_triangle(S, idx, f3(q.a), f3(q.b), f3(q.b.w, tail.x, tail.y), o, tri_ray(tr), tmin, tmax, t, b1, b2,
                             media_key);
     if (kind == kSphere)
-        return hit_sphere(S, f3(q.a), q.b.x, __float_as_int(q.b.y), o, d, tmin, tmax, t);
+        return hit_sphere<Tri::kFixed>(S, f3(q.a), q.b.x, __float_as_int(q.b.y), o, d, tmin, tmax, t);
     if (kind == kQuad) {
         const Float8 e = ldg8(p + 2);
         return hit_quad(f3(q.a), f3(q.b), f3(e.a), f3(e.b), f3(q.b.w, e.a.w, e.b.w), o, d, tmin, tmax, t, b1, b2);
@@ -718,6 +735,32 @@ MYPBR_DEV bool hit_leaf(const DeviceScene& S, int slot, float3 o, float3 d, cons
     return false;
 }
 
+template <bool VOX, class Tri>
+MYPBR_DEV bool hit_leaf(const DeviceScene& S, int slot, float3 o, float3 d, const Tri& tr, float tmin, float tmax,
+                        uint64_t media_key, float& t, float& b1, float& b2, uint32_t& ref) {
+    return hit_record<VOX>(S, S.leaves + 4 * size_t(slot), o, d, tr, tmin, tmax, media_key, t, b1, b2, ref);
+}
+
+// The nearest of the scene's emitting surfaces along the ray.
+MYPBR_DEV HitInfo nearest_emitter(const DeviceScene& S, float3 o, float3 d, float tmin, uint64_t media_key) {
+    HitInfo h;
+    h.prim = kMiss;
+    h.t = 3.0e38f;
+    h.b1 = h.b2 = 0.0f;
+    const TriRay tr = make_tri_ray(d);
+    for (int k = 0; k < S.emitter_count; k++) {
+        float t, b1, b2;
+        uint32_t ref;
+        if (hit_record<false>(S, S.emitters + 4 * k, o, d, tr, tmin, h.t, media_key, t, b1, b2, ref)) {
+            h.t = t;
+            h.b1 = b1;
+            h.b2 = b2;
+            h.prim = ref;
+        }
+    }
+    return h;
+}
+
 MYPBR_DEV float safe_inv(float x) { return fabsf(x) > 1e-30f ? 1.0f / x : copysignf(1e30f, x); }
 
 // The closest hit along o + t d, t in (tmin, tmax): the BVH, then the
@@ -728,148 +771,42 @@ MYPBR_DEV float safe_inv(float x) { return fabsf(x) > 1e-30f ? 1.0f / x : copysi
 // leave that code out, and with it its registers).
 // WALK: which walk. 0: the binary tree, leaves tested as soon as they are
 // met; 1: the 4-wide tree (S.bvh4); 2: the binary tree with leaves postponed
-// until every lane of the warp holds one (walk_postponed).
-enum : int { kWalkBinary = 0, kWalkWide = 1, kWalkPostponed = 2, kWalkWide8 = 3 };
-template <bool ANY, bool VOX = true, int WALK = kWalkBinary>
-MYPBR_DEV HitInfo walk(const DeviceScene& S, float3 o, float3 d, float tmin, float tmax, uint64_t media_key);
+// until every lane of the warp holds one (walk_postponed); 3: the 8-wide tree
+// with quantised boxes; 4 and 5: the binary walk with leaves at once and
+// postponed, in kernels whose lanes take new rays (LaneWalk).
+enum : int { kWalkBinary = 0, kWalkWide = 1, kWalkPostponed = 2, kWalkWide8 = 3, kWalkLanes = 4, kWalkLanesPostponed = 5 };
+template <bool ANY, bool VOX, int WALK>
+MYPBR_DEV bool walk(const DeviceScene& S, float3 o, float3 d, float tmin, uint64_t media_key, HitInfo& h);
 
 template <bool VOX = true, int WALK = kWalkBinary>
 MYPBR_DEV HitInfo closest_hit(const DeviceScene& S, float3 o, float3 d, float tmin, float tmax, uint64_t media_key) {
-    return walk<false, VOX, WALK>(S, o, d, tmin, tmax, media_key);
-}
-
-// Whether anything at all lies along o + t d, t in (tmin, tmax): the walk stops
-// at the first primitive it hits. For shadow rays in scenes where nothing
-// hittable can emit, this is all the reference's closest-hit query decides.
-template <bool VOX = true, int WALK = kWalkBinary>
-MYPBR_DEV bool any_hit(const DeviceScene& S, float3 o, float3 d, float tmin, float tmax, uint64_t media_key) {
-    return walk<true, VOX, WALK>(S, o, d, tmin, tmax, media_key).prim != 0xffffffffu;
-}
-
-// A ray's BVH walk, advanced one interior node at a time (walk_node), so that
-// a persistent kernel can give a lane a new ray as soon as its last one is
-// done instead of waiting for the slowest lane of its warp.
-struct WalkState {
-    float3 o, d, inv, oi;
-    TriRay tr;
-    float tmin;
-    uint64_t media_key;
     HitInfo h;
-    int node, sp, visits;
-};
-// The walk's stack lives beside its state (a kBvhStack-entry local array),
-// so that the state's scalars can stay in registers.
-
-MYPBR_DEV void walk_init(const DeviceScene& S, WalkState& W, float3 o, float3 d, float tmin, float tmax,
-                         uint64_t media_key) {
-    W.o = o;
-    W.d = d;
-    W.tmin = tmin;
-    W.media_key = media_key;
-    W.h.prim = kMiss;
-    W.h.t = tmax;
-    W.h.b1 = W.h.b2 = 0.0f;
-    W.inv = f3(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
-    W.oi = -1.0f * (o * W.inv);
-    W.tr = make_tri_ray(d);
-    W.node = 0;
-    W.sp = S.has_bvh ? 0 : -1;  // -1: nothing (left) to walk
-    W.visits = 0;
+    h.prim = kMiss;
+    h.t = tmax;
+    h.b1 = h.b2 = 0.0f;
+    walk<false, VOX, WALK>(S, o, d, tmin, media_key, h);
+    return h;
 }
 
-// One interior node: slab tests of both children, the primitives of child
-// leaves, then the next node. Returns false once the walk is over (or, with
-// ANY, a hit was found).
-template <bool ANY, bool VOX>
-MYPBR_DEV bool walk_node(const DeviceScene& S, WalkState& W, int* stack) {
-    if (W.sp < 0)
-        return false;
-    // A tree walk enters each interior node at most once; the cap only guards
-    // against a malformed tree, which it reports instead of spinning.
-    if (++W.visits > S.bvh_node_count + 1) {
-        atomicCAS(S.error, 0, 1);
-        W.sp = -1;
-        return false;
-    }
-    const float3 o = W.o, d = W.d, inv = W.inv, oi = W.oi;
-    const float tmin = W.tmin;
-    HitInfo& h = W.h;
-    const float4* n = S.bvh + 4 * W.node;
-    const Float8 na = ldg8(n), nc = ldg8(n + 2);
-    const float4 a0 = na.a, a1 = na.b, c0 = nc.a, c1 = nc.b;
-    // slab tests of both children against (tmin, best)
-    float lx0 = fmaf(a0.x, inv.x, oi.x), hx0 = fmaf(a1.x, inv.x, oi.x);
-    float ly0 = fmaf(a0.y, inv.y, oi.y), hy0 = fmaf(a1.y, inv.y, oi.y);
-    float lz0 = fmaf(a0.z, inv.z, oi.z), hz0 = fmaf(a1.z, inv.z, oi.z);
-    float n0 = fmaxf(fmaxf(fminf(lx0, hx0), fminf(ly0, hy0)), fmaxf(fminf(lz0, hz0), tmin));
-    float f0 = fminf(fminf(fmaxf(lx0, hx0), fmaxf(ly0, hy0)), fminf(fmaxf(lz0, hz0), h.t));
-    float lx1 = fmaf(c0.x, inv.x, oi.x), hx1 = fmaf(c1.x, inv.x, oi.x);
-    float ly1 = fmaf(c0.y, inv.y, oi.y), hy1 = fmaf(c1.y, inv.y, oi.y);
-    float lz1 = fmaf(c0.z, inv.z, oi.z), hz1 = fmaf(c1.z, inv.z, oi.z);
-    float n1 = fmaxf(fmaxf(fminf(lx1, hx1), fminf(ly1, hy1)), fmaxf(fminf(lz1, hz1), tmin));
-    float f1 = fminf(fminf(fmaxf(lx1, hx1), fmaxf(ly1, hy1)), fminf(fmaxf(lz1, hz1), h.t));
-    // A small relative widening keeps FP32 slab tests conservative
-    bool h0 = n0 <= f0 * 1.00000024f + 1e-30f;
-    bool h1 = n1 <= f1 * 1.00000024f + 1e-30f;
-    int i0 = __float_as_int(a0.w), k0 = __float_as_int(a1.w);
-    int i1 = __float_as_int(c0.w), k1 = __float_as_int(c1.w);
-#pragma unroll
-    for (int side = 0; side < 2; side++) {
-        bool hit = side == 0 ? h0 : h1;
-        int cnt = side == 0 ? k0 : k1;
-        int first = side == 0 ? i0 : i1;
-        if (!(hit && cnt > 0))
-            continue;
-        for (int k = 0; k < cnt; k++) {
-            float t, b1, b2;
-            uint32_t ref;
-            if (hit_leaf<VOX>(S, first + k, o, d, W.tr, tmin, h.t, W.media_key, t, b1, b2, ref)) {
-                h.t = t;
-                h.b1 = b1;
-                h.b2 = b2;
-                h.prim = ref;
-                if (ANY) {
-                    W.sp = -1;
-                    return false;
-                }
-            }
-        }
-    }
-    h0 = h0 && k0 == 0;
-    h1 = h1 && k1 == 0;
-    if (h0 && h1) {
-        bool first0 = n0 <= n1;
-        if (W.sp == kBvhStack) {  // deeper than the host-checked depth: report, stop
-            atomicCAS(S.error, 0, 2);
-            W.sp = -1;
-            return false;
-        }
-        stack[W.sp++] = first0 ? i1 : i0;
-        W.node = first0 ? i0 : i1;
-    } else if (h0) {
-        W.node = i0;
-    } else if (h1) {
-        W.node = i1;
-    } else {
-        if (W.sp == 0) {
-            W.sp = -1;
-            return false;
-        }
-        W.node = stack[--W.sp];
-    }
-    return true;
+// Whether anything but primitive `skip` lies along o + t d, t in (tmin,
+// tmax): the walk stops at the first primitive it hits. For shadow rays that
+// need no more than whether something dark is in the way, this is all the
+// reference's closest-hit query decides.
+template <bool VOX = true, int WALK = kWalkBinary>
+MYPBR_DEV bool any_hit(const DeviceScene& S, float3 o, float3 d, float tmin, float tmax, uint64_t media_key,
+                       uint32_t skip = kMiss) {
+    HitInfo h;
+    h.prim = skip;
+    h.t = tmax;
+    h.b1 = h.b2 = 0.0f;
+    return walk<true, VOX, WALK>(S, o, d, tmin, media_key, h);
 }
 
-// The unbounded objects beside the BVH, after the walk.
+// The unbounded objects beside the BVH, after the walk: the ground
+// (plane.h:17-34) and height fog (medium.h:352-381). True when ANY and one
+// was met.
 template <bool ANY>
-MYPBR_DEV void walk_unbounded(const DeviceScene& S, WalkState& W) {
-    const float3 o = W.o, d = W.d;
-    const float tmin = W.tmin;
-    const uint64_t media_key = W.media_key;
-    HitInfo& h = W.h;
-    if (ANY && h.prim != kMiss)
-        return;
-    // The ground (plane.h:17-34) and height fog (medium.h:352-381) beside the BVH
+MYPBR_DEV bool walk_unbounded(const DeviceScene& S, float3 o, float3 d, float tmin, uint64_t media_key, HitInfo& h) {
     for (int k = 0; k < S.unbounded_count; k++) {
         DevUnbounded ub = S.unbounded[k];
         if (ub.kind == 0) {
@@ -877,13 +814,13 @@ MYPBR_DEV void walk_unbounded(const DeviceScene& S, WalkState& W) {
                 continue;
             float t = (ub.height - o.y) / d.y;
             if (t > tmin && t < h.t) {
+                if (ANY)
+                    return true;
                 h.t = t;
                 h.prim = (uint32_t(kGround) << kKindShift) | uint32_t(k);
-                if (ANY)
-                    return;
             }
         } else if (media_key != 0) {
-            float len = length(d);
+            float len = sqrtf(dot_x(d, d));
             float kk = d.y / ub.scale_height;
             float start = ub.density * len * expf(-(o.y + tmin * d.y - ub.height) / ub.scale_height);
             if (!(start > 0.0f))
@@ -899,30 +836,34 @@ MYPBR_DEV void walk_unbounded(const DeviceScene& S, WalkState& W) {
                 t = tmin - logf(x) / kk;
             }
             if (t < h.t && isfinite(t)) {
+                if (ANY)
+                    return true;
                 h.t = t;
                 h.prim = (uint32_t(kHeightFog) << kKindShift) | uint32_t(k);
-                if (ANY)
-                    return;
             }
         }
     }
+    return false;
 }
 
 // The primitives of one leaf (count refs from first) against the ray; true
-// when ANY and one was hit.
-template <bool ANY, bool VOX>
-MYPBR_DEV bool test_leaf(const DeviceScene& S, int first, int count, float3 o, float3 d, const TriRay& tr, float tmin,
+// when ANY and one other than h.prim was hit.
+template <bool ANY, bool VOX, class Tri>
+MYPBR_DEV bool test_leaf(const DeviceScene& S, int first, int count, float3 o, float3 d, const Tri& tr, float tmin,
                          uint64_t media_key, HitInfo& h) {
     for (int k = 0; k < count; k++) {
         float t, b1, b2;
         uint32_t ref;
         if (hit_leaf<VOX>(S, first + k, o, d, tr, tmin, h.t, media_key, t, b1, b2, ref)) {
+            if (ANY) {
+                if (ref != h.prim)
+                    return true;
+                continue;
+            }
             h.t = t;
             h.b1 = b1;
             h.b2 = b2;
             h.prim = ref;
-            if (ANY)
-                return true;
         }
     }
     return false;
@@ -1106,6 +1047,125 @@ MYPBR_DEV bool walk_postponed(const DeviceScene& S, float3 o, float3 d, float tm
     return false;
 }
 
+// A walk of the binary tree as a lane's state, advanced by a whole warp, so
+// that a kernel can give a lane its next ray as soon as its last one is done
+// (k_extend_lanes and k_shadow_lanes in render.cu).
+struct LaneWalk {
+    float3 o, d, inv, oi;
+    float tmin;
+    uint64_t media_key;
+    HitInfo h;
+    int node, leaf, sp, visits;
+    bool found;  // an ANY walk met something
+    MYPBR_DEV bool done() const { return node == kWalkDone && leaf == 0; }
+    MYPBR_DEV void stop() {
+        node = kWalkDone;
+        leaf = 0;
+    }
+    // skip: the primitive that an ANY walk ignores (kMiss: none)
+    MYPBR_DEV void start(const DeviceScene& S, float3 from, float3 dir, float t_min, float t_max, uint64_t key,
+                         uint32_t skip = kMiss) {
+        o = from;
+        d = dir;
+        tmin = t_min;
+        media_key = key;
+        found = false;
+        h.prim = skip;
+        h.t = t_max;
+        h.b1 = h.b2 = 0.0f;
+        inv = f3(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
+        oi = -1.0f * (o * inv);
+        node = S.has_bvh ? 0 : kWalkDone;
+        leaf = sp = visits = 0;
+    }
+    // POSTPONED: inner nodes until every lane of the warp that walks holds a
+    // leaf or is done, then the leaves. Else nodes, each with its leaves at
+    // once, until fewer than `least` lanes of the warp walk. Primitives are
+    // tested in the order of walk_postponed or walk_binary, so that of two
+    // hits at the same t the same one stays. With ANY a hit ends the walk.
+    template <bool ANY, bool VOX, bool POSTPONED>
+    MYPBR_DEV void advance(const DeviceScene& S, int* stack, int least) {
+        while (node >= 0) {
+            // A tree walk enters each inner node at most once; the cap only
+            // guards against a malformed tree, which it reports.
+            if (++visits > S.bvh_node_count + 1) {
+                atomicCAS(S.error, 0, 1);
+                stop();
+                break;
+            }
+            const float4* n = S.bvh + 4 * node;
+            const Float8 na = ldg8(n), nc = ldg8(n + 2);
+            const float4 a0 = na.a, a1 = na.b, c0 = nc.a, c1 = nc.b;
+            float lx0 = fmaf(a0.x, inv.x, oi.x), hx0 = fmaf(a1.x, inv.x, oi.x);
+            float ly0 = fmaf(a0.y, inv.y, oi.y), hy0 = fmaf(a1.y, inv.y, oi.y);
+            float lz0 = fmaf(a0.z, inv.z, oi.z), hz0 = fmaf(a1.z, inv.z, oi.z);
+            float n0 = fmaxf(fmaxf(fminf(lx0, hx0), fminf(ly0, hy0)), fmaxf(fminf(lz0, hz0), tmin));
+            float f0 = fminf(fminf(fmaxf(lx0, hx0), fmaxf(ly0, hy0)), fminf(fmaxf(lz0, hz0), h.t));
+            float lx1 = fmaf(c0.x, inv.x, oi.x), hx1 = fmaf(c1.x, inv.x, oi.x);
+            float ly1 = fmaf(c0.y, inv.y, oi.y), hy1 = fmaf(c1.y, inv.y, oi.y);
+            float lz1 = fmaf(c0.z, inv.z, oi.z), hz1 = fmaf(c1.z, inv.z, oi.z);
+            float n1 = fmaxf(fmaxf(fminf(lx1, hx1), fminf(ly1, hy1)), fmaxf(fminf(lz1, hz1), tmin));
+            float f1 = fminf(fminf(fmaxf(lx1, hx1), fmaxf(ly1, hy1)), fminf(fmaxf(lz1, hz1), h.t));
+            bool h0 = n0 <= f0 * 1.00000024f + 1e-30f;
+            bool h1 = n1 <= f1 * 1.00000024f + 1e-30f;
+            int k0 = __float_as_int(a1.w), k1 = __float_as_int(c1.w);
+            int e0 = __float_as_int(a0.w), e1 = __float_as_int(c0.w);
+            if constexpr (POSTPONED) {
+                e0 = k0 > 0 ? ~((e0 << 4) | k0) : e0;
+                e1 = k1 > 0 ? ~((e1 << 4) | k1) : e1;
+            } else {
+                if ((h0 && k0 > 0 && test_leaf<ANY, VOX>(S, e0, k0, o, d, LazyTriRay{d}, tmin, media_key, h)) ||
+                    (h1 && k1 > 0 && test_leaf<ANY, VOX>(S, e1, k1, o, d, LazyTriRay{d}, tmin, media_key, h))) {
+                    found = true;
+                    stop();
+                    break;
+                }
+                h0 = h0 && k0 == 0;
+                h1 = h1 && k1 == 0;
+            }
+            if (h0 && h1) {
+                bool first0 = n0 <= n1;
+                if (sp == kBvhStack) {  // deeper than the host-checked depth
+                    atomicCAS(S.error, 0, 2);
+                    stop();
+                    break;
+                }
+                stack[sp++] = first0 ? e1 : e0;
+                node = first0 ? e0 : e1;
+            } else if (h0) {
+                node = e0;
+            } else if (h1) {
+                node = e1;
+            } else {
+                node = sp > 0 ? stack[--sp] : kWalkDone;
+            }
+            if constexpr (POSTPONED) {
+                if (node < 0 && node != kWalkDone && leaf == 0) {
+                    leaf = node;
+                    node = sp > 0 ? stack[--sp] : kWalkDone;
+                }
+                if (__all_sync(__activemask(), leaf < 0 || node == kWalkDone))
+                    break;
+            } else if (__popc(__activemask()) < least) {
+                break;
+            }
+        }
+        while (POSTPONED && leaf < 0) {
+            const int packed = ~leaf;
+            if (test_leaf<ANY, VOX>(S, packed >> 4, packed & 15, o, d, LazyTriRay{d}, tmin, media_key, h)) {
+                found = true;
+                stop();
+                break;
+            }
+            leaf = 0;
+            if (node < 0 && node != kWalkDone) {
+                leaf = node;
+                node = sp > 0 ? stack[--sp] : kWalkDone;
+            }
+        }
+    }
+};
+
 // The walk over the 8-wide tree with quantised boxes (96-byte nodes, the
 // layout collapse_to_8q writes). Per node the eight child planes are decoded
 // from bytes as t = q (s / d) + (p - o) / d per axis (one FMA each); leaves
@@ -1209,136 +1269,90 @@ MYPBR_DEV bool walk_tree8q(const DeviceScene& S, float3 o, float3 d, float tmin,
     }
 }
 
-// The whole walk in one loop (the form the per-ray kernels use; walk_node
-// above is the same step, resumable, for k_extend_pt).
-template <bool ANY, bool VOX, int WALK>
-MYPBR_DEV HitInfo walk(const DeviceScene& S, float3 o, float3 d, float tmin, float tmax, uint64_t media_key) {
-    HitInfo h;
-    h.prim = kMiss;
-    h.t = tmax;
-    h.b1 = h.b2 = 0.0f;
-    if constexpr (WALK == kWalkWide) {
-        if (S.has_bvh && walk_tree4<ANY, VOX>(S, o, d, tmin, media_key, h))
-            return h;
-    } else if constexpr (WALK == kWalkWide8) {
-        if (S.has_bvh && walk_tree8q<ANY, VOX>(S, o, d, tmin, media_key, h))
-            return h;
-    } else if constexpr (WALK == kWalkPostponed) {
-        if (S.has_bvh && walk_postponed<ANY, VOX>(S, o, d, tmin, media_key, h))
-            return h;
-    } else if (S.has_bvh) {
-        float3 inv = f3(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
-        float3 oi = -1.0f * (o * inv);
-        TriRay tr = make_tri_ray(d);
-        int stack[kBvhStack];
-        int sp = 0;
-        int node = 0;
-        // A tree walk enters each interior node at most once; the cap only
-        // guards against a malformed tree, which it reports instead of spinning.
-        int visits = 0;
-        while (true) {
-            if (++visits > S.bvh_node_count + 1) {
-                atomicCAS(S.error, 0, 1);
-                break;
-            }
-            const float4* n = S.bvh + 4 * node;
-            const Float8 na = ldg8(n), nc = ldg8(n + 2);
-            const float4 a0 = na.a, a1 = na.b, c0 = nc.a, c1 = nc.b;
-            // slab tests of both children against (tmin, best)
-            float lx0 = fmaf(a0.x, inv.x, oi.x), hx0 = fmaf(a1.x, inv.x, oi.x);
-            float ly0 = fmaf(a0.y, inv.y, oi.y), hy0 = fmaf(a1.y, inv.y, oi.y);
-            float lz0 = fmaf(a0.z, inv.z, oi.z), hz0 = fmaf(a1.z, inv.z, oi.z);
-            float n0 = fmaxf(fmaxf(fminf(lx0, hx0), fminf(ly0, hy0)), fmaxf(fminf(lz0, hz0), tmin));
-            float f0 = fminf(fminf(fmaxf(lx0, hx0), fmaxf(ly0, hy0)), fminf(fmaxf(lz0, hz0), h.t));
-            float lx1 = fmaf(c0.x, inv.x, oi.x), hx1 = fmaf(c1.x, inv.x, oi.x);
-            float ly1 = fmaf(c0.y, inv.y, oi.y), hy1 = fmaf(c1.y, inv.y, oi.y);
-            float lz1 = fmaf(c0.z, inv.z, oi.z), hz1 = fmaf(c1.z, inv.z, oi.z);
-            float n1 = fmaxf(fmaxf(fminf(lx1, hx1), fminf(ly1, hy1)), fmaxf(fminf(lz1, hz1), tmin));
-            float f1 = fminf(fminf(fmaxf(lx1, hx1), fmaxf(ly1, hy1)), fminf(fmaxf(lz1, hz1), h.t));
-            // A small relative widening keeps FP32 slab tests conservative
-            bool h0 = n0 <= f0 * 1.00000024f + 1e-30f;
-            bool h1 = n1 <= f1 * 1.00000024f + 1e-30f;
-            int i0 = __float_as_int(a0.w), k0 = __float_as_int(a1.w);
-            int i1 = __float_as_int(c0.w), k1 = __float_as_int(c1.w);
+// The binary walk, leaves tested as soon as they are met.
+template <bool ANY, bool VOX>
+MYPBR_DEV bool walk_binary(const DeviceScene& S, float3 o, float3 d, float tmin, uint64_t media_key, HitInfo& h) {
+    float3 inv = f3(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
+    float3 oi = -1.0f * (o * inv);
+    TriRay tr = make_tri_ray(d);
+    int stack[kBvhStack];
+    int sp = 0;
+    int node = 0;
+    // A tree walk enters each interior node at most once; the cap only
+    // guards against a malformed tree, which it reports instead of spinning.
+    int visits = 0;
+    while (true) {
+        if (++visits > S.bvh_node_count + 1) {
+            atomicCAS(S.error, 0, 1);
+            return false;
+        }
+        const float4* n = S.bvh + 4 * node;
+        const Float8 na = ldg8(n), nc = ldg8(n + 2);
+        const float4 a0 = na.a, a1 = na.b, c0 = nc.a, c1 = nc.b;
+        // slab tests of both children against (tmin, best)
+        float lx0 = fmaf(a0.x, inv.x, oi.x), hx0 = fmaf(a1.x, inv.x, oi.x);
+        float ly0 = fmaf(a0.y, inv.y, oi.y), hy0 = fmaf(a1.y, inv.y, oi.y);
+        float lz0 = fmaf(a0.z, inv.z, oi.z), hz0 = fmaf(a1.z, inv.z, oi.z);
+        float n0 = fmaxf(fmaxf(fminf(lx0, hx0), fminf(ly0, hy0)), fmaxf(fminf(lz0, hz0), tmin));
+        float f0 = fminf(fminf(fmaxf(lx0, hx0), fmaxf(ly0, hy0)), fminf(fmaxf(lz0, hz0), h.t));
+        float lx1 = fmaf(c0.x, inv.x, oi.x), hx1 = fmaf(c1.x, inv.x, oi.x);
+        float ly1 = fmaf(c0.y, inv.y, oi.y), hy1 = fmaf(c1.y, inv.y, oi.y);
+        float lz1 = fmaf(c0.z, inv.z, oi.z), hz1 = fmaf(c1.z, inv.z, oi.z);
+        float n1 = fmaxf(fmaxf(fminf(lx1, hx1), fminf(ly1, hy1)), fmaxf(fminf(lz1, hz1), tmin));
+        float f1 = fminf(fminf(fmaxf(lx1, hx1), fmaxf(ly1, hy1)), fminf(fmaxf(lz1, hz1), h.t));
+        // A small relative widening keeps FP32 slab tests conservative
+        bool h0 = n0 <= f0 * 1.00000024f + 1e-30f;
+        bool h1 = n1 <= f1 * 1.00000024f + 1e-30f;
+        int i0 = __float_as_int(a0.w), k0 = __float_as_int(a1.w);
+        int i1 = __float_as_int(c0.w), k1 = __float_as_int(c1.w);
 #pragma unroll
-            for (int side = 0; side < 2; side++) {
-                bool hit = side == 0 ? h0 : h1;
-                int cnt = side == 0 ? k0 : k1;
-                int first = side == 0 ? i0 : i1;
-                if (!(hit && cnt > 0))
-                    continue;
-                for (int k = 0; k < cnt; k++) {
-                    float t, b1, b2;
-                    uint32_t ref;
-                    if (hit_leaf<VOX>(S, first + k, o, d, tr, tmin, h.t, media_key, t, b1, b2, ref)) {
-                        h.t = t;
-                        h.b1 = b1;
-                        h.b2 = b2;
-                        h.prim = ref;
-                        if (ANY)
-                            return h;
-                    }
-                }
+        for (int side = 0; side < 2; side++) {
+            bool hit = side == 0 ? h0 : h1;
+            int cnt = side == 0 ? k0 : k1;
+            int first = side == 0 ? i0 : i1;
+            if (hit && cnt > 0 && test_leaf<ANY, VOX>(S, first, cnt, o, d, tr, tmin, media_key, h))
+                return true;
+        }
+        h0 = h0 && k0 == 0;
+        h1 = h1 && k1 == 0;
+        if (h0 && h1) {
+            bool first0 = n0 <= n1;
+            if (sp == kBvhStack) {  // deeper than the host-checked depth: report, stop
+                atomicCAS(S.error, 0, 2);
+                return false;
             }
-            h0 = h0 && k0 == 0;
-            h1 = h1 && k1 == 0;
-            if (h0 && h1) {
-                bool first0 = n0 <= n1;
-                if (sp == kBvhStack) {  // deeper than the host-checked depth: report, stop
-                    atomicCAS(S.error, 0, 2);
-                    break;
-                }
-                stack[sp++] = first0 ? i1 : i0;
-                node = first0 ? i0 : i1;
-            } else if (h0) {
-                node = i0;
-            } else if (h1) {
-                node = i1;
-            } else {
-                if (sp == 0)
-                    break;
-                node = stack[--sp];
-            }
+            stack[sp++] = first0 ? i1 : i0;
+            node = first0 ? i0 : i1;
+        } else if (h0) {
+            node = i0;
+        } else if (h1) {
+            node = i1;
+        } else {
+            if (sp == 0)
+                return false;
+            node = stack[--sp];
         }
     }
-    // The ground (plane.h:17-34) and height fog (medium.h:352-381) beside the BVH
-    for (int k = 0; k < S.unbounded_count; k++) {
-        DevUnbounded ub = S.unbounded[k];
-        if (ub.kind == 0) {
-            if (fabsf(d.y) < 1e-12f)
-                continue;
-            float t = (ub.height - o.y) / d.y;
-            if (t > tmin && t < h.t) {
-                h.t = t;
-                h.prim = (uint32_t(kGround) << kKindShift) | uint32_t(k);
-                if (ANY)
-                    return h;
-            }
-        } else if (media_key != 0) {
-            float len = length(d);
-            float kk = d.y / ub.scale_height;
-            float start = ub.density * len * expf(-(o.y + tmin * d.y - ub.height) / ub.scale_height);
-            if (!(start > 0.0f))
-                continue;
-            float tau = -logf(1.0f - hash_uniform(media_key, 0x40000000u + uint32_t(k)));
-            float t;
-            if (fabsf(kk) < 1e-12f) {
-                t = tmin + tau / start;
-            } else {
-                float x = 1.0f - tau * kk / start;
-                if (x <= 0.0f)
-                    continue;
-                t = tmin - logf(x) / kk;
-            }
-            if (t < h.t && isfinite(t)) {
-                h.t = t;
-                h.prim = (uint32_t(kHeightFog) << kKindShift) | uint32_t(k);
-                if (ANY)
-                    return h;
-            }
-        }
+}
+
+// The whole walk of one ray: the tree, then the unbounded objects. h.t holds
+// tmax, h.prim the primitive that ANY ignores; true when ANY and one was hit.
+template <bool ANY, bool VOX, int WALK>
+MYPBR_DEV bool walk(const DeviceScene& S, float3 o, float3 d, float tmin, uint64_t media_key, HitInfo& h) {
+    if (S.has_bvh) {
+        bool found;
+        if constexpr (WALK == kWalkWide)
+            found = walk_tree4<ANY, VOX>(S, o, d, tmin, media_key, h);
+        else if constexpr (WALK == kWalkWide8)
+            found = walk_tree8q<ANY, VOX>(S, o, d, tmin, media_key, h);
+        else if constexpr (WALK == kWalkPostponed)
+            found = walk_postponed<ANY, VOX>(S, o, d, tmin, media_key, h);
+        else
+            found = walk_binary<ANY, VOX>(S, o, d, tmin, media_key, h);
+        if (ANY && found)
+            return true;
     }
-    return h;
+    return walk_unbounded<ANY>(S, o, d, tmin, media_key, h);
 }
 
 // ------------------------------------------------------- surface records
@@ -1392,9 +1406,10 @@ MYPBR_DEV float float_step(float x, float dir) {
 // origin's largest coordinate, in units of d. Below that the intersection
 // arithmetic cannot tell on which side of the origin a surface lies; the
 // spawn offset has already put the surface just left behind the origin.
+template <bool Y_FIRST = false>
 MYPBR_DEV float spawn_tmin(float3 o, float3 d) {
     float m = fmaxf(fabsf(o.x), fmaxf(fabsf(o.y), fabsf(o.z)));
-    return m * 9.5367431640625e-7f * rsqrtf(dot(d, d));
+    return m * 9.5367431640625e-7f * rsqrtf(Y_FIRST ? dot_y(d, d) : dot_x(d, d));
 }
 
 // Where a ray leaving surface s in direction w starts. Y_FIRST: which product

@@ -824,8 +824,9 @@ MYPBR_DEV bool is_volume(const DeviceScene& S, int mi) { return S.materials[mi].
 // ------------------------------------------------------------------ lights
 
 // environment.h:334-339
+template <bool FIXED = false>
 MYPBR_DEV void env_angles(const DeviceScene& S, float3 dir, float& u, float& theta) {
-    float3 d = normalize(dir);
+    float3 d = FIXED ? normalize_x(dir) : normalize(dir);
     theta = acosf(clampf(d.y, -1.0f, 1.0f));
     // fused by hand: left to the compiler, whether it fuses depends on the code around
     u = fmaf(atan2f(d.x, -d.z), 0.5f * kInvPi, 0.5f) + S.env_rotation;
@@ -833,9 +834,10 @@ MYPBR_DEV void env_angles(const DeviceScene& S, float3 dir, float& u, float& the
 }
 
 // environment.h:202-215 (bilinear)
+template <bool FIXED = false>
 MYPBR_DEV float3 env_radiance(const DeviceScene& S, float3 dir) {
     float u, theta;
-    env_angles(S, dir, u, theta);
+    env_angles<FIXED>(S, dir, u, theta);
     int w = S.env_w, h = S.env_h;
     float x = u * w - 0.5f;
     float y = clampf(theta * kInvPi * h - 0.5f, 0.0f, h - 1.0f);
@@ -919,7 +921,12 @@ MYPBR_DEV bool env_only(const DeviceScene& S) {
     return S.light_count == 1 && S.env_w > 0 && !S.sun_enabled && S.lights[0].kind == 1;
 }
 
+// FIXED (here and in escaped_radiance): sums of products in a stated order,
+// for the kernels whose frames must be those of others to the last bit.
+template <bool FIXED = false>
 MYPBR_DEV bool sun_in_cone(const DeviceScene& S, float3 dir) {
+    if constexpr (FIXED)
+        return dot_x(normalize_x(dir), S.sun_dir) >= S.sun_cos_max;
     return dot(normalize(dir), S.sun_dir) >= S.sun_cos_max;
 }
 
@@ -1074,10 +1081,11 @@ MYPBR_DEV float3 lights_sample(const DeviceScene& S, float3 o, Rng& g) {
 }
 
 // camera.h:515-529
+template <bool FIXED = false>
 MYPBR_DEV float3 escaped_radiance(const DeviceScene& S, float3 dir, bool camera_ray) {
     float3 sky;
     if (S.env_w > 0) {
-        sky = env_radiance(S, dir);
+        sky = env_radiance<FIXED>(S, dir);
     } else if (!S.use_sky) {
         sky = S.background;
     } else {
@@ -1085,7 +1093,7 @@ MYPBR_DEV float3 escaped_radiance(const DeviceScene& S, float3 dir, bool camera_
         float a = 0.5f * (ud.y + 1.0f);
         sky = (1.0f - a) * f3(1.0f) + a * f3(0.5f, 0.7f, 1.0f);
     }
-    if (S.sun_enabled && (S.sun_disk_visible || !camera_ray) && sun_in_cone(S, dir))
+    if (S.sun_enabled && (S.sun_disk_visible || !camera_ray) && sun_in_cone<FIXED>(S, dir))
         sky += S.sun_radiance;
     return sky;
 }

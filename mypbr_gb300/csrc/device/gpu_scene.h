@@ -95,9 +95,9 @@ struct mypbr_gpu_scene {
     // autotuned launch settings (0: built-in defaults)
     size_t tuned_wave_paths = 0;
     int tuned_block = 0;
-    int tuned_traversal = 0;  // 0: the scene's default (3 or 4); 1: lanes take new rays (k_extend_pt);
-                              // 2: the 4-wide tree; 3: postponed leaves; 4: the plain binary walk
-    bool prefer_postponed = false;  // spheres fill fewer than half the leaves: traversal 0 means 3
+    int tuned_traversal = 0;  // 0: the default (1); 1: lanes take new rays (k_extend_lanes); 2: the 4-wide
+                              // tree; 3: postponed leaves; 4: the plain binary walk
+    bool prefer_postponed = false;  // spheres fill fewer than half the leaves: lanes postpone them
     // the instantiated graph of the last batch whose first job used this
     // handle, replayed while a batch captures to the same launches
     mypbr_dev::BatchGraphCache* batch_graph = nullptr;
@@ -132,6 +132,8 @@ int guide_train(mypbr_gpu_scene* G, int steps, int batch_tiles, float lr, cudaSt
 int guide_fit_box(mypbr_gpu_scene* G, cudaStream_t st);
 // The walk's leaf records (dev_scene.cuh's pack_leaf) for the scene's leaf references, on the device.
 int build_leaves(mypbr_gpu_scene* G);
+// The same for any n references (in device memory); the records belong to the handle.
+int pack_leaves(mypbr_gpu_scene* G, const uint32_t* refs, int n, float4*& out);
 // The binary tree's device nodes collapsed to four children per node (walk_tree4's layout); depth: deepest level.
 void collapse_to_4(const std::vector<float4>& bin, std::vector<float4>& out, int& depth);
 // The binary tree collapsed to 8 children per node with quantised child boxes

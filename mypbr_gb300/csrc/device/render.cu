@@ -80,15 +80,16 @@ struct WaveParams {
 };
 
 // Counters: extension queue length entering bounce d; shadow queue length of
-// bounce d; rays of the extension queue handed out so far (the persistent
-// extend kernel); length of shading class c's queue at bounce d.
+// bounce d; rays of either handed out so far (the kernels whose lanes take
+// new rays); length of shading class c's queue at bounce d.
 MYPBR_DEV uint32_t* ext_counter(const WaveParams& P, int d) { return P.B.counters + d; }
 MYPBR_DEV uint32_t* sh_counter(const WaveParams& P, int d) { return P.B.counters + P.B.depth_slots + d; }
 MYPBR_DEV uint32_t* fetch_counter(const WaveParams& P, int d) { return P.B.counters + 2 * P.B.depth_slots + d; }
+MYPBR_DEV uint32_t* sh_fetch_counter(const WaveParams& P, int d) { return P.B.counters + 3 * P.B.depth_slots + d; }
 MYPBR_DEV uint32_t* class_counter(const WaveParams& P, int d, int c) {
-    return P.B.counters + 3 * P.B.depth_slots + d * kShadeClasses + c;
+    return P.B.counters + 4 * P.B.depth_slots + d * kShadeClasses + c;
 }
-constexpr int kCounterRows = 3 + kShadeClasses;
+constexpr int kCounterRows = 4 + kShadeClasses;
 // Place i of class c's queue: two classes share an array, one from its front,
 // the other from its back (together they hold a wave's paths at most).
 MYPBR_DEV uint32_t* class_entry(const WaveParams& P, int c, uint32_t i) {
@@ -322,7 +323,8 @@ __global__ void k_features(WaveParams P, int gated) {
         float3 tint = f3(1.0f), albedo = f3(1.0f), normal = f3(0.0f);
         bool done = false;
         for (int b = 0; b < 8 && !done; b++) {
-            HitInfo h = closest_hit<true>(P.S, o, d, spawn_tmin(o, d), 3.0e38f, media_key(P, pixel, pass, 100 + b, 3));
+            HitInfo h = closest_hit<true>(P.S, o, d, spawn_tmin<true>(o, d), 3.0e38f,
+                                           media_key(P, pixel, pass, 100 + b, 3));
             if (h.prim == kMiss)
                 break;
             Surface s = make_surface(P.S, h, o, d);
@@ -399,58 +401,90 @@ __global__ void __launch_bounds__(256, 3) k_extend(WaveParams P, int depth) {
     }
 }
 
-// k_extend with lanes that take a new ray as soon as theirs is done: a warp
-// advances all its rays one BVH node per step, and when at least a quarter of
-// its lanes are idle (or all), it takes that many rays from the queue with
-// one atomic. Lanes then do not wait for the slowest ray of their warp (the
-// replacement of terminated rays of Aila and Laine, "Understanding the
-// Efficiency of Ray Traversal on GPUs", HPG 2009). Same hits as k_extend.
-template <bool VOX>
-__global__ void __launch_bounds__(256, 3) k_extend_pt(WaveParams P, int depth) {
+// How many lanes of a warp stand idle before it takes new rays. Fewer keep
+// more lanes busy, more keep the warp's rays in step. Measured (extend ms at
+// 12 / 16 / 20 / 24): 2 M-triangle room 55.5 / 55.6 / 53.8 / 54.1, voxel hall
+// 22.1 / 20.2 / 19.1 / 19.0, guided hall 44.4 / 44.5 / 45.6 / 48.9, sphere
+// field 27.0 / 27.1 / 27.5 / 28.1.
+constexpr int kTakeAt = 20;
+
+// Rays of a queue handed to the lanes of a warp: the warp takes a run of them
+// with one atomic and its lanes take from the run.
+struct WarpRun {
+    uint32_t at = 0, end = 0;  // the same in every lane
+    bool dry = false;
+    // Below how many walking lanes it is time to take rays (none are left: 0).
+    MYPBR_DEV int least() const { return dry ? 0 : 33 - kTakeAt; }
+    // One entry for each lane that asks (n: none left for it). Whole warp.
+    MYPBR_DEV uint32_t take(uint32_t* fetch, uint32_t n, uint32_t run, bool ask) {
+        const unsigned lane = threadIdx.x & 31, asking = __ballot_sync(0xffffffffu, ask);
+        if (at == end && !dry) {
+            uint32_t first = 0;
+            if (lane == 0)
+                first = atomicAdd(fetch, run);
+            at = min(__shfl_sync(0xffffffffu, first, 0), n);
+            end = min(at + run, n);
+            dry = at == end;
+        }
+        const uint32_t k = at + uint32_t(__popc(asking & ((1u << lane) - 1u)));
+        const bool got = ask && k < end;
+        at = min(at + uint32_t(__popc(asking)), end);
+        return got ? k : n;
+    }
+};
+MYPBR_DEV uint32_t warp_run(uint32_t n) {
+    const uint32_t share = n / (gridDim.x * (blockDim.x / 32) * 4 + 1);
+    return share >= 128 ? 128 : share <= 32 ? 32 : share / 32 * 32;
+}
+
+// k_extend with lanes that take a new ray as soon as theirs is done and
+// kTakeAt lanes of the warp are: they do not wait for the slowest ray of their
+// warp (the replacement of terminated rays of Aila and Laine, "Understanding
+// the Efficiency of Ray Traversal on GPUs", HPG 2009), on top of the postponed
+// leaves. Same hits as k_extend. The walk is bound by issue and by L1; what is
+// gained is lanes at work per instruction. Against postponed leaves alone
+// (extend ms, one box): guided voxel hall 89.4 -> 45.6 (rays through the slits
+// cross the whole terrain, the others a room), plain hall 21.6 -> 19.1, sphere
+// field 32.3 -> 27.5 (binary walk 29.6), 300 k-triangle band 14.6 -> 14.2.
+// Registers: more resident warps against spills (extend ms at 80 / 72 / 64
+// registers: sphere field 28.9 / 26.4 / 27.9, 2 M-triangle room 53.9 / 54.4 /
+// 50.7, voxel hall 19.1 / 23.3 at 80 / 72).
+constexpr int lane_registers(bool vox, bool postponed) { return vox ? 80 : postponed ? 64 : 72; }
+template <bool VOX, bool POSTPONED>
+__global__ void __maxnreg__(lane_registers(VOX, POSTPONED)) k_extend_lanes(WaveParams P, int depth) {
     depth = bounce_of(P, depth);
     const uint32_t n = *ext_counter(P, depth);
     if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0)
         atomicAdd(&P.totals[0], (unsigned long long)n);
     const float4* rays = P.B.ray[depth & 1];
     const int2 wave = wave_of(P);
-    uint32_t* fetch = fetch_counter(P, depth);
-    const int lane = threadIdx.x & 31;
-    const unsigned lanes_below = (1u << lane) - 1u;
-    WalkState W;
+    const uint32_t run = warp_run(n);
+    WarpRun take;
+    LaneWalk W;
     int stack[kBvhStack];
-    uint32_t entry = 0;
-    bool active = false, exhausted = false;
-    // every lane's walk is bounded (node visits); this bounds the warp's steps
-    // by the rays one warp could ever be given, were it given all of them
-    const long long max_steps = (long long)(n + 32) * (long long)(P.S.bvh_node_count + 2) + 64;
-    for (long long step = 0; step < max_steps; step++) {
-        unsigned idle = __ballot_sync(0xffffffffu, !active && !exhausted);
-        unsigned busy = __ballot_sync(0xffffffffu, active);
-        if (idle != 0 && (__popc(idle) >= 8 || busy == 0)) {
-            int leader = __ffs(idle) - 1;
-            uint32_t base = 0;
-            if (lane == leader)
-                base = atomicAdd(fetch, uint32_t(__popc(idle)));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (!active && !exhausted) {
-                entry = base + uint32_t(__popc(idle & lanes_below));
-                if (entry < n) {
-                    const Pair r = load_pair(rays, entry);
-                    walk_init(P.S, W, f3(r.a), f3(r.b), spawn_tmin(f3(r.a), f3(r.b)), 3.0e38f,
-                              extend_key(P, wave, depth, entry));
-                    active = true;
-                } else {
-                    exhausted = true;
+    uint32_t entry = n;
+    W.stop();
+    while (true) {
+        const bool idle = W.done();
+        const unsigned idle_lanes = __ballot_sync(0xffffffffu, idle);
+        if (__popc(idle_lanes) >= kTakeAt) {
+            if (idle && entry < n) {
+                walk_unbounded<false>(P.S, W.o, W.d, W.tmin, W.media_key, W.h);
+                put_hit(P, entry, W.h);
+            }
+            const uint32_t k = take.take(fetch_counter(P, depth), n, run, idle);
+            if (idle) {
+                entry = k;
+                if (k < n) {
+                    const Pair r = load_pair(rays, k);
+                    W.start(P.S, f3(r.a), f3(r.b), spawn_tmin(f3(r.a), f3(r.b)), 3.0e38f,
+                            extend_key(P, wave, depth, k));
                 }
             }
+            if (!__any_sync(0xffffffffu, entry < n))
+                break;
         }
-        if (__all_sync(0xffffffffu, exhausted))
-            break;
-        if (active && !walk_node<false, VOX>(P.S, W, stack)) {
-            walk_unbounded<false>(P.S, W);
-            put_hit(P, entry, W.h);
-            active = false;
-        }
+        W.advance<false, VOX, POSTPONED>(P.S, stack, take.least());
     }
 }
 
@@ -794,7 +828,75 @@ __global__ void __launch_bounds__(256, 2) k_shade_guided(WaveParams P, int depth
     shade_body<C, true>(P, bounce_of(P, depth));
 }
 
-template <bool VOX, int WALK>
+// What a shadow ray has to find out (the host picks it by scene and options).
+// kShadowAny: nothing the ray can reach emits, and nothing lets it through:
+// only whether it escapes matters (camera.h:488-503). kShadowEmitters: the
+// surfaces that emit are few, so the nearest of them along the ray is found
+// first, from their list; then only whether something lies before it matters
+// (or, with none, whether the ray escapes), and a ray that would bring no
+// light anyway is not walked at all. kShadowClosest: the closest hit, through
+// clear glass if the options say so.
+// The 2 M-triangle room (16 lamps) at 1080p, 16 spp: shadow 58.5 ms with
+// closest hits, 40.5 with its emitters first and lanes that take new rays.
+enum : int { kShadowAny = 0, kShadowEmitters = 1, kShadowClosest = 2 };
+
+// The light of a shadow ray that ends, to its path.
+MYPBR_DEV void shadow_end(const WaveParams& P, int2 wave, int depth, uint2 entry, float3 through, float3 emission) {
+    const float4 sc = P.B.state[depth & 1][2 * size_t(entry.x)];
+    const bool ends = entry.y & kShadowEnds;
+    float4* to = ends ? P.B.out + (entry.y & ~kShadowEnds) : P.B.state[(depth + 1) & 1] + 2 * size_t(entry.y) + 1;
+    float3 rad = f3(*to) + f3(sc) * through * emission;
+    *to = make_float4(rad.x, rad.y, rad.z, 0.0f);
+    if (P.record && ends) {
+        const SlotPath sp = slot_path(P, wave, entry.y & ~kShadowEnds);
+        if (sp.band_pass < uint32_t(P.rec_passes))
+            P.rec.fin[sp.band_pixel * uint32_t(P.rec_passes) + sp.band_pass] = make_float4(rad.x, rad.y, rad.z, 0.0f);
+    }
+}
+
+MYPBR_DEV uint64_t shadow_key(const WaveParams& P, int2 wave, int depth, float4 origin, int hop) {
+    if (!P.keyed)
+        return 0;
+    const SlotPath sp = slot_path(P, wave, f_bits(origin.w));
+    return media_key(P, sp.pixel, sp.pass, uint32_t(depth), 1 + 4 * hop);
+}
+
+// The light that reaches a ray whose nearest emitter is h, were nothing in
+// between (a sky-only sample, sky != 0, already holds the sky's radiance).
+template <bool FIXED = false>
+MYPBR_DEV float3 unblocked(const DeviceScene& S, const HitInfo& h, float3 o, float3 d, float sky) {
+    if (h.prim == kMiss)
+        return sky != 0.0f ? f3(1.0f) : escaped_radiance<FIXED>(S, d, false);
+    const Surface s = make_surface(S, h, o, d);
+    return emitted(S, s.material, d, s);
+}
+
+// Where a closest-hit shadow ray stands after a walk: true when it goes on
+// behind clear glass (o and through moved on), else emission is what it found.
+MYPBR_DEV bool shadow_hop(const WaveParams& P, const HitInfo& h, float3& o, float3 d, int hop, float3& through,
+                          float3& emission) {
+    const DeviceScene& S = P.S;
+    if (h.prim == kMiss) {
+        emission = escaped_radiance(S, d, false);
+        return false;
+    }
+    int kind = int(h.prim >> kKindShift);
+    int mat = (kind == kSphere || kind == kQuad || kind == kTriangle || kind == kVoxel) ? hit_material(S, h) : -1;
+    // media, the ground and fog neither emit nor let shadows through
+    bool through_glass = P.transparent_shadows && hop < 16 && mat >= 0 && lets_shadows_through(S, mat);
+    if (!through_glass && (mat < 0 || !may_emit(S, mat)))
+        return false;  // blocked by something dark
+    Surface s = make_surface(S, h, o, d);
+    if (through_glass) {
+        through *= interior_transmittance(S, mat, h.t * length(d), s.front);
+        o = spawn_origin(s, d);
+        return true;
+    }
+    emission = emitted(S, mat, d, s);
+    return false;
+}
+
+template <bool VOX, int WALK, int MODE>
 __global__ void __launch_bounds__(256, 3) k_shadow(WaveParams P, int depth) {
     depth = bounce_of(P, depth);
     uint32_t n = *sh_counter(P, depth);
@@ -803,63 +905,96 @@ __global__ void __launch_bounds__(256, 3) k_shadow(WaveParams P, int depth) {
     const DeviceScene& S = P.S;
     uint32_t stride = gridDim.x * blockDim.x;
     const float4* rays = P.B.ray[depth & 1];
-    const float4* states = P.B.state[depth & 1];
     const int2 wave = wave_of(P);
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += stride) {
         const uint2 entry = P.B.shadow_queue[k];
         const Pair ray = load_pair(rays, entry.x);
-        float3 o = f3(ray.a), d = f3(ray.b);
-        uint64_t key = 0;
-        uint32_t pixel = 0, pass = 0;
-        if (P.keyed) {
-            const SlotPath sp = slot_path(P, wave, f_bits(ray.a.w));
-            pixel = sp.pixel;
-            pass = sp.pass;
-        }
+        float3 o = f3(ray.a);
+        const float3 d = f3(ray.b);
         float3 through = f3(1.0f), emission = f3(0.0f);
-        if (!S.has_emitters && !(P.transparent_shadows && S.has_clear_glass)) {
-            // Nothing the ray can reach emits, and nothing lets it through:
-            // only whether it escapes matters (camera.h:488-503). A sky-only
-            // sample already holds the sky's radiance (marked beside the direction).
-            if (P.keyed)
-                key = media_key(P, pixel, pass, uint32_t(depth), 1);
-            if (!any_hit<VOX, WALK>(S, o, d, spawn_tmin(o, d), 3.0e38f, key))
-                emission = ray.b.w != 0.0f ? f3(1.0f) : escaped_radiance(S, d, false);
-        } else
-        for (int hop = 0; hop <= 16; hop++) {
-            if (P.keyed)
-                key = media_key(P, pixel, pass, uint32_t(depth), 1 + 4 * hop);
-            HitInfo h = closest_hit<VOX, WALK>(S, o, d, spawn_tmin(o, d), 3.0e38f, key);
-            if (h.prim == kMiss) {
-                emission = escaped_radiance(S, d, false);
+        if constexpr (MODE == kShadowClosest) {
+            for (int hop = 0; hop <= 16; hop++) {
+                const uint64_t key = shadow_key(P, wave, depth, ray.a, hop);
+                const HitInfo h = closest_hit<VOX, WALK>(S, o, d, spawn_tmin(o, d), 3.0e38f, key);
+                if (!shadow_hop(P, h, o, d, hop, through, emission))
+                    break;
+            }
+        } else {
+            const uint64_t key = shadow_key(P, wave, depth, ray.a, 0);
+            const float tmin = spawn_tmin(o, d);
+            HitInfo e;
+            e.prim = kMiss;
+            e.t = 3.0e38f;
+            if constexpr (MODE == kShadowEmitters) {
+                e = nearest_emitter(S, o, d, tmin, key);
+                emission = e.prim == kMiss && S.dark_sky ? f3(0.0f) : unblocked(S, e, o, d, ray.b.w);
+                if (!is_zero(emission) && any_hit<VOX, WALK>(S, o, d, tmin, e.t, key, e.prim))
+                    emission = f3(0.0f);
+            } else if (!any_hit<VOX, WALK>(S, o, d, tmin, e.t, key)) {
+                emission = unblocked(S, e, o, d, ray.b.w);
+            }
+        }
+        shadow_end(P, wave, depth, entry, through, emission);
+    }
+}
+
+// k_shadow with lanes that take a new ray as soon as theirs is done (see
+// k_extend_lanes), for the two modes whose rays are one walk each.
+template <bool VOX, int MODE>
+__global__ void __maxnreg__(lane_registers(VOX, true)) k_shadow_lanes(WaveParams P, int depth) {
+    depth = bounce_of(P, depth);
+    const uint32_t n = *sh_counter(P, depth);
+    if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0)
+        atomicAdd(&P.totals[1], (unsigned long long)n);
+    const DeviceScene& S = P.S;
+    const float4* rays = P.B.ray[depth & 1];
+    const int2 wave = wave_of(P);
+    const uint32_t run = warp_run(n);
+    WarpRun take;
+    LaneWalk W;
+    int stack[kBvhStack];
+    uint32_t k = n;
+    uint2 entry = make_uint2(0u, 0u);
+    float3 emission = f3(0.0f);
+    W.stop();
+    while (true) {
+        const bool idle = W.done();
+        if (__popc(__ballot_sync(0xffffffffu, idle)) >= kTakeAt) {
+            if (idle && k < n) {
+                if (W.found || walk_unbounded<true>(S, W.o, W.d, W.tmin, W.media_key, W.h))
+                    emission = f3(0.0f);
+                else if (MODE == kShadowAny)
+                    emission = unblocked<true>(S, W.h, W.o, W.d, rays[2 * size_t(entry.x) + 1].w);
+                shadow_end(P, wave, depth, entry, f3(1.0f), emission);
+            }
+            const uint32_t next = take.take(sh_fetch_counter(P, depth), n, run, idle);
+            if (idle) {
+                k = next;
+                if (k < n) {
+                    entry = P.B.shadow_queue[k];
+                    const Pair ray = load_pair(rays, entry.x);
+                    const float3 o = f3(ray.a), d = f3(ray.b);
+                    const uint64_t key = shadow_key(P, wave, depth, ray.a, 0);
+                    const float tmin = spawn_tmin(o, d);
+                    emission = f3(0.0f);
+                    HitInfo e;
+                    e.prim = kMiss;
+                    e.t = 3.0e38f;
+                    if constexpr (MODE == kShadowEmitters) {
+                        e = nearest_emitter(S, o, d, tmin, key);
+                        emission = e.prim == kMiss && S.dark_sky ? f3(0.0f) : unblocked<true>(S, e, o, d, ray.b.w);
+                    }
+                    W.start(S, o, d, tmin, e.t, key, e.prim);
+                    if (MODE == kShadowEmitters && is_zero(emission)) {
+                        W.found = true;  // nothing to bring: not walked
+                        W.stop();
+                    }
+                }
+            }
+            if (!__any_sync(0xffffffffu, k < n))
                 break;
-            }
-            int kind = int(h.prim >> kKindShift);
-            int mat = (kind == kSphere || kind == kQuad || kind == kTriangle || kind == kVoxel) ? hit_material(S, h) : -1;
-            // media, the ground and fog neither emit nor let shadows through
-            bool through_glass = P.transparent_shadows && hop < 16 && mat >= 0 && lets_shadows_through(S, mat);
-            if (!through_glass && (mat < 0 || !may_emit(S, mat)))
-                break;  // blocked by something dark
-            Surface s = make_surface(S, h, o, d);
-            if (through_glass) {
-                through *= interior_transmittance(S, mat, h.t * length(d), s.front);
-                o = spawn_origin(s, d);
-                continue;
-            }
-            emission = emitted(S, mat, d, s);
-            break;
         }
-        const float4 sc = states[2 * size_t(entry.x)];
-        const bool ends = entry.y & kShadowEnds;
-        float4* to = ends ? P.B.out + (entry.y & ~kShadowEnds) : P.B.state[(depth + 1) & 1] + 2 * size_t(entry.y) + 1;
-        float3 rad = f3(*to) + f3(sc) * through * emission;
-        *to = make_float4(rad.x, rad.y, rad.z, 0.0f);
-        if (P.record && ends) {
-            const SlotPath sp = slot_path(P, wave, entry.y & ~kShadowEnds);
-            if (sp.band_pass < uint32_t(P.rec_passes))
-                P.rec.fin[sp.band_pixel * uint32_t(P.rec_passes) + sp.band_pass] =
-                    make_float4(rad.x, rad.y, rad.z, 0.0f);
-        }
+        W.advance<true, VOX, true>(S, stack, take.least());
     }
 }
 
@@ -1190,8 +1325,9 @@ int bad_arg(const std::string& m) {
 struct Launch {
     int grid_extend, grid_shade, grid_shadow, grid_stream;
     int block = 256;              // threads per block of extend, shade and shadow
-    bool persistent = false;      // extend with lanes that take new rays (k_extend_pt)
-    int walk = kWalkBinary;       // which walk extend and shadow use
+    int walk = kWalkBinary;       // which walk extend uses
+    int shadow_walk = kWalkBinary;  // and shadow
+    int shadow_mode = kShadowClosest;
     bool guided_kernels = false;  // the shading variants of guided renders
     int grid_guide = 0;
     size_t guide_smem = 0;
@@ -1207,6 +1343,10 @@ void launch_bounce_kernel(const void* fn, int grid, int block, cudaStream_t st, 
 
 // The extend and shadow kernels of a walk, with or without the voxel code.
 const void* extend_kernel(bool vox, int walk) {
+    if (walk == kWalkLanes)
+        return (const void*)k_extend_lanes<false, false>;
+    if (walk == kWalkLanesPostponed)
+        return vox ? (const void*)k_extend_lanes<true, true> : (const void*)k_extend_lanes<false, true>;
     if (walk == kWalkWide8)
         return vox ? (const void*)k_extend<true, kWalkWide8> : (const void*)k_extend<false, kWalkWide8>;
     if (walk == kWalkWide)
@@ -1215,14 +1355,31 @@ const void* extend_kernel(bool vox, int walk) {
         return vox ? (const void*)k_extend<true, kWalkPostponed> : (const void*)k_extend<false, kWalkPostponed>;
     return vox ? (const void*)k_extend<true, kWalkBinary> : (const void*)k_extend<false, kWalkBinary>;
 }
-const void* shadow_kernel(bool vox, int walk) {
-    if (walk == kWalkWide8)
-        return vox ? (const void*)k_shadow<true, kWalkWide8> : (const void*)k_shadow<false, kWalkWide8>;
-    if (walk == kWalkWide)
-        return vox ? (const void*)k_shadow<true, kWalkWide> : (const void*)k_shadow<false, kWalkWide>;
-    if (walk == kWalkPostponed)
-        return vox ? (const void*)k_shadow<true, kWalkPostponed> : (const void*)k_shadow<false, kWalkPostponed>;
-    return vox ? (const void*)k_shadow<true, kWalkBinary> : (const void*)k_shadow<false, kWalkBinary>;
+template <bool VOX, int MODE>
+const void* shadow_kernel_of(int walk) {
+    if constexpr (MODE != kShadowClosest)
+        if (walk == kWalkLanesPostponed)
+            return (const void*)k_shadow_lanes<VOX, MODE>;
+    return walk == kWalkWide8       ? (const void*)k_shadow<VOX, kWalkWide8, MODE>
+           : walk == kWalkWide      ? (const void*)k_shadow<VOX, kWalkWide, MODE>
+           : walk == kWalkPostponed ? (const void*)k_shadow<VOX, kWalkPostponed, MODE>
+                                    : (const void*)k_shadow<VOX, kWalkBinary, MODE>;
+}
+template <bool VOX>
+const void* shadow_kernel_of(int walk, int mode) {
+    return mode == kShadowAny        ? shadow_kernel_of<VOX, kShadowAny>(walk)
+           : mode == kShadowEmitters ? shadow_kernel_of<VOX, kShadowEmitters>(walk)
+                                     : shadow_kernel_of<VOX, kShadowClosest>(walk);
+}
+const void* shadow_kernel(bool vox, int walk, int mode) {
+    return vox ? shadow_kernel_of<true>(walk, mode) : shadow_kernel_of<false>(walk, mode);
+}
+
+// What the shadow rays of a scene have to find out.
+int shadow_mode(const DeviceScene& S, int transparent_shadows) {
+    if (transparent_shadows && S.has_clear_glass)
+        return kShadowClosest;
+    return !S.has_emitters ? kShadowAny : S.emitter_count >= 0 ? kShadowEmitters : kShadowClosest;
 }
 
 // The path kernels keep their data in L1 (tree nodes, voxel cells, material
@@ -1235,23 +1392,20 @@ void prefer_l1(int device) {
     const uint64_t bit = uint64_t(1) << (device & 63);
     if (done.load() & bit)
         return;
-    const void* kernels[] = {
+    std::vector<const void*> kernels = {
         (const void*)k_generate, (const void*)k_features,
-        (const void*)k_extend<true, kWalkBinary>, (const void*)k_extend<false, kWalkBinary>,
-        (const void*)k_extend<true, kWalkWide>, (const void*)k_extend<false, kWalkWide>,
-        (const void*)k_extend<true, kWalkPostponed>, (const void*)k_extend<false, kWalkPostponed>,
-        (const void*)k_extend<true, kWalkWide8>, (const void*)k_extend<false, kWalkWide8>,
-        (const void*)k_shadow<true, kWalkWide8>, (const void*)k_shadow<false, kWalkWide8>,
-        (const void*)k_extend_pt<true>, (const void*)k_extend_pt<false>,
-        (const void*)k_shadow<true, kWalkBinary>, (const void*)k_shadow<false, kWalkBinary>,
-        (const void*)k_shadow<true, kWalkWide>, (const void*)k_shadow<false, kWalkWide>,
-        (const void*)k_shadow<true, kWalkPostponed>, (const void*)k_shadow<false, kWalkPostponed>,
         (const void*)k_shade<kClassMiss>, (const void*)k_shade<kClassLambert>, (const void*)k_shade<kClassMetal>,
         (const void*)k_shade<kClassDielectric>, (const void*)k_shade<kClassPrincipled>,
         (const void*)k_shade<kClassGeneric>, (const void*)k_shade_guided<kClassMiss>,
         (const void*)k_shade_guided<kClassLambert>, (const void*)k_shade_guided<kClassMetal>,
         (const void*)k_shade_guided<kClassDielectric>, (const void*)k_shade_guided<kClassPrincipled>,
         (const void*)k_shade_guided<kClassGeneric>};
+    for (bool vox : {false, true})
+        for (int walk : {kWalkBinary, kWalkWide, kWalkPostponed, kWalkWide8, kWalkLanes, kWalkLanesPostponed}) {
+            kernels.push_back(extend_kernel(vox, walk));
+            for (int mode : {kShadowAny, kShadowEmitters, kShadowClosest})
+                kernels.push_back(shadow_kernel(vox, walk, mode));
+        }
     for (const void* k : kernels)
         cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, int(cudaSharedmemCarveoutMaxL1));
     cudaGetLastError();  // a hint: a driver that ignores it changes nothing
@@ -1259,20 +1413,21 @@ void prefer_l1(int device) {
 }
 
 // Grids of `block` threads: SMs x resident blocks (persistent-style loops).
-Launch launch_config(const mypbr_gpu_scene& G, int block = 0) {
+Launch launch_config(const mypbr_gpu_scene& G, const mypbr_render_opts& o, int block = 0) {
     prefer_l1(G.device);
     Launch L{};
-    // 128-thread blocks suit the postponed-leaf walk (6 % faster on the
-    // 2 M-triangle room, 6 % on the guided voxel hall), 256 the rest
-    int default_block = G.prefer_postponed && G.tuned_traversal == 0 ? 128 : 256;
-    L.block = block == 128 || block == 256 ? block : (G.tuned_block ? G.tuned_block : default_block);
-    // traversal 0 is the scene's default: leaves postponed unless spheres fill
-    // most of the leaves (other leaves' tests diverge), the plain binary walk else
-    int trav = G.tuned_traversal;
-    if (trav == 0)
-        trav = G.prefer_postponed && G.dev.postponed_ok ? 3 : 4;
-    L.persistent = trav == 1;
-    if (trav == 2 && G.dev.bvh4 != nullptr)
+    // Traversal 0 is lanes that take new rays, in blocks of 128, which leave
+    // the warps more independent (2 M-triangle room: extend 55.6 ms against
+    // 61.1 with 256, shadow 40.2 against 43.7; sphere field 27.1 against 29.0)
+    const int trav = G.tuned_traversal == 0 ? 1 : G.tuned_traversal;
+    L.block = block == 128 || block == 256 ? block
+              : G.tuned_block              ? G.tuned_block
+              : trav == 1 && G.dev.postponed_ok ? 128
+                                           : 256;
+    const bool lanes = trav == 1 && G.dev.postponed_ok && (G.prefer_postponed || !G.dev.has_voxels);
+    if (lanes)
+        L.walk = G.prefer_postponed ? kWalkLanesPostponed : kWalkLanes;
+    else if (trav == 2 && G.dev.bvh4 != nullptr)
         L.walk = kWalkWide;
     else if (trav == 3 && G.dev.postponed_ok)
         L.walk = kWalkPostponed;
@@ -1280,8 +1435,16 @@ Launch launch_config(const mypbr_gpu_scene& G, int block = 0) {
         L.walk = kWalkWide8;
     int per_sm = 0;
     bool vox = G.dev.has_voxels;
+    L.shadow_mode = shadow_mode(G.dev, o.transparent_shadows);
+    // whether anything is in the way does not depend on the order of the
+    // tests, so those rays postpone their leaves on sphere scenes too (sphere
+    // field: shadow 12.3 ms against 14.0); hits at the same t do
+    L.shadow_walk = !lanes                             ? L.walk
+                    : L.shadow_mode != kShadowClosest  ? kWalkLanesPostponed
+                    : G.prefer_postponed               ? kWalkPostponed
+                                                       : kWalkBinary;
     const void* extend = extend_kernel(vox, L.walk);
-    const void* shadow = shadow_kernel(vox, L.walk);
+    const void* shadow = shadow_kernel(vox, L.shadow_walk, L.shadow_mode);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, extend, L.block, 0);
     L.grid_extend = G.sm_count * std::max(per_sm, 1);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, shadow, L.block, 0);
@@ -1390,12 +1553,7 @@ int run_suffix(WaveParams& P, const Launch& L, cudaStream_t st, uint64_t& launch
 // One bounce: extend, the guiding network's mixtures (guided renders), the
 // shading classes, shadow rays. depth -1: the bounce counter in device memory.
 int run_bounce(WaveParams& P, const Launch& L, cudaStream_t st, uint64_t& launches, KernelTimer& T, int depth) {
-    if (L.persistent && P.S.has_voxels)
-        TIMED(1, (k_extend_pt<true><<<L.grid_extend, L.block, 0, st>>>(P, depth)));
-    else if (L.persistent)
-        TIMED(1, (k_extend_pt<false><<<L.grid_extend, L.block, 0, st>>>(P, depth)));
-    else
-        TIMED(1, (launch_bounce_kernel(extend_kernel(P.S.has_voxels, L.walk), L.grid_extend, L.block, st, P, depth)));
+    TIMED(1, (launch_bounce_kernel(extend_kernel(P.S.has_voxels, L.walk), L.grid_extend, L.block, st, P, depth)));
     TIMED(2, (k_classify<<<L.grid_stream, 256, 0, st>>>(P, depth)));
     if (P.guided && (depth < 0 || depth < P.guide_depths)) {  // the mixtures of this bounce's guidable vertices
         TIMED(4, (k_guide_forward<GuideQueueSource, GuidePackSink><<<L.grid_guide, 128 * kGuideGroups, L.guide_smem, st>>>(
@@ -1417,7 +1575,7 @@ int run_bounce(WaveParams& P, const Launch& L, cudaStream_t st, uint64_t& launch
         TIMED(2, (k_shade<kClassPrincipled><<<L.grid_shade, L.block, 0, st>>>(P, depth)));
         TIMED(2, (k_shade<kClassGeneric><<<L.grid_shade, L.block, 0, st>>>(P, depth)));
     }
-    TIMED(3, (launch_bounce_kernel(shadow_kernel(P.S.has_voxels, L.walk), L.grid_shadow, L.block, st, P, depth)));
+    TIMED(3, (launch_bounce_kernel(shadow_kernel(P.S.has_voxels, L.shadow_walk, L.shadow_mode), L.grid_shadow, L.block, st, P, depth)));
     launches += 3 + kShadeClasses;
     return MYPBR_OK;
 }
@@ -1602,7 +1760,7 @@ int prepare(mypbr_gpu_scene* G, const mypbr_camera* cam, const mypbr_render_opts
     if (s != MYPBR_OK)
         return s;
     P.B = G->rb;
-    R.L = launch_config(*G);
+    R.L = launch_config(*G, *o);
     R.guided = o->guided != 0;
     R.fixed_waves = o->samples_per_wave > 0;
     if (R.guided) {
@@ -2423,7 +2581,7 @@ extern "C" int mypbr_gpu_render_noalloc(mypbr_gpu_scene* G, const mypbr_camera* 
     P.B.film -= 3 * first_pixel;
     P.B.film2 -= 3 * first_pixel;
     P.B.feat -= 7 * first_pixel;
-    Launch L = launch_config(*G);
+    Launch L = launch_config(*G, *o);
     uint64_t launches = 0;
     KernelTimer T;  // off: no events are created
     T.st = st;
