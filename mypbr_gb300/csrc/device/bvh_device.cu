@@ -308,15 +308,6 @@ int pack_leaves(mypbr_gpu_scene* G, const uint32_t* refs, int n, float4*& out) {
     return MYPBR_OK;
 }
 
-int build_leaves(mypbr_gpu_scene* G) {
-    float4* leaves = nullptr;
-    if (G->leaf_ref_count > 0)
-        if (int s = pack_leaves(G, G->dev.leaf_refs, int(G->leaf_ref_count), leaves); s != MYPBR_OK)
-            return s;
-    G->dev.leaves = leaves;
-    return MYPBR_OK;
-}
-
 }  // namespace mypbr_dev
 
 using namespace mypbr_dev;
@@ -410,15 +401,15 @@ extern "C" int mypbr_gpu_scene_rebuild_bvh(mypbr_gpu_scene* G, int32_t method, m
         MYPBR_CUDA(cudaMemcpy(wide8_p, wide8.data(), wide8.size() * sizeof(uint4), cudaMemcpyHostToDevice));
         G->allocations.push_back(wide8_p);
     }
-    const uint32_t* host_refs = D.leaf_refs;
-    D.leaf_refs = sorted_refs.p;
-    if ((s = build_leaves(G)) != MYPBR_OK) {  // the host tree stays
-        D.leaf_refs = host_refs;
+    float4* leaves = nullptr;
+    if ((s = pack_leaves(G, sorted_refs.p, n, leaves)) != MYPBR_OK) {  // the host tree stays
         nodes.p = nullptr;  // freed with the handle
         sorted_refs.p = nullptr;
         return s;
     }
     D.bvh = nodes.p;
+    D.leaf_refs = sorted_refs.p;
+    D.leaves = leaves;
     D.bvh_node_count = n - 1;
     D.bvh4 = wide_p;
     D.bvh8 = wide8_p;

@@ -88,6 +88,7 @@ struct mypbr_gpu_scene {
     int max_depth_bvh = 0;
     size_t leaf_ref_count = 0;
     int64_t material_count = 0;
+    uint32_t shade_classes = 1u;  // bit c: paths can meet shading class c (0, a miss, always)
     mypbr_dev::RenderBuffers rb;
     mypbr_dev::GuideState guide;
     float3 box_lo{-1.0f, -1.0f, -1.0f}, box_hi{1.0f, 1.0f, 1.0f};  // bounds of the BVH's primitives
@@ -130,9 +131,7 @@ int guide_train(mypbr_gpu_scene* G, int steps, int batch_tiles, float lr, cudaSt
 // (1st to 99th percentile per axis, plus a margin) and re-expresses the
 // records in it. Synchronises the stream once.
 int guide_fit_box(mypbr_gpu_scene* G, cudaStream_t st);
-// The walk's leaf records (dev_scene.cuh's pack_leaf) for the scene's leaf references, on the device.
-int build_leaves(mypbr_gpu_scene* G);
-// The same for any n references (in device memory); the records belong to the handle.
+// The walk's leaf records (dev_scene.cuh's pack_leaf) for n references in device memory; they belong to the handle.
 int pack_leaves(mypbr_gpu_scene* G, const uint32_t* refs, int n, float4*& out);
 // The binary tree's device nodes collapsed to four children per node (walk_tree4's layout); depth: deepest level.
 void collapse_to_4(const std::vector<float4>& bin, std::vector<float4>& out, int& depth);

@@ -191,8 +191,12 @@ MYPBR_DEV int2 wave_of(const WaveParams& P) {
 
 // The bounce a kernel works on: its argument, or, given -1 (the kernels of a
 // replayed wave graph, which loops over bounces on the device), the bounce
-// counter in device memory.
-MYPBR_DEV int bounce_of(const WaveParams& P, int depth) { return depth >= 0 ? depth : P.B.wave_state[2]; }
+// counter in device memory; given kBounceBefore, the one before that (below
+// 0: none).
+constexpr int kBounceBefore = -2;
+MYPBR_DEV int bounce_of(const WaveParams& P, int depth) {
+    return depth >= 0 ? depth : P.B.wave_state[2] - (depth == kBounceBefore ? 1 : 0);
+}
 
 // A slot's pixel (of the whole image) and pass: the passes of one pixel are
 // neighbouring slots.
@@ -308,6 +312,7 @@ __global__ void k_generate(WaveParams P, int gated) {
 }
 
 // camera.h:253-277: albedo and normal of the first non-specular surface
+template <bool VOX>
 __global__ void k_features(WaveParams P, int gated) {
     if (!wave_starting(P, gated))
         return;
@@ -323,7 +328,7 @@ __global__ void k_features(WaveParams P, int gated) {
         float3 tint = f3(1.0f), albedo = f3(1.0f), normal = f3(0.0f);
         bool done = false;
         for (int b = 0; b < 8 && !done; b++) {
-            HitInfo h = closest_hit<true>(P.S, o, d, spawn_tmin<true>(o, d), 3.0e38f,
+            HitInfo h = closest_hit<VOX>(P.S, o, d, spawn_tmin<true>(o, d), 3.0e38f,
                                            media_key(P, pixel, pass, 100 + b, 3));
             if (h.prim == kMiss)
                 break;
@@ -899,6 +904,8 @@ MYPBR_DEV bool shadow_hop(const WaveParams& P, const HitInfo& h, float3& o, floa
 template <bool VOX, int WALK, int MODE>
 __global__ void __launch_bounds__(256, 3) k_shadow(WaveParams P, int depth) {
     depth = bounce_of(P, depth);
+    if (depth < 0)
+        return;
     uint32_t n = *sh_counter(P, depth);
     if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0)
         atomicAdd(&P.totals[1], (unsigned long long)n);
@@ -943,6 +950,8 @@ __global__ void __launch_bounds__(256, 3) k_shadow(WaveParams P, int depth) {
 template <bool VOX, int MODE>
 __global__ void __maxnreg__(lane_registers(VOX, true)) k_shadow_lanes(WaveParams P, int depth) {
     depth = bounce_of(P, depth);
+    if (depth < 0)
+        return;
     const uint32_t n = *sh_counter(P, depth);
     if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0)
         atomicAdd(&P.totals[1], (unsigned long long)n);
@@ -1324,6 +1333,7 @@ int bad_arg(const std::string& m) {
 
 struct Launch {
     int grid_extend, grid_shade, grid_shadow, grid_stream;
+    uint32_t shade_classes = 0;   // the shading kernels that can have work
     int block = 256;              // threads per block of extend, shade and shadow
     int walk = kWalkBinary;       // which walk extend uses
     int shadow_walk = kWalkBinary;  // and shadow
@@ -1375,6 +1385,19 @@ const void* shadow_kernel(bool vox, int walk, int mode) {
     return vox ? shadow_kernel_of<true>(walk, mode) : shadow_kernel_of<false>(walk, mode);
 }
 
+// The shading kernel of a class, plain or guided.
+const void* shade_kernel(int c, bool guided) {
+    static const void* const plain[kShadeClasses] = {
+        (const void*)k_shade<kClassMiss>,       (const void*)k_shade<kClassLambert>,
+        (const void*)k_shade<kClassMetal>,      (const void*)k_shade<kClassDielectric>,
+        (const void*)k_shade<kClassPrincipled>, (const void*)k_shade<kClassGeneric>};
+    static const void* const learned[kShadeClasses] = {
+        (const void*)k_shade_guided<kClassMiss>,       (const void*)k_shade_guided<kClassLambert>,
+        (const void*)k_shade_guided<kClassMetal>,      (const void*)k_shade_guided<kClassDielectric>,
+        (const void*)k_shade_guided<kClassPrincipled>, (const void*)k_shade_guided<kClassGeneric>};
+    return guided ? learned[c] : plain[c];
+}
+
 // What the shadow rays of a scene have to find out.
 int shadow_mode(const DeviceScene& S, int transparent_shadows) {
     if (transparent_shadows && S.has_clear_glass)
@@ -1398,13 +1421,10 @@ void prefer_l1(int device) {
     if (done.load() & bit)
         return;
     std::vector<const void*> kernels = {
-        (const void*)k_generate, (const void*)k_features,
-        (const void*)k_shade<kClassMiss>, (const void*)k_shade<kClassLambert>, (const void*)k_shade<kClassMetal>,
-        (const void*)k_shade<kClassDielectric>, (const void*)k_shade<kClassPrincipled>,
-        (const void*)k_shade<kClassGeneric>, (const void*)k_shade_guided<kClassMiss>,
-        (const void*)k_shade_guided<kClassLambert>, (const void*)k_shade_guided<kClassMetal>,
-        (const void*)k_shade_guided<kClassDielectric>, (const void*)k_shade_guided<kClassPrincipled>,
-        (const void*)k_shade_guided<kClassGeneric>};
+        (const void*)k_generate, (const void*)k_features<true>, (const void*)k_features<false>};
+    for (int c = 0; c < kShadeClasses; c++)
+        for (bool guided : {false, true})
+            kernels.push_back(shade_kernel(c, guided));
     for (bool vox : {false, true})
         for (int walk : {kWalkBinary, kWalkWide, kWalkPostponed, kWalkWide8, kWalkLanes, kWalkLanesPostponed}) {
             kernels.push_back(extend_kernel(vox, walk));
@@ -1417,8 +1437,10 @@ void prefer_l1(int device) {
     done.fetch_or(bit);
 }
 
-// Grids of `block` threads: SMs x resident blocks (persistent-style loops).
-Launch launch_config(const mypbr_gpu_scene& G, const mypbr_render_opts& o, int block = 0) {
+// Grids of `block` threads: SMs x resident blocks (persistent-style loops),
+// and no more blocks than a wave of `paths` paths has work for (a thousand
+// empty blocks cost a kernel of a small wave more than its work).
+Launch launch_config(const mypbr_gpu_scene& G, const mypbr_render_opts& o, size_t paths, int block = 0) {
     prefer_l1(G.device);
     Launch L{};
     // Traversal 0 is lanes that take new rays, in blocks of 128, which leave
@@ -1451,18 +1473,20 @@ Launch launch_config(const mypbr_gpu_scene& G, const mypbr_render_opts& o, int b
     const void* extend = extend_kernel(vox, L.walk);
     const void* shadow = shadow_kernel(vox, L.shadow_walk, L.shadow_mode);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, extend, L.block, 0);
-    L.grid_extend = G.sm_count * std::max(per_sm, 1);
+    auto grid = [&](int blocks, int threads) {
+        return int(std::min<size_t>(size_t(G.sm_count) * std::max(blocks, 1), (paths + threads - 1) / threads));
+    };
+    L.grid_extend = grid(per_sm, L.block);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, shadow, L.block, 0);
-    L.grid_shadow = G.sm_count * std::max(per_sm, 1);
-    L.grid_stream = G.sm_count * 8;
+    L.grid_shadow = grid(per_sm, L.block);
+    L.grid_stream = grid(8, 256);
+    L.shade_classes = G.shade_classes;
     int worst = 1;
-    for (auto f : {(const void*)k_shade<kClassMiss>, (const void*)k_shade<kClassLambert>,
-                   (const void*)k_shade<kClassMetal>, (const void*)k_shade<kClassDielectric>,
-                   (const void*)k_shade<kClassPrincipled>, (const void*)k_shade<kClassGeneric>}) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, L.block, 0);
+    for (int c = 0; c < kShadeClasses; c++) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, shade_kernel(c, false), L.block, 0);
         worst = std::max(worst, per_sm);
     }
-    L.grid_shade = G.sm_count * worst;
+    L.grid_shade = grid(worst, L.block);
     return L;
 }
 
@@ -1541,7 +1565,10 @@ int run_prefix(WaveParams& P, const Launch& L, cudaStream_t st, uint64_t& launch
     TIMED(0, (k_generate<<<L.grid_stream, 256, 0, st>>>(P, 0)));
     launches++;
     if (P.collect_features) {
-        TIMED(4, (k_features<<<L.grid_shade, 256, 0, st>>>(P, 0)));
+        if (P.S.has_voxels)
+            TIMED(4, (k_features<true><<<L.grid_stream, 256, 0, st>>>(P, 0)));
+        else
+            TIMED(4, (k_features<false><<<L.grid_stream, 256, 0, st>>>(P, 0)));
         launches++;
     }
     return MYPBR_OK;
@@ -1565,23 +1592,13 @@ int run_bounce(WaveParams& P, const Launch& L, cudaStream_t st, uint64_t& launch
                      L.net, GuideQueueSource{P, depth}, GuidePackSink{P}, 0)));
         launches++;
     }
-    if (L.guided_kernels) {
-        TIMED(2, (k_shade_guided<kClassMiss><<<L.grid_shade, L.block, 0, st>>>(P, depth)));
-        TIMED(2, (k_shade_guided<kClassLambert><<<L.grid_shade, L.block, 0, st>>>(P, depth)));
-        TIMED(2, (k_shade_guided<kClassMetal><<<L.grid_shade, L.block, 0, st>>>(P, depth)));
-        TIMED(2, (k_shade_guided<kClassDielectric><<<L.grid_shade, L.block, 0, st>>>(P, depth)));
-        TIMED(2, (k_shade_guided<kClassPrincipled><<<L.grid_shade, L.block, 0, st>>>(P, depth)));
-        TIMED(2, (k_shade_guided<kClassGeneric><<<L.grid_shade, L.block, 0, st>>>(P, depth)));
-    } else {
-        TIMED(2, (k_shade<kClassMiss><<<L.grid_shade, L.block, 0, st>>>(P, depth)));
-        TIMED(2, (k_shade<kClassLambert><<<L.grid_shade, L.block, 0, st>>>(P, depth)));
-        TIMED(2, (k_shade<kClassMetal><<<L.grid_shade, L.block, 0, st>>>(P, depth)));
-        TIMED(2, (k_shade<kClassDielectric><<<L.grid_shade, L.block, 0, st>>>(P, depth)));
-        TIMED(2, (k_shade<kClassPrincipled><<<L.grid_shade, L.block, 0, st>>>(P, depth)));
-        TIMED(2, (k_shade<kClassGeneric><<<L.grid_shade, L.block, 0, st>>>(P, depth)));
-    }
+    for (int c = 0; c < kShadeClasses; c++)
+        if (L.shade_classes >> c & 1u) {
+            TIMED(2, (launch_bounce_kernel(shade_kernel(c, L.guided_kernels), L.grid_shade, L.block, st, P, depth)));
+            launches++;
+        }
     TIMED(3, (launch_bounce_kernel(shadow_kernel(P.S.has_voxels, L.shadow_walk, L.shadow_mode), L.grid_shadow, L.block, st, P, depth)));
-    launches += 3 + kShadeClasses;
+    launches += 3;
     return MYPBR_OK;
 }
 
@@ -1604,6 +1621,13 @@ int run_wave(WaveParams& P, const Launch& L, cudaStream_t st, uint64_t& launches
 // after max_depth bodies at most. The wave's start (counters, camera rays,
 // features) is launched before the graph, with the pass range in device
 // memory (wave_state) set by a one-thread kernel.
+//
+// Kernels that do not need one another are branches of the body: the shading
+// classes, and a bounce's shadow rays beside the next bounce's extension rays
+// (they touch different halves of the throughput records). A small wave's
+// kernels are each one long chain of reads (11 to 17 us for a 4096-path wave
+// of the Cornell box, whatever their work), so the branches take the time of
+// the longest; a large wave's fill each other's last blocks.
 struct WaveGraph {
     cudaGraphExec_t exec = nullptr;
     int key = -1;
@@ -1614,7 +1638,62 @@ struct WaveGraph {
     }
 };
 
-int build_wave_graph(WaveParams& P, const Launch& L, cudaStream_t st, WaveGraph* graph) {
+using Nodes = std::vector<cudaGraphNode_t>;
+
+// A kernel node after `deps`.
+int add_kernel(cudaGraph_t g, const Nodes& deps, const void* fn, int grid, int block, size_t smem, void** args,
+               cudaGraphNode_t& node) {
+    cudaKernelNodeParams kp = {};
+    kp.func = const_cast<void*>(fn);
+    kp.gridDim = dim3(unsigned(grid));
+    kp.blockDim = dim3(unsigned(block));
+    kp.sharedMemBytes = unsigned(smem);
+    kp.kernelParams = args;
+    MYPBR_CUDA(cudaGraphAddKernelNode(&node, g, deps.data(), deps.size(), &kp));
+    return MYPBR_OK;
+}
+
+// One bounce as nodes of g after `deps`; `last` gets the nodes that what
+// follows waits for. beside: the shadow rays are the previous bounce's, beside
+// this one's extension rays (the wave's last are launched after its loop);
+// else they follow the shading.
+int add_bounce(cudaGraph_t g, WaveParams& P, const Launch& L, bool beside, const Nodes& deps, Nodes& last,
+               uint64_t& count) {
+    int s = MYPBR_OK, depth = -1, before = kBounceBefore;
+    cudaGraphNode_t node = nullptr;
+    auto add = [&](const Nodes& after, const void* fn, int grid, int block, size_t smem, void** args) {
+        if (s == MYPBR_OK) {
+            s = add_kernel(g, after, fn, grid, block, smem, args, node);
+            count++;
+        }
+        return node;
+    };
+    void* args[] = {&P, &depth};
+    void* args_before[] = {&P, &before};
+    const void* shadow = shadow_kernel(P.S.has_voxels, L.shadow_walk, L.shadow_mode);
+    Nodes hits = {add(deps, extend_kernel(P.S.has_voxels, L.walk), L.grid_extend, L.block, 0, args)};
+    if (beside)
+        hits.push_back(add(deps, shadow, L.grid_shadow, L.block, 0, args_before));
+    Nodes queued = {add(hits, (const void*)k_classify, L.grid_stream, 256, 0, args)};
+    if (P.guided) {
+        GuideNetView net = L.net;
+        GuideQueueSource source{P, -1};
+        GuidePackSink sink{P};
+        long long rows = 0;
+        void* guide_args[] = {&net, &source, &sink, &rows};
+        queued = {add(queued, (const void*)k_guide_forward<GuideQueueSource, GuidePackSink>, L.grid_guide,
+                      128 * kGuideGroups, L.guide_smem, guide_args)};
+    }
+    last.clear();
+    for (int c = 0; c < kShadeClasses; c++)
+        if (L.shade_classes >> c & 1u)
+            last.push_back(add(queued, shade_kernel(c, L.guided_kernels), L.grid_shade, L.block, 0, args));
+    if (!beside)
+        last = {add(last, shadow, L.grid_shadow, L.block, 0, args)};
+    return s;
+}
+
+int build_wave_graph(WaveParams& P, const Launch& L, WaveGraph* graph) {
     cudaGraph_t g = nullptr;
     MYPBR_CUDA(cudaGraphCreate(&g, 0));
     struct Owned {
@@ -1631,21 +1710,15 @@ int build_wave_graph(WaveParams& P, const Launch& L, cudaStream_t st, WaveGraph*
     cudaGraphNode_t node;
     MYPBR_CUDA(cudaGraphAddNode(&node, g, nullptr, nullptr, 0, &cp));
     cudaGraph_t body = cp.conditional.phGraph_out[0];
-    MYPBR_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     uint64_t n = 0;
-    KernelTimer off;  // no events inside a graph
-    off.st = st;
-    int s = run_bounce(P, L, st, n, off, -1);
-    if (s == MYPBR_OK)
-        k_next_bounce<<<1, 1, 0, st>>>(P, loop);
-    cudaGraph_t captured = nullptr;
-    cudaError_t e = cudaStreamEndCapture(st, &captured);
+    Nodes last;
+    int s = add_bounce(body, P, L, true, {}, last, n);
     if (s != MYPBR_OK)
         return s;
-    if (e != cudaSuccess)
-        return cuda_fail(e, "cudaStreamEndCapture (wave graph body)");
-    MYPBR_CUDA(cudaGetLastError());
-    e = cudaGraphInstantiate(&graph->exec, g, 0);
+    void* args[] = {&P, &loop};
+    if ((s = add_kernel(body, last, (const void*)k_next_bounce, 1, 1, 0, args, node)) != MYPBR_OK)
+        return s;
+    cudaError_t e = cudaGraphInstantiate(&graph->exec, g, 0);
     if (e != cudaSuccess)
         return cuda_fail(e, "cudaGraphInstantiate");
     graph->per_bounce = n + 1;
@@ -1667,7 +1740,7 @@ int launch_wave(WaveParams& P, const Launch& L, cudaStream_t st, uint64_t& launc
             cudaGraphExecDestroy(graph->exec);
             graph->exec = nullptr;
         }
-        int s = build_wave_graph(P, L, st, graph);
+        int s = build_wave_graph(P, L, graph);
         if (s != MYPBR_OK)
             return s;
         graph->key = key;
@@ -1678,6 +1751,9 @@ int launch_wave(WaveParams& P, const Launch& L, cudaStream_t st, uint64_t& launc
     if (s != MYPBR_OK)
         return s;
     MYPBR_CUDA(cudaGraphLaunch(graph->exec, st));
+    launch_bounce_kernel(shadow_kernel(P.S.has_voxels, L.shadow_walk, L.shadow_mode), L.grid_shadow, L.block, st, P,
+                         kBounceBefore);
+    launches++;
     return run_suffix(P, L, st, launches, T);
 }
 
@@ -1765,7 +1841,7 @@ int prepare(mypbr_gpu_scene* G, const mypbr_camera* cam, const mypbr_render_opts
     if (s != MYPBR_OK)
         return s;
     P.B = G->rb;
-    R.L = launch_config(*G, *o);
+    R.L = launch_config(*G, *o, R.npix * size_t(per_wave));
     R.guided = o->guided != 0;
     R.fixed_waves = o->samples_per_wave > 0;
     if (R.guided) {
@@ -2077,8 +2153,8 @@ int job_start(mypbr_batch_job& jb, BatchJob& j) {
 // the whole batch is one graph launch and the GPU schedules the branches.
 
 // Captures job `jb` at the end of the capture running on `st` (whose graph
-// is g); the loop body is captured on `side`.
-int capture_job(const mypbr_batch_job& jb, RenderSetup& R, cudaStream_t st, cudaStream_t side, cudaGraph_t g) {
+// is g); the loop body is built node by node.
+int capture_job(const mypbr_batch_job& jb, RenderSetup& R, cudaStream_t st, cudaGraph_t g) {
     WaveParams& P = R.P;
     size_t full = size_t(P.cam.width) * P.cam.height;
     MYPBR_CUDA(cudaMemsetAsync(P.totals, 0, 3 * sizeof(unsigned long long), st));
@@ -2101,24 +2177,26 @@ int capture_job(const mypbr_batch_job& jb, RenderSetup& R, cudaStream_t st, cuda
     cudaGraphNode_t node;
     MYPBR_CUDA(cudaGraphAddNode(&node, g, deps, nullptr, ndeps, &cp));
     MYPBR_CUDA(cudaStreamUpdateCaptureDependencies(st, &node, nullptr, 1, cudaStreamSetCaptureDependencies));
-    MYPBR_CUDA(cudaStreamBeginCaptureToGraph(side, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                             cudaStreamCaptureModeThreadLocal));
+    cudaGraph_t body = cp.conditional.phGraph_out[0];
     uint64_t n = 0;
-    KernelTimer off;  // no events inside a graph
-    off.st = side;
-    k_generate<<<R.L.grid_stream, 256, 0, side>>>(P, 1);
-    if (P.collect_features)
-        k_features<<<R.L.grid_shade, 256, 0, side>>>(P, 1);
-    int s = run_bounce(P, R.L, side, n, off, -1);
-    k_accumulate<<<R.L.grid_stream, 256, 0, side>>>(P, 1);
-    if (s == MYPBR_OK)
-        k_job_step<<<1, 256, 0, side>>>(P, loop, R.per_wave, R.spp, words);
-    cudaGraph_t body = nullptr;
-    cudaError_t e = cudaStreamEndCapture(side, &body);
-    if (s != MYPBR_OK)
+    int one = 1, spp = R.spp, per_wave = R.per_wave, s = MYPBR_OK;
+    Nodes last;
+    void* gated[] = {&P, &one};
+    cudaGraphNode_t at = nullptr;
+    if ((s = add_kernel(body, {}, (const void*)k_generate, R.L.grid_stream, 256, 0, gated, at)) != MYPBR_OK)
         return s;
-    if (e != cudaSuccess)
-        return cuda_fail(e, "cudaStreamEndCapture (batch job body)");
+    if (P.collect_features) {
+        const void* fn = P.S.has_voxels ? (const void*)k_features<true> : (const void*)k_features<false>;
+        if ((s = add_kernel(body, {at}, fn, R.L.grid_stream, 256, 0, gated, at)) != MYPBR_OK)
+            return s;
+    }
+    if ((s = add_bounce(body, P, R.L, false, {at}, last, n)) != MYPBR_OK ||
+        (s = add_kernel(body, last, (const void*)k_accumulate, R.L.grid_stream, 256, 0, gated, at)) != MYPBR_OK)
+        return s;
+    int counters = words;
+    void* step[] = {&P, &loop, &per_wave, &spp, &counters};
+    if ((s = add_kernel(body, {at}, (const void*)k_job_step, 1, 256, 0, step, at)) != MYPBR_OK)
+        return s;
     k_resolve<<<R.L.grid_stream, 256, 0, st>>>(P, R.spp, jb.radiance, jb.albedo, jb.normal, jb.variance);
     MYPBR_CUDA(cudaGetLastError());
     return MYPBR_OK;
@@ -2196,22 +2274,18 @@ int batch_one_graph(mypbr_batch_job* jobs, int n, const std::vector<mypbr_gpu_sc
             R[size_t(i)].P.totals = c->totals + 3 * size_t(i);
         struct Owned {
             cudaGraph_t g = nullptr;
-            cudaStream_t side = nullptr;
             ~Owned() {
                 if (g)
                     cudaGraphDestroy(g);
-                if (side)
-                    cudaStreamDestroy(side);
             }
         } o;
-        MYPBR_CUDA(cudaStreamCreateWithFlags(&o.side, cudaStreamNonBlocking));
         MYPBR_CUDA(cudaGraphCreate(&o.g, 0));
         for (size_t k = 0; k < scenes.size(); k++) {
             cudaStream_t sk = scenes[k]->stream;
             MYPBR_CUDA(cudaStreamBeginCaptureToGraph(sk, o.g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
             int s = MYPBR_OK;
             for (int i : order[k]) {
-                s = capture_job(jobs[i], R[size_t(i)], sk, o.side, o.g);
+                s = capture_job(jobs[i], R[size_t(i)], sk, o.g);
                 if (s != MYPBR_OK)
                     break;
             }
@@ -2586,7 +2660,7 @@ extern "C" int mypbr_gpu_render_noalloc(mypbr_gpu_scene* G, const mypbr_camera* 
     P.B.film -= 3 * first_pixel;
     P.B.film2 -= 3 * first_pixel;
     P.B.feat -= 7 * first_pixel;
-    Launch L = launch_config(*G, *o);
+    Launch L = launch_config(*G, *o, npix * size_t(per_wave));
     uint64_t launches = 0;
     KernelTimer T;  // off: no events are created
     T.st = st;

@@ -380,6 +380,35 @@ int create_scene(const mypbr_flat_scene* Fp, mypbr_gpu_scene** out) {
         for (int64_t k = 0; k < F.bvh_prim_count; k++)
             refs[size_t(k)] = (uint32_t(F.bvh_prims[k].kind) << kKindShift) | uint32_t(F.bvh_prims[k].index);
     }
+    // the surfaces that can emit, where no voxel does and they are few: their
+    // references follow the leaves', so that one launch packs both
+    std::vector<uint32_t> glowing;
+    {
+        auto emits = [&](int64_t m) {
+            return F.materials[m].type == MYPBR_MAT_DIFFUSE_LIGHT || F.materials[m].emission_tex >= 0;
+        };
+        bool few = true;
+        for (int64_t k = 0; few && k < F.voxel_palette_count; k++)
+            few = F.voxel_palettes[k].kind == 0 || !emits(F.voxel_palettes[k].material);
+        for (int64_t k = 0; few && k < F.voxel_model_count; k++)
+            few = F.voxel_models[k].edge_material < 0 || !emits(F.voxel_models[k].edge_material);
+        for (int64_t k = 0; few && k < F.bvh_prim_count; k++) {
+            const auto& p = F.bvh_prims[k];
+            const int64_t m = p.kind == MYPBR_PRIM_SPHERE     ? F.spheres[p.index].material
+                              : p.kind == MYPBR_PRIM_QUAD     ? F.quads[p.index].material
+                              : p.kind == MYPBR_PRIM_TRIANGLE ? F.triangles[p.index].material
+                                                              : -1;
+            if (m >= 0 && emits(m)) {
+                glowing.push_back((uint32_t(p.kind) << kKindShift) | uint32_t(p.index));
+                few = glowing.size() <= kFewEmitters;
+            }
+        }
+        D.emitter_count = few ? int(glowing.size()) : -1;
+        if (!few)
+            glowing.clear();
+    }
+    G.leaf_ref_count = refs.size();
+    refs.insert(refs.end(), glowing.begin(), glowing.end());
     PUT(nodes, D.bvh);
     PUT(refs, D.leaf_refs);
     D.bvh_node_count = interior;
@@ -430,7 +459,6 @@ int create_scene(const mypbr_flat_scene* Fp, mypbr_gpu_scene** out) {
         PUT(zero, err);
         D.error = const_cast<int*>(err);
     }
-    G.leaf_ref_count = refs.size();
 
     // ---- primitives
     std::vector<float4> spheres;
@@ -602,6 +630,7 @@ int create_scene(const mypbr_flat_scene* Fp, mypbr_gpu_scene** out) {
         else if (plain && m.type == MYPBR_MAT_PRINCIPLED)
             c = 4;
         cls.push_back(c);
+        G.shade_classes |= 1u << c;
     }
     PUT(cls, D.mat_class);
     for (int64_t k = 0; k < F.material_count; k++) {
@@ -738,42 +767,15 @@ int create_scene(const mypbr_flat_scene* Fp, mypbr_gpu_scene** out) {
                                      float(F.sun.irradiance[2] / omega));
     }
     D.leaf_tails = F.triangle_count > 0 || F.quad_count > 0;
-    if (int st = build_leaves(&G); st != MYPBR_OK)
-        return fail_cleanup(st);
+    if (!refs.empty()) {
+        float4* records = nullptr;
+        if (int st = pack_leaves(&G, D.leaf_refs, int(refs.size()), records); st != MYPBR_OK)
+            return fail_cleanup(st);
+        D.leaves = records;
+        D.emitters = records + 4 * G.leaf_ref_count;
+    }
     D.dark_sky = D.env_w == 0 && !F.use_sky && !D.sun_enabled && F.background[0] == 0 && F.background[1] == 0 &&
                  F.background[2] == 0;
-    {
-        // the surfaces that can emit, where no voxel does and they are few
-        auto emits = [&](int64_t m) {
-            return F.materials[m].type == MYPBR_MAT_DIFFUSE_LIGHT || F.materials[m].emission_tex >= 0;
-        };
-        std::vector<uint32_t> glowing;
-        bool few = true;
-        for (int64_t k = 0; few && k < F.voxel_palette_count; k++)
-            few = F.voxel_palettes[k].kind == 0 || !emits(F.voxel_palettes[k].material);
-        for (int64_t k = 0; few && k < F.voxel_model_count; k++)
-            few = F.voxel_models[k].edge_material < 0 || !emits(F.voxel_models[k].edge_material);
-        for (int64_t k = 0; few && k < F.bvh_prim_count; k++) {
-            const auto& p = F.bvh_prims[k];
-            const int64_t m = p.kind == MYPBR_PRIM_SPHERE     ? F.spheres[p.index].material
-                              : p.kind == MYPBR_PRIM_QUAD     ? F.quads[p.index].material
-                              : p.kind == MYPBR_PRIM_TRIANGLE ? F.triangles[p.index].material
-                                                              : -1;
-            if (m >= 0 && emits(m)) {
-                glowing.push_back((uint32_t(p.kind) << kKindShift) | uint32_t(p.index));
-                few = glowing.size() <= kFewEmitters;
-            }
-        }
-        D.emitter_count = few ? int(glowing.size()) : -1;
-        if (few && !glowing.empty()) {
-            const uint32_t* refs = nullptr;
-            float4* records = nullptr;
-            PUT(glowing, refs);
-            if (int st = pack_leaves(&G, refs, int(glowing.size()), records); st != MYPBR_OK)
-                return fail_cleanup(st);
-            D.emitters = records;
-        }
-    }
     G.material_count = F.material_count;
     D.use_sky = F.use_sky;
     D.background = make_float3(float(F.background[0]), float(F.background[1]), float(F.background[2]));
