@@ -15,6 +15,7 @@
 
 #include "dev_math.cuh"
 #include "gpu_scene.h"
+#include "transfer.h"
 
 namespace mypbr_dev {
 namespace {
@@ -158,14 +159,6 @@ __global__ void k_dn_finish(const float4* L, const double* alb, double* out, int
     }
 }
 
-struct Buf {
-    void* p = nullptr;
-    ~Buf() {
-        if (p)
-            cudaFree(p);
-    }
-};
-
 int bad(const std::string& m) {
     set_error_message(m);
     return MYPBR_ERR_INVALID_ARGUMENT;
@@ -205,29 +198,31 @@ extern "C" int mypbr_gpu_denoise(const double* radiance, const double* albedo, c
     MYPBR_CUDA(cudaGetDevice(&dev));
     int sms = 1;
     MYPBR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    Buf bL0, bL1, bA, bN, bBV, din[4], dout;
-    MYPBR_CUDA(cudaMalloc(&bL0.p, n * sizeof(float4)));
-    MYPBR_CUDA(cudaMalloc(&bL1.p, n * sizeof(float4)));
-    MYPBR_CUDA(cudaMalloc(&bA.p, n * sizeof(float4)));
-    MYPBR_CUDA(cudaMalloc(&bN.p, n * sizeof(float4)));
-    MYPBR_CUDA(cudaMalloc(&bBV.p, n * sizeof(float)));
+    // five planes, and with host buffers the frame in and out (Workspace keeps
+    // them for the next frame: allocating and freeing them took longer than the
+    // filter, 1.27 ms a 1080p frame against 0.5)
+    Workspace mem;
+    const size_t planes = 4 * Workspace::padded<float4>(n) + Workspace::padded<float>(n);
+    const size_t frame = on_device ? 0 : 4 * Workspace::padded<double>(3 * n) + Workspace::padded<double>(n);
+    if (int s = mem.reserve(planes + frame); s != MYPBR_OK)
+        return s;
+    float4* L0 = mem.take<float4>(n);
+    float4* L1 = mem.take<float4>(n);
+    float4* A = mem.take<float4>(n);
+    float4* N = mem.take<float4>(n);
+    float* BV = mem.take<float>(n);
     const double* in[4] = {radiance, albedo, normal, variance};
     double* dst = out;
     if (!on_device) {
         size_t sizes[4] = {3 * n, 3 * n, 3 * n, n};
         for (int k = 0; k < 4; k++) {
-            MYPBR_CUDA(cudaMalloc(&din[k].p, sizes[k] * sizeof(double)));
-            MYPBR_CUDA(cudaMemcpy(din[k].p, in[k], sizes[k] * sizeof(double), cudaMemcpyHostToDevice));
-            in[k] = static_cast<const double*>(din[k].p);
+            double* d = mem.take<double>(sizes[k]);
+            if (int s = copy_to_device(d, in[k], sizes[k] * sizeof(double)); s != MYPBR_OK)
+                return s;
+            in[k] = d;
         }
-        MYPBR_CUDA(cudaMalloc(&dout.p, 3 * n * sizeof(double)));
-        dst = static_cast<double*>(dout.p);
+        dst = mem.take<double>(3 * n);
     }
-    float4* L0 = static_cast<float4*>(bL0.p);
-    float4* L1 = static_cast<float4*>(bL1.p);
-    float4* A = static_cast<float4*>(bA.p);
-    float4* N = static_cast<float4*>(bN.p);
-    float* BV = static_cast<float*>(bBV.p);
     int blocks = int(std::min<size_t>((n + 255) / 256, size_t(sms) * 16));
     k_dn_prepare<<<blocks, 256>>>(in[0], in[1], in[2], in[3], int(n), L0, A, N);
     k_dn_fireflies<<<blocks, 256>>>(L0, L1, width, height);
@@ -248,8 +243,7 @@ extern "C" int mypbr_gpu_denoise(const double* radiance, const double* albedo, c
     k_dn_finish<<<blocks, 256>>>(cur, in[1], dst, int(n));
     MYPBR_CUDA(cudaGetLastError());
     if (!on_device)
-        MYPBR_CUDA(cudaMemcpy(out, dst, 3 * n * sizeof(double), cudaMemcpyDeviceToHost));
-    else
-        MYPBR_CUDA(cudaDeviceSynchronize());
+        return copy_to_host(out, dst, 3 * n * sizeof(double), nullptr);
+    MYPBR_CUDA(cudaDeviceSynchronize());
     return MYPBR_OK;
 }

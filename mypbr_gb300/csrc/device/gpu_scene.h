@@ -90,6 +90,9 @@ struct mypbr_gpu_scene {
     int64_t material_count = 0;
     uint32_t shade_classes = 1u;  // bit c: paths can meet shading class c (0, a miss, always)
     mypbr_dev::RenderBuffers rb;
+    unsigned long long* totals = nullptr;  // a render's ray totals (3)
+    double* frame = nullptr;               // the planes of renders with host outputs, kept like the scratch
+    size_t frame_doubles = 0;
     mypbr_dev::GuideState guide;
     float3 box_lo{-1.0f, -1.0f, -1.0f}, box_hi{1.0f, 1.0f, 1.0f};  // bounds of the BVH's primitives
     cudaStream_t stream = nullptr;  // the handle's own stream, for renders with host buffers (graph capture needs one)

@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "gpu_scene.h"
+#include "transfer.h"
 
 namespace mypbr_dev {
 
@@ -115,7 +116,6 @@ __device__ void sample(const Img& m, double x, double y, double* c) {
 struct Display {
     double scale;  // 2^exposure
     int op;        // MYPBR_TONEMAP_*
-    int bytes;     // 1: quantise to 8-bit sRGB; 0: keep linear (postprocess only)
     double bloom, vignette;
 };
 
@@ -160,6 +160,8 @@ __device__ unsigned char to_byte(double x) {  // color3.h:17-36
     return (unsigned char)(256 * s);
 }
 
+// The post-processed pixel, kept linear (lin) and as display bytes (rgb8),
+// either of which may be null: one pass over the bloom levels for both.
 __global__ void k_compose(const double* in, int w, int h, Levels L, Display D, double* lin, unsigned char* rgb8) {
     int n = w * h;
     double cx = 0.5 * w, cy = 0.5 * h;
@@ -190,41 +192,52 @@ __global__ void k_compose(const double* in, int w, int h, Levels L, Display D, d
             c[1] = inv * c[1];
             c[2] = inv * c[2];
         }
-        if (D.bytes) {
-            apply(D, c);
-            rgb8[3 * size_t(k)] = to_byte(c[0]);
-            rgb8[3 * size_t(k) + 1] = to_byte(c[1]);
-            rgb8[3 * size_t(k) + 2] = to_byte(c[2]);
-        } else {
+        if (lin) {
             lin[3 * size_t(k)] = c[0];
             lin[3 * size_t(k) + 1] = c[1];
             lin[3 * size_t(k) + 2] = c[2];
         }
+        if (rgb8) {
+            apply(D, c);
+            rgb8[3 * size_t(k)] = to_byte(c[0]);
+            rgb8[3 * size_t(k) + 1] = to_byte(c[1]);
+            rgb8[3 * size_t(k) + 2] = to_byte(c[2]);
+        }
     }
 }
 
-struct DevMem {
-    std::vector<void*> ptrs;
-    ~DevMem() {
-        for (void* p : ptrs)
-            cudaFree(p);
-    }
-    template <typename T>
-    int get(T*& p, size_t n) {
-        void* q = nullptr;
-        MYPBR_CUDA(cudaMalloc(&q, std::max<size_t>(n, 1) * sizeof(T)));
-        ptrs.push_back(q);
-        p = static_cast<T*>(q);
-        return MYPBR_OK;
-    }
-};
-
 int grid_for(size_t n) { return int(std::min<size_t>((n + 255) / 256, 152 * 16)); }
 
-// Bloom, vignette and (bytes) the display transform of a device image.
-int run_post(const double* d_in, int w, int h, const mypbr_display_opts& o, bool bytes, double* d_lin,
-             unsigned char* d_rgb8) {
-    DevMem mem;
+// The bloom pyramid's levels of a w x h image: the sizes of its half-size images.
+int bloom_levels(int w, int h, const mypbr_display_opts& o, Img* sizes) {
+    if (!(o.bloom > 0))
+        return 0;
+    double reach = std::fmax(o.bloom_radius * w, 1.0);
+    int levels = std::clamp(int(std::ceil(std::log2(reach))), 1, 10);
+    int n = 0;
+    for (; n < levels && w > 1 && h > 1; n++) {
+        w = std::max(1, w / 2);
+        h = std::max(1, h / 2);
+        sizes[n] = Img{w, h, nullptr};
+    }
+    return n;
+}
+
+size_t image_bytes(int w, int h) { return Workspace::padded<double>(3 * size_t(w) * h); }
+
+// The workspace run_post takes.
+size_t post_bytes(int w, int h, const mypbr_display_opts& o) {
+    Img sizes[10];
+    const int levels = bloom_levels(w, h, o, sizes);
+    size_t bytes = o.bloom > 0 ? image_bytes(w, h) : 0;
+    for (int k = 0; k < levels; k++)
+        bytes += 3 * image_bytes(sizes[k].w, sizes[k].h);
+    return bytes;
+}
+
+// Bloom, vignette and the display transform of a device image.
+int run_post(const double* d_in, int w, int h, const mypbr_display_opts& o, double* d_lin, unsigned char* d_rgb8,
+             Workspace& mem) {
     Levels L{};
     size_t n = size_t(w) * h;
     if (o.bloom > 0) {
@@ -235,28 +248,24 @@ int run_post(const double* d_in, int w, int h, const mypbr_display_opts& o, bool
         for (double& k : kernel)
             k /= sum;
         MYPBR_CUDA(cudaMemcpyToSymbol(c_blur, kernel, sizeof kernel));
-        Img bright{w, h, nullptr};
-        int s = mem.get(bright.px, 3 * n);
-        if (s != MYPBR_OK)
-            return s;
-        k_bright<<<grid_for(n), 256>>>(d_in, int(n), o.bloom_threshold, bright.px);
-        double reach = std::fmax(o.bloom_radius * w, 1.0);
-        int levels = std::clamp(int(std::ceil(std::log2(reach))), 1, 10);
-        Img level = bright;
-        for (int k = 0; k < levels && level.w > 1 && level.h > 1; k++) {
-            Img down{std::max(1, level.w / 2), std::max(1, level.h / 2), nullptr};
-            Img tmp = down, blurred = down;
+        Img level{w, h, mem.take<double>(3 * n)};
+        k_bright<<<grid_for(n), 256>>>(d_in, int(n), o.bloom_threshold, level.px);
+        Img sizes[10];
+        L.n = bloom_levels(w, h, o, sizes);
+        for (int k = 0; k < L.n; k++) {
+            Img down = sizes[k], tmp = sizes[k], blurred = sizes[k];
             size_t m = size_t(down.w) * down.h;
-            if ((s = mem.get(down.px, 3 * m)) || (s = mem.get(tmp.px, 3 * m)) || (s = mem.get(blurred.px, 3 * m)))
-                return s;
+            down.px = mem.take<double>(3 * m);
+            tmp.px = mem.take<double>(3 * m);
+            blurred.px = mem.take<double>(3 * m);
             k_down<<<grid_for(m), 256>>>(level, down);
             k_blur<<<grid_for(m), 256>>>(down, tmp, 1);
             k_blur<<<grid_for(m), 256>>>(tmp, blurred, 0);
-            L.lv[L.n++] = blurred;
+            L.lv[k] = blurred;
             level = down;
         }
     }
-    Display D{std::pow(2.0, o.exposure), o.tonemap, bytes ? 1 : 0, o.bloom, o.vignette};
+    Display D{std::pow(2.0, o.exposure), o.tonemap, o.bloom, o.vignette};
     k_compose<<<grid_for(n), 256>>>(d_in, w, h, L, D, d_lin, d_rgb8);
     MYPBR_CUDA(cudaGetLastError());
     MYPBR_CUDA(cudaDeviceSynchronize());
@@ -438,34 +447,27 @@ int mypbr_gpu_display(const double* radiance, int32_t w, int32_t h, const mypbr_
     if (opts)
         o = *opts;
     size_t n = size_t(w) * h;
-    DevMem mem;
+    // host frames go through a kept workspace and are copied by several threads
+    Workspace mem;
+    const size_t staged = on_device ? 0 : 2 * image_bytes(w, h) + Workspace::padded<unsigned char>(3 * n);
+    if ((s = mem.reserve(post_bytes(w, h, o) + staged)) != MYPBR_OK)
+        return s;
     const double* d_in = radiance;
+    double* d_lin = linear;
+    unsigned char* d_b = rgb8;
     if (!on_device) {
-        double* p;
-        if ((s = mem.get(p, 3 * n)) != MYPBR_OK)
+        double* p = mem.take<double>(3 * n);
+        if ((s = copy_to_device(p, radiance, 3 * n * sizeof(double))) != MYPBR_OK)
             return s;
-        MYPBR_CUDA(cudaMemcpy(p, radiance, 3 * n * sizeof(double), cudaMemcpyHostToDevice));
         d_in = p;
+        d_lin = linear ? mem.take<double>(3 * n) : nullptr;
+        d_b = rgb8 ? mem.take<unsigned char>(3 * n) : nullptr;
     }
-    if (linear) {
-        double* d_lin = linear;
-        if (!on_device && (s = mem.get(d_lin, 3 * n)) != MYPBR_OK)
-            return s;
-        if ((s = run_post(d_in, w, h, o, false, d_lin, nullptr)) != MYPBR_OK)
-            return s;
-        if (!on_device)
-            MYPBR_CUDA(cudaMemcpy(linear, d_lin, 3 * n * sizeof(double), cudaMemcpyDeviceToHost));
-    }
-    if (rgb8) {
-        unsigned char* d_b = rgb8;
-        if (!on_device && (s = mem.get(d_b, 3 * n)) != MYPBR_OK)
-            return s;
-        if ((s = run_post(d_in, w, h, o, true, nullptr, d_b)) != MYPBR_OK)
-            return s;
-        if (!on_device)
-            MYPBR_CUDA(cudaMemcpy(rgb8, d_b, 3 * n, cudaMemcpyDeviceToHost));
-    }
-    return MYPBR_OK;
+    if ((s = run_post(d_in, w, h, o, d_lin, d_b, mem)) != MYPBR_OK || on_device)
+        return s;
+    if (linear && (s = copy_to_host(linear, d_lin, 3 * n * sizeof(double), nullptr)) != MYPBR_OK)
+        return s;
+    return rgb8 ? copy_to_host(rgb8, d_b, 3 * n, nullptr) : MYPBR_OK;
 }
 
 int mypbr_write_image(const char* path, const double* radiance, int32_t w, int32_t h, const mypbr_display_opts* opts,

@@ -30,6 +30,7 @@
 #include "../host/host_math.h"
 #include "dev_shading.cuh"
 #include "gpu_scene.h"
+#include "transfer.h"
 
 namespace mypbr_dev {
 
@@ -1246,7 +1247,12 @@ namespace {
 
 template <typename T>
 int alloc(T*& p, size_t count) {
-    MYPBR_CUDA(cudaMalloc(reinterpret_cast<void**>(&p), std::max<size_t>(count, 1) * sizeof(T)));
+    const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
+    if (cudaMalloc(reinterpret_cast<void**>(&p), bytes) == cudaSuccess)
+        return MYPBR_OK;
+    cudaGetLastError();
+    release_workspaces();  // what calls without a handle keep between them
+    MYPBR_CUDA(cudaMalloc(reinterpret_cast<void**>(&p), bytes));
     return MYPBR_OK;
 }
 
@@ -1928,23 +1934,22 @@ int render_wave(mypbr_gpu_scene* G, RenderSetup& R, int wave, int pass0, int sav
     return MYPBR_OK;
 }
 
-struct Totals {
-    unsigned long long* d = nullptr;
-    ~Totals() {
-        if (d)
-            cudaFree(d);
-    }
-};
+// The handle's ray totals, cleared on st.
+int clear_totals(mypbr_gpu_scene* G, WaveParams& P, cudaStream_t st) {
+    if (!G->totals)
+        MYPBR_CUDA(cudaMalloc(&G->totals, 3 * sizeof(unsigned long long)));
+    MYPBR_CUDA(cudaMemsetAsync(G->totals, 0, 3 * sizeof(unsigned long long), st));
+    P.totals = G->totals;
+    return MYPBR_OK;
+}
 
 int render_all(mypbr_gpu_scene* G, RenderSetup& R, cudaStream_t st, double* d_rad, double* d_alb, double* d_nrm,
                double* d_var, double* d_chvar, int save_every, mypbr_pass_callback cb, void* user,
                double* h_rad, double* h_alb, double* h_nrm, double* h_var, mypbr_render_stats* stats) {
     NvtxRange range("mypbr render");
     WaveParams& P = R.P;
-    Totals tot;
-    MYPBR_CUDA(cudaMalloc(&tot.d, 3 * sizeof(unsigned long long)));
-    MYPBR_CUDA(cudaMemsetAsync(tot.d, 0, 3 * sizeof(unsigned long long), st));
-    P.totals = tot.d;
+    if (int s = clear_totals(G, P, st); s != MYPBR_OK)
+        return s;
     P.moments = d_chvar != nullptr;
     size_t full = size_t(P.cam.width) * P.cam.height;
     MYPBR_CUDA(cudaMemsetAsync(P.B.film, 0, 3 * full * sizeof(double), st));
@@ -2000,7 +2005,7 @@ int render_all(mypbr_gpu_scene* G, RenderSetup& R, cudaStream_t st, double* d_ra
     if (stats) {
         *stats = mypbr_render_stats{};
         unsigned long long t[3];
-        MYPBR_CUDA(cudaMemcpyAsync(t, tot.d, sizeof t, cudaMemcpyDeviceToHost, st));
+        MYPBR_CUDA(cudaMemcpyAsync(t, G->totals, sizeof t, cudaMemcpyDeviceToHost, st));
         MYPBR_CUDA(cudaStreamSynchronize(st));
         stats->paths = uint64_t(R.npix) * uint64_t(R.spp);
         stats->extension_rays = t[0];
@@ -2028,8 +2033,19 @@ extern "C" int mypbr_gpu_render_device(mypbr_gpu_scene* G, const mypbr_camera* c
     int s = prepare(G, cam, opts, 0, R);
     if (s != MYPBR_OK)
         return s;
-    return render_all(G, R, static_cast<cudaStream_t>(cuda_stream), d_radiance, d_albedo, d_normal, d_variance,
-                      nullptr, 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, stats);
+    cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
+    s = render_all(G, R, st, d_radiance, d_albedo, d_normal, d_variance, nullptr, 0, nullptr, nullptr, nullptr, nullptr,
+                   nullptr, nullptr, stats);
+    if (s != MYPBR_OK)
+        return s;
+    // the render is done when the call returns (the handle's scratch serves
+    // the next one on any stream), unless the caller is capturing it
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (st != nullptr)
+        MYPBR_CUDA(cudaStreamIsCapturing(st, &capturing));
+    if (capturing == cudaStreamCaptureStatusNone)
+        MYPBR_CUDA(cudaStreamSynchronize(st));
+    return MYPBR_OK;
 }
 
 namespace {
@@ -2059,37 +2075,39 @@ extern "C" int mypbr_gpu_render_ex(mypbr_gpu_scene* G, const mypbr_camera* cam, 
     // only the band's rows come back.
     size_t full = size_t(R.P.cam.width) * R.P.cam.height;
     size_t off = size_t(R.P.first_row) * R.P.cam.width, n = R.npix;
-    DevBuf rad, alb, nrm, var, chv;
-    MYPBR_CUDA(cudaMalloc(&rad.p, 3 * full * sizeof(double)));
+    const size_t need = full * size_t(3 + (feats ? 7 : 0) + (channel_variance ? 3 : 0));
+    if (G->frame_doubles < need) {
+        cudaFree(G->frame);
+        G->frame = nullptr;
+        G->frame_doubles = 0;
+        MYPBR_CUDA(cudaMalloc(&G->frame, need * sizeof(double)));
+        G->frame_doubles = need;
+    }
+    double* const rad = G->frame;
+    double *alb = nullptr, *nrm = nullptr, *var = nullptr, *chv = nullptr, *next = rad + 3 * full;
     if (feats) {
-        MYPBR_CUDA(cudaMalloc(&alb.p, 3 * full * sizeof(double)));
-        MYPBR_CUDA(cudaMalloc(&nrm.p, 3 * full * sizeof(double)));
-        MYPBR_CUDA(cudaMalloc(&var.p, full * sizeof(double)));
+        alb = next;
+        nrm = alb + 3 * full;
+        var = nrm + 3 * full;
+        next = var + full;
     }
     if (channel_variance)
-        MYPBR_CUDA(cudaMalloc(&chv.p, 3 * full * sizeof(double)));
+        chv = next;
     cudaStream_t st = G->stream;
-    s = render_all(G, R, st, rad.p, alb.p, nrm.p, var.p, chv.p, save_every, on_pass, user, radiance,
+    s = render_all(G, R, st, rad, alb, nrm, var, chv, save_every, on_pass, user, radiance,
                    feats ? albedo : nullptr, feats ? normal : nullptr, feats ? variance : nullptr, stats);
     if (s != MYPBR_OK)
         return s;
     auto back = [&](double* host, const double* dev, size_t per_pixel) {
-        return cudaMemcpyAsync(host + per_pixel * off, dev + per_pixel * off, per_pixel * n * sizeof(double),
-                               cudaMemcpyDeviceToHost, st);
+        if (s == MYPBR_OK && host && dev)
+            s = copy_to_host(host + per_pixel * off, dev + per_pixel * off, per_pixel * n * sizeof(double), st);
     };
-    MYPBR_CUDA(back(radiance, rad.p, 3));
-    if (feats) {
-        if (albedo)
-            MYPBR_CUDA(back(albedo, alb.p, 3));
-        if (normal)
-            MYPBR_CUDA(back(normal, nrm.p, 3));
-        if (variance)
-            MYPBR_CUDA(back(variance, var.p, 1));
-    }
-    if (channel_variance)
-        MYPBR_CUDA(back(channel_variance, chv.p, 3));
-    MYPBR_CUDA(cudaStreamSynchronize(st));
-    return check_device_error(G);
+    back(radiance, rad, 3);
+    back(albedo, alb, 3);
+    back(normal, nrm, 3);
+    back(variance, var, 1);
+    back(channel_variance, chv, 3);
+    return s == MYPBR_OK ? check_device_error(G) : s;
 }
 
 extern "C" int mypbr_gpu_render(mypbr_gpu_scene* G, const mypbr_camera* cam, const mypbr_render_opts* opts,
@@ -2114,7 +2132,6 @@ struct BatchJob {
     RenderSetup R;
     WaveGraph graph;
     KernelTimer T;
-    Totals tot;
     uint64_t launches = 0;
     int pass0 = 0, wave = 0;
     bool started = false;
@@ -2129,9 +2146,8 @@ int job_start(mypbr_batch_job& jb, BatchJob& j) {
         return s;
     WaveParams& P = j.R.P;
     cudaStream_t st = G->stream;
-    MYPBR_CUDA(cudaMalloc(&j.tot.d, 3 * sizeof(unsigned long long)));
-    MYPBR_CUDA(cudaMemsetAsync(j.tot.d, 0, 3 * sizeof(unsigned long long), st));
-    P.totals = j.tot.d;
+    if ((s = clear_totals(G, P, st)) != MYPBR_OK)
+        return s;
     size_t full = size_t(P.cam.width) * P.cam.height;
     MYPBR_CUDA(cudaMemsetAsync(P.B.film, 0, 3 * full * sizeof(double), st));
     if (P.collect_features)

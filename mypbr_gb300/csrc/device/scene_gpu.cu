@@ -1100,6 +1100,8 @@ extern "C" void mypbr_gpu_scene_destroy(mypbr_gpu_scene* scene) {
         return;
     mypbr_dev::release_batch_graph(scene);
     mypbr_dev::release_buffers(scene->rb);
+    cudaFree(scene->totals);
+    cudaFree(scene->frame);
     mypbr_dev::release_guide(scene->guide);
     for (void* p : scene->allocations)
         cudaFree(p);
