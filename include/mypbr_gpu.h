@@ -628,12 +628,11 @@ int mypbr_gpu_render_batch(mypbr_batch_job* jobs, int32_t n);
 
 /* The autotuner's choice for a scene handle and view: threads per block of
  * the bounce kernels, paths per wave and the traversal scheme (1: lanes take
- * new rays as theirs finish; 2: each lane walks its ray to the end over the
+ * new rays as theirs finish, the default; 2: each lane walks its ray to the end over the
  * tree collapsed to 4 children per node; 3: the binary tree with leaves
  * postponed until the warp's lanes all hold one; 4: the plain binary walk;
  * 5: each lane walks the tree collapsed to 8 children per node with
- * quantised boxes; 0, the default, is 4 for trees whose leaves are mostly
- * spheres and 3 otherwise), with the Mpaths/s of each of the 40 trials
+ * quantised boxes), with the Mpaths/s of each of the 40 trials
  * (traversal 1 to 5; within each, block 128 then 256; within each, 16M,
  * 32M, 64M, 128M paths; 0 for trials skipped because the scene's tree does
  * not allow that walk). */
@@ -646,12 +645,13 @@ typedef struct mypbr_tune_result {
 } mypbr_tune_result;
 
 /* Sets the launch settings the autotuner would set (0 keeps a setting's
- * default: block 256, 128M paths per wave for plain renders and 32M for
- * guided ones, traversal 0). Traversal: 0 the
- * scene's default, 1 lanes that take new rays, 2 the 4-wide tree, 3 postponed
- * leaves, 4 the plain binary walk, 5 the 8-wide tree with quantised boxes. A
- * traversal the scene's tree does not allow (2 or 5 without that tree, 3 or
- * 5 with leaves of 16 or more references) walks the plain binary tree. */
+ * default: block 128 with traversal 1 and 256 with the others, 128M paths per
+ * wave for plain renders and 32M for guided ones, traversal 1). Traversal: 1
+ * lanes that take new rays (leaves postponed, unless spheres fill most of
+ * them), 2 the 4-wide tree, 3 postponed leaves, 4 the plain binary walk, 5 the
+ * 8-wide tree with quantised boxes. A traversal the scene's tree does not allow
+ * (2 or 5 without that tree, 1, 3 or 5 with leaves of 16 or more references, 1
+ * with voxel models in a tree of mostly spheres) walks the plain binary tree. */
 int mypbr_gpu_set_launch(mypbr_gpu_scene* scene, int32_t block, int64_t wave_paths, int32_t traversal);
 
 /* Times short renders of the view with each setting and keeps the fastest on
