@@ -47,9 +47,8 @@ the oracle beside it; with --hidden H the triangle room also renders guided
 and compares plain and guided relMSE at equal time against --c3-ref-spp.
 batch: C4, 64 scenes in one mypbr_gpu_render_batch call with feature guides,
 every frame denoised, per-scene relMSE against 4x-spp renders.
---traversal 0..5 picks the walk (the scene's default: postponed leaves where
-triangles fill most leaves, else binary; lanes taking new rays; 4-wide tree;
-postponed leaves; plain binary; 8-wide tree with quantised boxes), --block
+--traversal 0..5 picks the walk (the default, lanes taking new rays; the same;
+4-wide tree; postponed leaves; plain binary; 8-wide tree with quantised boxes), --block
 the threads per block.
 
 --impl reference times the CPU implementation of the same path (the FP64
@@ -81,10 +80,10 @@ WIDTH, HEIGHT = 1920, 1080
 # (ray records in, hit records and queue entries out, the tree staying in L2)
 # and the issue figures of bounces 0 and 1.
 EXTEND_PROFILE = {
-    "profile": "profiles/k_extend_sphere_field_1080p.md",
-    "commit": "c7bbfab",
-    "dram_bytes": 298.96e6 + 135.59e6, "rays": 8294400,
-    "issue_active_frac": [0.600, 0.620], "threads_per_instruction": [26.57, 12.92],
+    "profile": "profiles/k_extend_lanes_sphere_field_1080p.md",
+    "commit": "0b9b04f",
+    "dram_bytes": 265.77e6 + 112.12e6, "rays": 8294400,
+    "issue_active_frac": [0.710, 0.694], "threads_per_instruction": [28.52, 16.50],
 }
 EXTEND_DRAM_BYTES_PER_RAY = EXTEND_PROFILE["dram_bytes"] / EXTEND_PROFILE["rays"]
 METRIC = "Mpaths/s at 1080p"
@@ -369,10 +368,10 @@ def run_ours(args):
 
     if rank == 0:
         # roofline of the dominant kernel, extend: algorithmic bytes per ray =
-        # ray record read (origin + tmin, direction + pdf: 32 B) + queue index
-        # (4 B) + hit record written (16 B)
+        # ray record read (origin + flags, direction + pdf: 32 B), hit record
+        # (16 B) and shading class (1 B) written
         ms_ext = kst.ms_extend / max(kst.launches_extend, 1)
-        bytes_per_ray = 52
+        bytes_per_ray = 49
         ext_per_launch = kst.extension_rays / max(kst.launches_extend, 1)
         achieved = bytes_per_ray * ext_per_launch / (ms_ext * 1e-3) / 1e9 if ms_ext > 0 else 0.0
         peak = None
@@ -870,7 +869,7 @@ def main():
                    help="hall_render: every kernel launched on its own with events (profilers cannot look inside "
                         "graphs with conditional nodes)")
     p.add_argument("--traversal", type=int, default=0, choices=[0, 1, 2, 3, 4, 5],
-                   help="0: the scene's default; 1: extend lanes take new rays as theirs finish; 2: the 4-wide "
+                   help="0: the default; 1: lanes take new rays as theirs finish (the default); 2: the 4-wide "
                         "tree; 3: postponed leaves; 4: the plain binary walk; 5: the 8-wide tree with quantised "
                         "boxes")
     p.add_argument("--block", type=int, default=0, choices=[0, 128, 256])
