@@ -88,7 +88,8 @@ cudaError_t copy_part(Lane& l, char* dst, const char* src, size_t bytes, bool to
     return e != cudaSuccess ? e : last;
 }
 
-int copy(void* dst, const void* src, size_t bytes, bool to_host) {
+// st carries the copies that are not split, after its work.
+int copy(void* dst, const void* src, size_t bytes, bool to_host, cudaStream_t st) {
     int device = 0;
     MYPBR_CUDA(cudaGetDevice(&device));
     const int threads = std::min<int>(kThreads, int(std::max(1u, std::thread::hardware_concurrency())));
@@ -125,7 +126,8 @@ int copy(void* dst, const void* src, size_t bytes, bool to_host) {
             return MYPBR_OK;
         }
     }
-    MYPBR_CUDA(cudaMemcpy(dst, src, bytes, to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice));
+    MYPBR_CUDA(cudaMemcpyAsync(dst, src, bytes, to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, st));
+    MYPBR_CUDA(cudaStreamSynchronize(st));
     return MYPBR_OK;
 }
 
@@ -140,16 +142,12 @@ Kept g_kept[kMaxDevices];
 }  // namespace
 
 int copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t st) {
-    if (bytes < kSplitFrom) {
-        MYPBR_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
+    if (bytes >= kSplitFrom)  // the parts are copied on streams of their own
         MYPBR_CUDA(cudaStreamSynchronize(st));
-        return MYPBR_OK;
-    }
-    MYPBR_CUDA(cudaStreamSynchronize(st));
-    return copy(dst, src, bytes, true);
+    return copy(dst, src, bytes, true, st);
 }
 
-int copy_to_device(void* dst, const void* src, size_t bytes) { return copy(dst, src, bytes, false); }
+int copy_to_device(void* dst, const void* src, size_t bytes) { return copy(dst, src, bytes, false, nullptr); }
 
 int Workspace::reserve(size_t bytes) {
     int device = 0;
