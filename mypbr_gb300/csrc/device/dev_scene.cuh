@@ -741,21 +741,34 @@ MYPBR_DEV bool hit_leaf(const DeviceScene& S, int slot, float3 o, float3 d, cons
     return hit_record<VOX>(S, S.leaves + 4 * size_t(slot), o, d, tr, tmin, tmax, media_key, t, b1, b2, ref);
 }
 
-// The nearest of the scene's emitting surfaces along the ray.
-MYPBR_DEV HitInfo nearest_emitter(const DeviceScene& S, float3 o, float3 d, float tmin, uint64_t media_key) {
+// Surfaces at one t (a lamp in the plane of the ceiling, two lamps that
+// overlap): which of them a ray meets is decided by the order in which the
+// walk for the closest hit tests them, and by nothing else. Whoever asks a
+// question that is cheaper than the closest hit takes t's this near to one
+// another (2^-20 of t: kinds of primitives, and kernels, round differently in
+// the last bits) for one t, and leaves the ray to that walk.
+constexpr float kSameT = 9.5367431640625e-7f;
+
+// The nearest of the scene's emitting surfaces along the ray; tied: another
+// of them lies at the same t.
+MYPBR_DEV HitInfo nearest_emitter(const DeviceScene& S, float3 o, float3 d, float tmin, uint64_t media_key, bool& tied) {
     HitInfo h;
     h.prim = kMiss;
     h.t = 3.0e38f;
     h.b1 = h.b2 = 0.0f;
+    tied = false;
     const TriRay tr = make_tri_ray(d);
     for (int k = 0; k < S.emitter_count; k++) {
         float t, b1, b2;
         uint32_t ref;
-        if (hit_record<false>(S, S.emitters + 4 * k, o, d, tr, tmin, h.t, media_key, t, b1, b2, ref)) {
-            h.t = t;
-            h.b1 = b1;
-            h.b2 = b2;
-            h.prim = ref;
+        if (hit_record<false>(S, S.emitters + 4 * k, o, d, tr, tmin, h.t * (1.0f + kSameT), media_key, t, b1, b2, ref)) {
+            tied = t >= h.t * (1.0f - kSameT);
+            if (t < h.t) {
+                h.t = t;
+                h.b1 = b1;
+                h.b2 = b2;
+                h.prim = ref;
+            }
         }
     }
     return h;
@@ -791,20 +804,26 @@ MYPBR_DEV HitInfo closest_hit(const DeviceScene& S, float3 o, float3 d, float tm
 // Whether anything but primitive `skip` lies along o + t d, t in (tmin,
 // tmax): the walk stops at the first primitive it hits. For shadow rays that
 // need no more than whether something dark is in the way, this is all the
-// reference's closest-hit query decides.
+// reference's closest-hit query decides. The walk goes a little past tmax;
+// tied: what it met lies at tmax itself (kSameT), and something nearer may or
+// may not.
+enum : int { kFree = 0, kBlocked = 1, kTied = 2 };
+MYPBR_DEV float past(float t) { return t * (1.0f + 0.5f * kSameT); }
+// What an ANY walk that met something at h.b1 says; h.t is past(tmax).
+MYPBR_DEV int blocked_or_tied(const HitInfo& h) { return h.b1 >= h.t * (1.0f - kSameT) ? kTied : kBlocked; }
 template <bool VOX = true, int WALK = kWalkBinary>
-MYPBR_DEV bool any_hit(const DeviceScene& S, float3 o, float3 d, float tmin, float tmax, uint64_t media_key,
-                       uint32_t skip = kMiss) {
+MYPBR_DEV int any_hit(const DeviceScene& S, float3 o, float3 d, float tmin, float tmax, uint64_t media_key,
+                      uint32_t skip = kMiss) {
     HitInfo h;
     h.prim = skip;
-    h.t = tmax;
+    h.t = past(tmax);
     h.b1 = h.b2 = 0.0f;
-    return walk<true, VOX, WALK>(S, o, d, tmin, media_key, h);
+    return walk<true, VOX, WALK>(S, o, d, tmin, media_key, h) ? blocked_or_tied(h) : kFree;
 }
 
 // The unbounded objects beside the BVH, after the walk: the ground
 // (plane.h:17-34) and height fog (medium.h:352-381). True when ANY and one
-// was met.
+// was met (at h.b1).
 template <bool ANY>
 MYPBR_DEV bool walk_unbounded(const DeviceScene& S, float3 o, float3 d, float tmin, uint64_t media_key, HitInfo& h) {
     for (int k = 0; k < S.unbounded_count; k++) {
@@ -814,8 +833,10 @@ MYPBR_DEV bool walk_unbounded(const DeviceScene& S, float3 o, float3 d, float tm
                 continue;
             float t = (ub.height - o.y) / d.y;
             if (t > tmin && t < h.t) {
-                if (ANY)
+                if (ANY) {
+                    h.b1 = t;
                     return true;
+                }
                 h.t = t;
                 h.prim = (uint32_t(kGround) << kKindShift) | uint32_t(k);
             }
@@ -836,8 +857,10 @@ MYPBR_DEV bool walk_unbounded(const DeviceScene& S, float3 o, float3 d, float tm
                 t = tmin - logf(x) / kk;
             }
             if (t < h.t && isfinite(t)) {
-                if (ANY)
+                if (ANY) {
+                    h.b1 = t;
                     return true;
+                }
                 h.t = t;
                 h.prim = (uint32_t(kHeightFog) << kKindShift) | uint32_t(k);
             }
@@ -847,7 +870,7 @@ MYPBR_DEV bool walk_unbounded(const DeviceScene& S, float3 o, float3 d, float tm
 }
 
 // The primitives of one leaf (count refs from first) against the ray; true
-// when ANY and one other than h.prim was hit.
+// when ANY and one other than h.prim was hit (at h.b1).
 template <bool ANY, bool VOX, class Tri>
 MYPBR_DEV bool test_leaf(const DeviceScene& S, int first, int count, float3 o, float3 d, const Tri& tr, float tmin,
                          uint64_t media_key, HitInfo& h) {
@@ -856,9 +879,10 @@ MYPBR_DEV bool test_leaf(const DeviceScene& S, int first, int count, float3 o, f
         uint32_t ref;
         if (hit_leaf<VOX>(S, first + k, o, d, tr, tmin, h.t, media_key, t, b1, b2, ref)) {
             if (ANY) {
-                if (ref != h.prim)
-                    return true;
-                continue;
+                if (ref == h.prim)
+                    continue;
+                h.b1 = t;
+                return true;
             }
             h.t = t;
             h.b1 = b1;
@@ -1056,23 +1080,25 @@ struct LaneWalk {
     uint64_t media_key;
     HitInfo h;
     int node, leaf, sp, visits;
-    bool found;  // an ANY walk met something
     MYPBR_DEV bool done() const { return node == kWalkDone && leaf == 0; }
     MYPBR_DEV void stop() {
         node = kWalkDone;
         leaf = 0;
     }
+    // An ANY walk has met something: at h.b1, which is below 0 until then.
+    MYPBR_DEV bool met() const { return h.b1 >= 0.0f; }
     // skip: the primitive that an ANY walk ignores (kMiss: none)
+    template <bool ANY>
     MYPBR_DEV void start(const DeviceScene& S, float3 from, float3 dir, float t_min, float t_max, uint64_t key,
                          uint32_t skip = kMiss) {
         o = from;
         d = dir;
         tmin = t_min;
         media_key = key;
-        found = false;
         h.prim = skip;
         h.t = t_max;
-        h.b1 = h.b2 = 0.0f;
+        h.b1 = ANY ? -1.0f : 0.0f;
+        h.b2 = 0.0f;
         inv = f3(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
         oi = -1.0f * (o * inv);
         node = S.has_bvh ? 0 : kWalkDone;
@@ -1116,7 +1142,6 @@ struct LaneWalk {
             } else {
                 if ((h0 && k0 > 0 && test_leaf<ANY, VOX>(S, e0, k0, o, d, LazyTriRay{d}, tmin, media_key, h)) ||
                     (h1 && k1 > 0 && test_leaf<ANY, VOX>(S, e1, k1, o, d, LazyTriRay{d}, tmin, media_key, h))) {
-                    found = true;
                     stop();
                     break;
                 }
@@ -1153,7 +1178,6 @@ struct LaneWalk {
         while (POSTPONED && leaf < 0) {
             const int packed = ~leaf;
             if (test_leaf<ANY, VOX>(S, packed >> 4, packed & 15, o, d, LazyTriRay{d}, tmin, media_key, h)) {
-                found = true;
                 stop();
                 break;
             }

@@ -483,8 +483,8 @@ __global__ void __maxnreg__(lane_registers(VOX, POSTPONED)) k_extend_lanes(WaveP
                 entry = k;
                 if (k < n) {
                     const Pair r = load_pair(rays, k);
-                    W.start(P.S, f3(r.a), f3(r.b), spawn_tmin(f3(r.a), f3(r.b)), 3.0e38f,
-                            extend_key(P, wave, depth, k));
+                    W.start<false>(P.S, f3(r.a), f3(r.b), spawn_tmin(f3(r.a), f3(r.b)), 3.0e38f,
+                                   extend_key(P, wave, depth, k));
                 }
             }
             if (!__any_sync(0xffffffffu, entry < n))
@@ -840,8 +840,9 @@ __global__ void __launch_bounds__(256, 2) k_shade_guided(WaveParams P, int depth
 // surfaces that emit are few, so the nearest of them along the ray is found
 // first, from their list; then only whether something lies before it matters
 // (or, with none, whether the ray escapes), and a ray that would bring no
-// light anyway is not walked at all. kShadowClosest: the closest hit, through
-// clear glass if the options say so.
+// light anyway is not walked at all; where something else lies at the nearest
+// emitter's t, the closest hit decides. kShadowClosest: the closest hit,
+// through clear glass if the options say so.
 // The 2 M-triangle room (16 lamps) at 1080p, 16 spp: shadow 58.5 ms with
 // closest hits, 40.5 with its emitters first and lanes that take new rays.
 enum : int { kShadowAny = 0, kShadowEmitters = 1, kShadowClosest = 2 };
@@ -902,6 +903,41 @@ MYPBR_DEV bool shadow_hop(const WaveParams& P, const HitInfo& h, float3& o, floa
     return false;
 }
 
+// A shadow ray traced by closest hits.
+template <bool VOX, int WALK>
+MYPBR_DEV void shadow_closest(const WaveParams& P, int2 wave, int depth, uint2 entry, const Pair& ray) {
+    float3 o = f3(ray.a);
+    const float3 d = f3(ray.b);
+    float3 through = f3(1.0f), emission = f3(0.0f);
+    for (int hop = 0; hop <= 16; hop++) {
+        const uint64_t key = shadow_key(P, wave, depth, ray.a, hop);
+        const HitInfo h = closest_hit<VOX, WALK>(P.S, o, d, spawn_tmin(o, d), 3.0e38f, key);
+        if (!shadow_hop(P, h, o, d, hop, through, emission))
+            break;
+    }
+    shadow_end(P, wave, depth, entry, through, emission);
+}
+
+// A thread's rays that kShadowEmitters leaves to the closest hit: a list by
+// their places in the shadow queue, linked through the sky word of their
+// records (nonzero only where the sky is the one light). They wait until the
+// thread's other rays are done: a second walk where they are found takes
+// registers from the first (k_shadow_lanes then spills 244 bytes in place of 28).
+constexpr uint32_t kNoTie = 0xffffffffu;
+MYPBR_DEV void put_tie(float4* rays, uint32_t& ties, uint32_t k, uint2 entry) {
+    rays[2 * size_t(entry.x) + 1].w = bits_f(ties);
+    ties = k;
+}
+template <bool VOX, int WALK>
+MYPBR_DEV void settle_ties(const WaveParams& P, int2 wave, int depth, const float4* rays, uint32_t ties) {
+    while (ties != kNoTie) {
+        const uint2 entry = P.B.shadow_queue[ties];
+        const Pair ray = load_pair(rays, entry.x);
+        ties = f_bits(ray.b.w);
+        shadow_closest<VOX, WALK>(P, wave, depth, entry, ray);
+    }
+}
+
 template <bool VOX, int WALK, int MODE>
 __global__ void __launch_bounds__(256, 3) k_shadow(WaveParams P, int depth) {
     depth = bounce_of(P, depth);
@@ -912,43 +948,49 @@ __global__ void __launch_bounds__(256, 3) k_shadow(WaveParams P, int depth) {
         atomicAdd(&P.totals[1], (unsigned long long)n);
     const DeviceScene& S = P.S;
     uint32_t stride = gridDim.x * blockDim.x;
-    const float4* rays = P.B.ray[depth & 1];
+    float4* const rays = P.B.ray[depth & 1];
     const int2 wave = wave_of(P);
+    uint32_t ties = kNoTie;
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += stride) {
         const uint2 entry = P.B.shadow_queue[k];
         const Pair ray = load_pair(rays, entry.x);
-        float3 o = f3(ray.a);
-        const float3 d = f3(ray.b);
-        float3 through = f3(1.0f), emission = f3(0.0f);
         if constexpr (MODE == kShadowClosest) {
-            for (int hop = 0; hop <= 16; hop++) {
-                const uint64_t key = shadow_key(P, wave, depth, ray.a, hop);
-                const HitInfo h = closest_hit<VOX, WALK>(S, o, d, spawn_tmin(o, d), 3.0e38f, key);
-                if (!shadow_hop(P, h, o, d, hop, through, emission))
-                    break;
-            }
+            shadow_closest<VOX, WALK>(P, wave, depth, entry, ray);
         } else {
+            const float3 o = f3(ray.a), d = f3(ray.b);
             const uint64_t key = shadow_key(P, wave, depth, ray.a, 0);
             const float tmin = spawn_tmin(o, d);
+            float3 emission = f3(0.0f);
             HitInfo e;
             e.prim = kMiss;
             e.t = 3.0e38f;
             if constexpr (MODE == kShadowEmitters) {
-                e = nearest_emitter(S, o, d, tmin, key);
+                bool tied;
+                e = nearest_emitter(S, o, d, tmin, key, tied);
                 emission = e.prim == kMiss && S.dark_sky ? f3(0.0f) : unblocked(S, e, o, d, ray.b.w);
-                if (!is_zero(emission) && any_hit<VOX, WALK>(S, o, d, tmin, e.t, key, e.prim))
+                int way = tied ? kTied : kFree;
+                if (!tied && !is_zero(emission))
+                    way = any_hit<VOX, WALK>(S, o, d, tmin, e.t, key, e.prim);
+                if (way == kTied) {
+                    put_tie(rays, ties, k, entry);
+                    continue;
+                }
+                if (way == kBlocked)
                     emission = f3(0.0f);
-            } else if (!any_hit<VOX, WALK>(S, o, d, tmin, e.t, key)) {
+            } else if (any_hit<VOX, WALK>(S, o, d, tmin, e.t, key) == kFree) {
                 emission = unblocked(S, e, o, d, ray.b.w);
             }
+            shadow_end(P, wave, depth, entry, f3(1.0f), emission);
         }
-        shadow_end(P, wave, depth, entry, through, emission);
     }
+    if constexpr (MODE == kShadowEmitters)
+        settle_ties<VOX, WALK>(P, wave, depth, rays, ties);
 }
 
 // k_shadow with lanes that take a new ray as soon as theirs is done (see
-// k_extend_lanes), for the two modes whose rays are one walk each.
-template <bool VOX, int MODE>
+// k_extend_lanes), for the two modes whose rays are one walk each. TIES: the
+// walk of kShadowClosest, for the rays it settles.
+template <bool VOX, int MODE, int TIES>
 __global__ void __maxnreg__(lane_registers(VOX, true)) k_shadow_lanes(WaveParams P, int depth) {
     depth = bounce_of(P, depth);
     if (depth < 0)
@@ -957,7 +999,7 @@ __global__ void __maxnreg__(lane_registers(VOX, true)) k_shadow_lanes(WaveParams
     if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0)
         atomicAdd(&P.totals[1], (unsigned long long)n);
     const DeviceScene& S = P.S;
-    const float4* rays = P.B.ray[depth & 1];
+    float4* const rays = P.B.ray[depth & 1];
     const int2 wave = wave_of(P);
     const uint32_t run = warp_run(n);
     WarpRun take;
@@ -966,16 +1008,21 @@ __global__ void __maxnreg__(lane_registers(VOX, true)) k_shadow_lanes(WaveParams
     uint32_t k = n;
     uint2 entry = make_uint2(0u, 0u);
     float3 emission = f3(0.0f);
+    uint32_t ties = kNoTie;
     W.stop();
     while (true) {
         const bool idle = W.done();
         if (__popc(__ballot_sync(0xffffffffu, idle)) >= kTakeAt) {
             if (idle && k < n) {
-                if (W.found || walk_unbounded<true>(S, W.o, W.d, W.tmin, W.media_key, W.h))
+                const bool met = W.met() || walk_unbounded<true>(S, W.o, W.d, W.tmin, W.media_key, W.h);
+                if (met)
                     emission = f3(0.0f);
                 else if (MODE == kShadowAny)
                     emission = unblocked<true>(S, W.h, W.o, W.d, rays[2 * size_t(entry.x) + 1].w);
-                shadow_end(P, wave, depth, entry, f3(1.0f), emission);
+                if (MODE == kShadowEmitters && met && blocked_or_tied(W.h) == kTied)
+                    put_tie(rays, ties, k, entry);
+                else
+                    shadow_end(P, wave, depth, entry, f3(1.0f), emission);
             }
             const uint32_t next = take.take(sh_fetch_counter(P, depth), n, run, idle);
             if (idle) {
@@ -990,13 +1037,14 @@ __global__ void __maxnreg__(lane_registers(VOX, true)) k_shadow_lanes(WaveParams
                     HitInfo e;
                     e.prim = kMiss;
                     e.t = 3.0e38f;
+                    bool tied = false;
                     if constexpr (MODE == kShadowEmitters) {
-                        e = nearest_emitter(S, o, d, tmin, key);
+                        e = nearest_emitter(S, o, d, tmin, key, tied);
                         emission = e.prim == kMiss && S.dark_sky ? f3(0.0f) : unblocked<true>(S, e, o, d, ray.b.w);
                     }
-                    W.start(S, o, d, tmin, e.t, key, e.prim);
-                    if (MODE == kShadowEmitters && is_zero(emission)) {
-                        W.found = true;  // nothing to bring: not walked
+                    W.start<true>(S, o, d, tmin, past(e.t), key, e.prim);
+                    if (MODE == kShadowEmitters && (tied || is_zero(emission))) {
+                        W.h.b1 = tied ? W.h.t : 0.0f;  // nothing to bring, or to be settled: not walked
                         W.stop();
                     }
                 }
@@ -1006,6 +1054,20 @@ __global__ void __maxnreg__(lane_registers(VOX, true)) k_shadow_lanes(WaveParams
         }
         W.advance<true, VOX, true>(S, stack, take.least());
     }
+    if constexpr (MODE == kShadowEmitters)
+        while (ties != kNoTie) {  // the same lane walk, for the closest hit
+            entry = P.B.shadow_queue[ties];
+            const Pair ray = load_pair(rays, entry.x);
+            ties = f_bits(ray.b.w);
+            float3 o = f3(ray.a), through = f3(1.0f);
+            W.start<false>(S, o, f3(ray.b), spawn_tmin(o, f3(ray.b)), 3.0e38f, shadow_key(P, wave, depth, ray.a, 0));
+            while (!W.done())
+                W.advance<false, VOX, TIES == kWalkPostponed>(S, stack, 0);
+            walk_unbounded<false>(S, W.o, W.d, W.tmin, W.media_key, W.h);
+            emission = f3(0.0f);
+            shadow_hop(P, W.h, o, W.d, 0, through, emission);
+            shadow_end(P, wave, depth, entry, f3(1.0f), emission);
+        }
 }
 
 // A finite FP32 value in FP64, by its bits: the FP64 pipe, which converts two
@@ -1373,9 +1435,15 @@ const void* extend_kernel(bool vox, int walk) {
 }
 template <bool VOX, int MODE>
 const void* shadow_kernel_of(int walk) {
-    if constexpr (MODE != kShadowClosest)
+    if constexpr (MODE == kShadowAny) {
+        if (walk == kWalkLanes || walk == kWalkLanesPostponed)
+            return (const void*)k_shadow_lanes<VOX, MODE, kWalkBinary>;
+    } else if constexpr (MODE == kShadowEmitters) {
+        if (walk == kWalkLanes)
+            return (const void*)k_shadow_lanes<VOX, MODE, kWalkBinary>;
         if (walk == kWalkLanesPostponed)
-            return (const void*)k_shadow_lanes<VOX, MODE>;
+            return (const void*)k_shadow_lanes<VOX, MODE, kWalkPostponed>;
+    }
     return walk == kWalkWide8       ? (const void*)k_shadow<VOX, kWalkWide8, MODE>
            : walk == kWalkWide      ? (const void*)k_shadow<VOX, kWalkWide, MODE>
            : walk == kWalkPostponed ? (const void*)k_shadow<VOX, kWalkPostponed, MODE>
@@ -1471,11 +1539,11 @@ Launch launch_config(const mypbr_gpu_scene& G, const mypbr_render_opts& o, size_
     L.shadow_mode = shadow_mode(G.dev, o.transparent_shadows);
     // whether anything is in the way does not depend on the order of the
     // tests, so those rays postpone their leaves on sphere scenes too (sphere
-    // field: shadow 12.3 ms against 14.0); hits at the same t do
-    L.shadow_walk = !lanes                             ? L.walk
-                    : L.shadow_mode != kShadowClosest  ? kWalkLanesPostponed
-                    : G.prefer_postponed               ? kWalkPostponed
-                                                       : kWalkBinary;
+    // field: shadow 12.3 ms against 14.0); hits at the same t do, and are
+    // settled by the walk that L.walk stands for
+    L.shadow_walk = !lanes || L.shadow_mode != kShadowClosest ? L.walk
+                    : G.prefer_postponed                      ? kWalkPostponed
+                                                              : kWalkBinary;
     const void* extend = extend_kernel(vox, L.walk);
     const void* shadow = shadow_kernel(vox, L.shadow_walk, L.shadow_mode);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, extend, L.block, 0);
