@@ -8,6 +8,7 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include "../../../include/mypbr_gpu.h"
+#include "cuda_check.h"
 #include "guide.cuh"
 
 namespace mypbr_dev {
@@ -119,7 +120,6 @@ struct NvtxRange {
 };
 
 void set_error_message(const std::string& m);
-int cuda_fail(cudaError_t e, const char* what);
 int release_buffers(RenderBuffers& rb);
 int check_device_error(mypbr_gpu_scene* G);
 int release_guide(GuideState& g);
@@ -148,10 +148,3 @@ int build_env_distribution(const float* rgb, int w, int h, float* texel_pdf, flo
 void env_distribution_host(const float* rgb, int w, int h, float* texel_pdf, float2* alias);
 
 }  // namespace mypbr_dev
-
-#define MYPBR_CUDA(call)                                       \
-    do {                                                       \
-        cudaError_t e_ = (call);                               \
-        if (e_ != cudaSuccess)                                 \
-            return ::mypbr_dev::cuda_fail(e_, #call);          \
-    } while (0)

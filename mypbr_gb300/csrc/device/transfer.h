@@ -8,8 +8,9 @@
 
 namespace mypbr_dev {
 
-// Copies that are done when they return; a copy to the host waits for the
-// work on st first. Large ones are split over host threads.
+// Copies that are done when they return, each ordered as one transfer on its
+// stream (to the device: the legacy stream). The pages of a new frame are made
+// before it is written.
 int copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t st);
 int copy_to_device(void* dst, const void* src, size_t bytes);
 

@@ -1,0 +1,119 @@
+// The frame copies (csrc/device/transfer.cu) against a CUDA runtime made of
+// host memory, for what no GPU is needed to see: which calls they make, in
+// which order, and what they do when one fails. One scenario per run, named
+// on the command line; exit code 0 when it holds.
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <string>
+#include <vector>
+
+#include "../mypbr_gb300/csrc/device/transfer.cu"
+
+namespace {
+
+struct Fake {
+    int copies = 0;
+    bool pages_made = false;     // when the transfer started
+    const char* host = nullptr;  // the caller's memory and what the driver calls it
+    cudaMemoryType kind = cudaMemoryTypeUnregistered;
+} fake;
+
+}  // namespace
+
+extern "C" {
+cudaError_t cudaGetDevice(int* d) { return *d = 0, cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaMalloc(void** p, size_t n) { return *p = std::malloc(n), cudaSuccess; }
+cudaError_t cudaFree(void* p) { return std::free(p), cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
+    a->type = p == fake.host ? fake.kind : cudaMemoryTypeUnregistered;
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
+    fake.copies++;
+    if ((d == fake.host || s == fake.host) && fake.kind == cudaMemoryTypeDevice)
+        return cudaErrorInvalidValue;
+    fake.pages_made = mypbr_dev::missing_pages(static_cast<char*>(d), n, size_t(sysconf(_SC_PAGESIZE)), false) == 0;
+    std::memcpy(d, s, n);
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind k) { return cudaMemcpyAsync(d, s, n, k, nullptr); }
+}
+
+int mypbr_dev::cuda_fail(cudaError_t, const char*) { return MYPBR_ERR_CUDA; }
+
+namespace {
+
+#define HOLDS(x)                                              \
+    do {                                                      \
+        if (!(x)) {                                           \
+            std::fprintf(stderr, "does not hold: %s\n", #x);  \
+            std::exit(1);                                     \
+        }                                                     \
+    } while (0)
+
+constexpr size_t kBytes = (size_t(20) << 20) + 24;
+
+std::vector<char> pattern() {
+    std::vector<char> v(kBytes);
+    for (size_t k = 0; k < kBytes; k++)
+        v[k] = char(k * 7 + k / 4096);
+    return v;
+}
+
+// Each way one transfer, whatever kind of host memory it is.
+void one_transfer(cudaMemoryType kind) {
+    std::vector<char> a = pattern(), dev(kBytes), back(kBytes);
+    fake.kind = kind;
+    fake.host = a.data();
+    HOLDS(mypbr_dev::copy_to_device(dev.data(), a.data(), kBytes) == MYPBR_OK && fake.copies == 1);
+    fake.host = back.data();
+    HOLDS(mypbr_dev::copy_to_host(back.data(), dev.data(), kBytes, nullptr) == MYPBR_OK && fake.copies == 2);
+    HOLDS(back == a);
+}
+
+// A new frame's pages exist when its transfer starts, and nothing around it is written; pages that exist keep their contents.
+void pages_are_made(size_t bytes, size_t offset) {
+    const size_t page = size_t(sysconf(_SC_PAGESIZE)), size = (offset + bytes + 2 * page) / page * page;
+    char* const map = static_cast<char*>(mmap(nullptr, size, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0));
+    HOLDS(map != MAP_FAILED);
+    std::vector<char> a(bytes, 3);
+    HOLDS(mypbr_dev::copy_to_host(map + offset, a.data(), bytes, nullptr) == MYPBR_OK);
+    HOLDS(fake.pages_made && std::memcmp(map + offset, a.data(), bytes) == 0);
+    mypbr_dev::make_pages(map + offset, bytes);
+    HOLDS(std::memcmp(map + offset, a.data(), bytes) == 0);
+    unsigned char there = 0;  // the page after the frame's last one
+    HOLDS(mincore(map + (offset + bytes + page - 1) / page * page, page, &there) == 0 && !(there & 1));
+    munmap(map, size);
+}
+
+// A device pointer where host memory is asked for: nothing here may touch it.
+void device_pointers_are_refused() {
+    std::vector<char> dev(kBytes);
+    char* const bad = reinterpret_cast<char*>(0x1000);
+    fake.kind = cudaMemoryTypeDevice;
+    fake.host = bad;
+    HOLDS(mypbr_dev::copy_to_device(dev.data(), bad, kBytes) == MYPBR_ERR_CUDA);
+    HOLDS(mypbr_dev::copy_to_host(bad, dev.data(), kBytes, nullptr) == MYPBR_ERR_CUDA);
+}
+
+}  // namespace
+
+int main(int argc, char** argv) {
+    const std::string name = argc > 1 ? argv[1] : "";
+    if (name == "pageable")
+        one_transfer(cudaMemoryTypeUnregistered);
+    else if (name == "pinned")
+        one_transfer(cudaMemoryTypeHost);
+    else if (name == "managed")
+        one_transfer(cudaMemoryTypeManaged);
+    else if (name == "device")
+        device_pointers_are_refused();
+    else if (name == "new_frame")  // <bytes> <offset in the mapping>
+        pages_are_made(std::strtoull(argv[2], nullptr, 10), std::strtoull(argv[3], nullptr, 10));
+    else
+        return 2;
+    return 0;
+}
