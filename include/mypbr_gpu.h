@@ -721,6 +721,11 @@ int mypbr_write_image(const char* path, const double* radiance, int32_t width, i
  * usable. For tests. */
 int mypbr_gpu_test_wait_timeout(void);
 
+/* Writes the handle's device error word, as a kernel's own check would (1 and
+ * 2: a BVH walk past its bounds; 3: a wait past its limit): the next call on
+ * the handle reports it. For tests. */
+int mypbr_gpu_test_device_error(mypbr_gpu_scene* scene, int32_t code);
+
 /* ----------------------------------------------------- path guiding
  *
  * No counterpart in the reference: a learned sampling proposal, used by

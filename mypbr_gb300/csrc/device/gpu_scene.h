@@ -121,7 +121,8 @@ struct NvtxRange {
 
 void set_error_message(const std::string& m);
 int release_buffers(RenderBuffers& rb);
-int check_device_error(mypbr_gpu_scene* G);
+// Waits for the work on st and reads (and clears) the device's error word.
+int check_device_error(mypbr_gpu_scene* G, cudaStream_t st = nullptr);
 int release_guide(GuideState& g);
 void release_batch_graph(mypbr_gpu_scene* G);
 // Creates the network (seeded initial weights) if the scene has none of this size.

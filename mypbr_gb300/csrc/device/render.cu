@@ -2117,9 +2117,7 @@ extern "C" int mypbr_gpu_render_device(mypbr_gpu_scene* G, const mypbr_camera* c
     // the next one on any stream), unless the caller is capturing it
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     MYPBR_CUDA(cudaStreamIsCapturing(st, &capturing));
-    if (capturing == cudaStreamCaptureStatusNone)
-        MYPBR_CUDA(cudaStreamSynchronize(st));
-    return MYPBR_OK;
+    return capturing == cudaStreamCaptureStatusNone ? check_device_error(G, st) : MYPBR_OK;
 }
 
 namespace {

@@ -1078,9 +1078,10 @@ extern "C" int mypbr_gpu_scene_create(const mypbr_flat_scene* scene, mypbr_gpu_s
 
 namespace mypbr_dev {
 // Reads and clears the sticky device error word after a synchronised call.
-int check_device_error(mypbr_gpu_scene* G) {
+int check_device_error(mypbr_gpu_scene* G, cudaStream_t st) {
     int e = 0;
-    MYPBR_CUDA(cudaMemcpy(&e, G->dev.error, sizeof e, cudaMemcpyDeviceToHost));
+    MYPBR_CUDA(cudaMemcpyAsync(&e, G->dev.error, sizeof e, cudaMemcpyDeviceToHost, st));
+    MYPBR_CUDA(cudaStreamSynchronize(st));
     if (e == 0)
         return MYPBR_OK;
     int zero = 0;
@@ -1094,6 +1095,15 @@ int check_device_error(mypbr_gpu_scene* G) {
     return MYPBR_ERR_DEVICE_CHECK;
 }
 }  // namespace mypbr_dev
+
+extern "C" int mypbr_gpu_test_device_error(mypbr_gpu_scene* scene, int32_t code) {
+    if (!scene || code < 1 || code > 3) {
+        mypbr_dev::set_error_message("mypbr_gpu_test_device_error: null scene, or a code that is none of the device's");
+        return MYPBR_ERR_INVALID_ARGUMENT;
+    }
+    MYPBR_CUDA(cudaMemcpy(scene->dev.error, &code, sizeof code, cudaMemcpyHostToDevice));
+    return MYPBR_OK;
+}
 
 extern "C" void mypbr_gpu_scene_destroy(mypbr_gpu_scene* scene) {
     if (!scene)
