@@ -458,9 +458,11 @@ int mypbr_gpu_render(mypbr_gpu_scene* scene, const mypbr_camera* cam, const mypb
                      int save_every, mypbr_pass_callback on_pass, void* user);
 
 /* The same, with outputs left in device memory (each a device pointer of the
- * sizes above, NULL allowed as for mypbr_gpu_render) and work issued on the
- * given CUDA stream (NULL = the legacy default stream). Returns once the
- * work is queued; stats (optional) are filled after a stream sync. */
+ * sizes above, NULL allowed as for mypbr_gpu_render). The work is issued on
+ * the given CUDA stream; with NULL or cudaStreamLegacy on the handle's own
+ * stream, once what the legacy stream and every blocking stream held is done.
+ * Returns when the render is done, or, on a stream that is being captured,
+ * when it is recorded. stats is optional (not while capturing). */
 typedef struct mypbr_render_stats {
     uint64_t paths;            /* camera rays traced */
     uint64_t extension_rays;   /* closest-hit rays traced for path continuation */
