@@ -282,7 +282,7 @@ struct DevArr {
             cudaFree(p);
     }
     int alloc(size_t n) {
-        MYPBR_CUDA(cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)));
+        MYPBR_CUDA(device_malloc(&p, std::max<size_t>(n, 1) * sizeof(T)));
         return MYPBR_OK;
     }
 };
@@ -388,7 +388,7 @@ extern "C" int mypbr_gpu_scene_rebuild_bvh(mypbr_gpu_scene* G, int32_t method, m
     collapse_to_4(after, wide, depth4);
     float4* wide_p = nullptr;
     if (3 * (depth4 + 1) <= kBvh4Stack) {
-        MYPBR_CUDA(cudaMalloc(&wide_p, wide.size() * sizeof(float4)));
+        MYPBR_CUDA(device_malloc(&wide_p, wide.size() * sizeof(float4)));
         MYPBR_CUDA(cudaMemcpy(wide_p, wide.data(), wide.size() * sizeof(float4), cudaMemcpyHostToDevice));
         G->allocations.push_back(wide_p);
     }
@@ -397,7 +397,7 @@ extern "C" int mypbr_gpu_scene_rebuild_bvh(mypbr_gpu_scene* G, int32_t method, m
     int depth8 = 0;
     uint4* wide8_p = nullptr;
     if (collapse_to_8q(after, wide8, depth8) && 7 * (depth8 + 1) <= kBvh8Stack) {
-        MYPBR_CUDA(cudaMalloc(&wide8_p, wide8.size() * sizeof(uint4)));
+        MYPBR_CUDA(device_malloc(&wide8_p, wide8.size() * sizeof(uint4)));
         MYPBR_CUDA(cudaMemcpy(wide8_p, wide8.data(), wide8.size() * sizeof(uint4), cudaMemcpyHostToDevice));
         G->allocations.push_back(wide8_p);
     }

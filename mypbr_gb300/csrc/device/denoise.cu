@@ -15,7 +15,6 @@
 
 #include "dev_math.cuh"
 #include "gpu_scene.h"
-#include "transfer.h"
 
 namespace mypbr_dev {
 namespace {

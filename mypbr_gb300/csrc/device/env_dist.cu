@@ -33,7 +33,7 @@ struct Scratch {
         if (p)
             cudaFree(p);
     }
-    cudaError_t alloc(size_t n) { return cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)); }
+    cudaError_t alloc(size_t n) { return device_malloc(&p, std::max<size_t>(n, 1) * sizeof(T)); }
 };
 
 constexpr double kPiD = 3.1415926535897932385;

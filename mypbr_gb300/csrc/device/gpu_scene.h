@@ -10,6 +10,7 @@
 #include "../../../include/mypbr_gpu.h"
 #include "cuda_check.h"
 #include "guide.cuh"
+#include "transfer.h"
 
 namespace mypbr_dev {
 

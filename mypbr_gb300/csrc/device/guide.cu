@@ -514,7 +514,7 @@ std::vector<float> initial_weights(int hidden, unsigned long long seed) {
 
 template <typename T>
 int dalloc(T*& p, size_t n) {
-    MYPBR_CUDA(cudaMalloc(&p, n * sizeof(T)));
+    MYPBR_CUDA(device_malloc(&p, n * sizeof(T)));
     return MYPBR_OK;
 }
 
@@ -628,7 +628,7 @@ int guide_fit_box(mypbr_gpu_scene* G, cudaStream_t st) {
         return MYPBR_OK;
     g.box_fitted = true;
     uint32_t* hist = nullptr;
-    MYPBR_CUDA(cudaMalloc(&hist, 3 * kBoxBins * sizeof(uint32_t)));
+    MYPBR_CUDA(device_malloc(&hist, 3 * kBoxBins * sizeof(uint32_t)));
     std::vector<uint32_t> h(3 * kBoxBins);
     int rc = MYPBR_OK;
     if (cudaMemsetAsync(hist, 0, 3 * kBoxBins * sizeof(uint32_t), st) != cudaSuccess)
@@ -1037,7 +1037,7 @@ extern "C" int mypbr_gpu_test_wait_timeout(void) {
         return MYPBR_ERR_NO_DEVICE;
     }
     int* err = nullptr;
-    MYPBR_CUDA(cudaMalloc(&err, sizeof(int)));
+    MYPBR_CUDA(device_malloc(&err, sizeof(int)));
     int rc = MYPBR_OK;
     if (cudaMemset(err, 0, sizeof(int)) != cudaSuccess)
         rc = cuda_fail(cudaGetLastError(), "mypbr_gpu_test_wait_timeout");

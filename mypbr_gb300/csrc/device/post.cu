@@ -21,7 +21,6 @@
 #include <vector>
 
 #include "gpu_scene.h"
-#include "transfer.h"
 
 namespace mypbr_dev {
 

@@ -175,9 +175,9 @@ extern "C" int mypbr_gpu_trace(mypbr_gpu_scene* G, const float* rays, int64_t n,
         return check_device_error(G);
     }
     Buf dr, dh, dp;
-    MYPBR_CUDA(cudaMalloc(&dr.p, size_t(n) * 8 * sizeof(float)));
-    MYPBR_CUDA(cudaMalloc(&dh.p, size_t(n) * 8 * sizeof(float)));
-    MYPBR_CUDA(cudaMalloc(&dp.p, size_t(n) * 2 * sizeof(int)));
+    MYPBR_CUDA(device_malloc(&dr.p, size_t(n) * 8 * sizeof(float)));
+    MYPBR_CUDA(device_malloc(&dh.p, size_t(n) * 8 * sizeof(float)));
+    MYPBR_CUDA(device_malloc(&dp.p, size_t(n) * 2 * sizeof(int)));
     MYPBR_CUDA(cudaMemcpy(dr.p, rays, size_t(n) * 8 * sizeof(float), cudaMemcpyHostToDevice));
     k_trace_walk<<<blocks, 128>>>(G->dev, static_cast<float*>(dr.p), (long long)n, static_cast<float*>(dh.p),
                                   static_cast<int*>(dp.p));
@@ -197,10 +197,10 @@ extern "C" int mypbr_gpu_bsdf_eval(mypbr_gpu_scene* G, int32_t material, const f
         return MYPBR_OK;
     MYPBR_CUDA(cudaSetDevice(G->device));
     Buf a, b, c, d;
-    MYPBR_CUDA(cudaMalloc(&a.p, size_t(n) * 16 * sizeof(float)));
-    MYPBR_CUDA(cudaMalloc(&b.p, size_t(n) * 3 * sizeof(float)));
-    MYPBR_CUDA(cudaMalloc(&c.p, size_t(n) * 3 * sizeof(float)));
-    MYPBR_CUDA(cudaMalloc(&d.p, size_t(n) * 4 * sizeof(float)));
+    MYPBR_CUDA(device_malloc(&a.p, size_t(n) * 16 * sizeof(float)));
+    MYPBR_CUDA(device_malloc(&b.p, size_t(n) * 3 * sizeof(float)));
+    MYPBR_CUDA(device_malloc(&c.p, size_t(n) * 3 * sizeof(float)));
+    MYPBR_CUDA(device_malloc(&d.p, size_t(n) * 4 * sizeof(float)));
     MYPBR_CUDA(cudaMemcpy(a.p, rec, size_t(n) * 16 * sizeof(float), cudaMemcpyHostToDevice));
     MYPBR_CUDA(cudaMemcpy(b.p, r_in, size_t(n) * 3 * sizeof(float), cudaMemcpyHostToDevice));
     MYPBR_CUDA(cudaMemcpy(c.p, wi, size_t(n) * 3 * sizeof(float), cudaMemcpyHostToDevice));
@@ -219,8 +219,8 @@ extern "C" int mypbr_gpu_test_spawn(mypbr_gpu_scene* G, const float* rays, int64
         return MYPBR_OK;
     MYPBR_CUDA(cudaSetDevice(G->device));
     Buf dr, dout;
-    MYPBR_CUDA(cudaMalloc(&dr.p, size_t(n) * 8 * sizeof(float)));
-    MYPBR_CUDA(cudaMalloc(&dout.p, size_t(n) * 8 * sizeof(int)));
+    MYPBR_CUDA(device_malloc(&dr.p, size_t(n) * 8 * sizeof(float)));
+    MYPBR_CUDA(device_malloc(&dout.p, size_t(n) * 8 * sizeof(int)));
     MYPBR_CUDA(cudaMemcpy(dr.p, rays, size_t(n) * 8 * sizeof(float), cudaMemcpyHostToDevice));
     int blocks = int(std::min<int64_t>((n + 127) / 128, int64_t(G->sm_count) * 16));
     k_spawn_probe<<<blocks, 128>>>(G->dev, static_cast<float*>(dr.p), (long long)n, static_cast<int*>(dout.p));

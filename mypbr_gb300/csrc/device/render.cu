@@ -30,7 +30,6 @@
 #include "../host/host_math.h"
 #include "dev_shading.cuh"
 #include "gpu_scene.h"
-#include "transfer.h"
 
 namespace mypbr_dev {
 
@@ -1309,12 +1308,7 @@ namespace {
 
 template <typename T>
 int alloc(T*& p, size_t count) {
-    const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
-    if (cudaMalloc(reinterpret_cast<void**>(&p), bytes) == cudaSuccess)
-        return MYPBR_OK;
-    cudaGetLastError();
-    release_workspaces();  // what calls without a handle keep between them
-    MYPBR_CUDA(cudaMalloc(reinterpret_cast<void**>(&p), bytes));
+    MYPBR_CUDA(device_malloc(&p, std::max<size_t>(count, 1) * sizeof(T)));
     return MYPBR_OK;
 }
 
@@ -2005,7 +1999,7 @@ int render_wave(mypbr_gpu_scene* G, RenderSetup& R, int wave, int pass0, int sav
 // The handle's ray totals, cleared on st.
 int clear_totals(mypbr_gpu_scene* G, WaveParams& P, cudaStream_t st) {
     if (!G->totals)
-        MYPBR_CUDA(cudaMalloc(&G->totals, 3 * sizeof(unsigned long long)));
+        MYPBR_CUDA(device_malloc(&G->totals, 3 * sizeof(unsigned long long)));
     MYPBR_CUDA(cudaMemsetAsync(G->totals, 0, 3 * sizeof(unsigned long long), st));
     P.totals = G->totals;
     return MYPBR_OK;
@@ -2152,7 +2146,7 @@ extern "C" int mypbr_gpu_render_ex(mypbr_gpu_scene* G, const mypbr_camera* cam, 
         cudaFree(G->frame);
         G->frame = nullptr;
         G->frame_doubles = 0;
-        MYPBR_CUDA(cudaMalloc(&G->frame, need * sizeof(double)));
+        MYPBR_CUDA(device_malloc(&G->frame, need * sizeof(double)));
         G->frame_doubles = need;
     }
     double* const rad = G->frame;
@@ -2357,7 +2351,7 @@ int batch_one_graph(mypbr_batch_job* jobs, int n, const std::vector<mypbr_gpu_sc
         release_batch_graph(owner);
         std::unique_ptr<BatchGraphCache> c(new BatchGraphCache());
         c->key = std::move(key);
-        MYPBR_CUDA(cudaMalloc(&c->totals, 3 * count * sizeof(unsigned long long)));
+        MYPBR_CUDA(device_malloc(&c->totals, 3 * count * sizeof(unsigned long long)));
         for (int i = 0; i < n; i++)
             R[size_t(i)].P.totals = c->totals + 3 * size_t(i);
         struct Owned {
@@ -2522,7 +2516,7 @@ extern "C" int mypbr_gpu_autotune(mypbr_gpu_scene* G, const mypbr_camera* cam, c
     o.samples_per_pixel = int(std::max<size_t>(1, std::min<size_t>(size_t(opts->samples_per_pixel),
                                                                        (size_t(256) << 20) / std::max<size_t>(npix, 1))));
     DevBuf rad;
-    MYPBR_CUDA(cudaMalloc(&rad.p, 3 * npix * sizeof(double)));
+    MYPBR_CUDA(device_malloc(&rad.p, 3 * npix * sizeof(double)));
     const int blocks[2] = {128, 256};
     const size_t waves[4] = {size_t(16) << 20, size_t(32) << 20, size_t(64) << 20, size_t(128) << 20};
     mypbr_tune_result res{};

@@ -76,7 +76,7 @@ struct Uploader {
         if (v.empty())
             return MYPBR_OK;
         void* p = nullptr;
-        MYPBR_CUDA(cudaMalloc(&p, v.size() * sizeof(T)));
+        MYPBR_CUDA(device_malloc(&p, v.size() * sizeof(T)));
         G.allocations.push_back(p);
         MYPBR_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
         out = static_cast<const T*>(p);
@@ -728,9 +728,9 @@ int create_scene(const mypbr_flat_scene* Fp, mypbr_gpu_scene** out) {
         float* rgb = nullptr;
         float* texel_pdf = nullptr;
         float2* alias = nullptr;
-        if (cudaMalloc(&rgb, n * 3 * sizeof(float)) != cudaSuccess ||
-            cudaMalloc(&texel_pdf, n * sizeof(float)) != cudaSuccess ||
-            cudaMalloc(&alias, n * sizeof(float2)) != cudaSuccess) {
+        if (device_malloc(&rgb, n * 3 * sizeof(float)) != cudaSuccess ||
+            device_malloc(&texel_pdf, n * sizeof(float)) != cudaSuccess ||
+            device_malloc(&alias, n * sizeof(float2)) != cudaSuccess) {
             cudaFree(rgb);
             cudaFree(texel_pdf);
             cudaFree(alias);

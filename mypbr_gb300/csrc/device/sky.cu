@@ -57,7 +57,7 @@ int mypbr_sky_bake(const mypbr_sky_settings* settings, const double sun_directio
     size_t n = size_t(width) * height;
     if (on_gpu) {
         double* d = nullptr;
-        MYPBR_CUDA(cudaMalloc(&d, 3 * n * sizeof(double)));
+        MYPBR_CUDA(device_malloc(&d, 3 * n * sizeof(double)));
         k_bake_sky<<<int((n + 127) / 128), 128>>>(st, make_double3(sun_direction[0], sun_direction[1], sun_direction[2]),
                                                   make_double3(sun_irradiance[0], sun_irradiance[1], sun_irradiance[2]),
                                                   width, height, d);

@@ -128,7 +128,7 @@ int Workspace::reserve(size_t bytes) {
         base_ = k.p;
         return MYPBR_OK;
     }
-    MYPBR_CUDA(cudaMalloc(reinterpret_cast<void**>(&base_), std::max<size_t>(bytes, 1)));
+    MYPBR_CUDA(device_malloc(&base_, std::max<size_t>(bytes, 1)));
     return MYPBR_OK;
 }
 
@@ -137,6 +137,16 @@ Workspace::~Workspace() {
         g_kept[kept_].busy.unlock();
     else if (base_)
         cudaFree(base_);
+}
+
+cudaError_t device_malloc_bytes(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        release_workspaces();
+        e = cudaMalloc(p, bytes);
+        cudaGetLastError();  // or the next check of a launch would report it
+    }
+    return e;
 }
 
 void release_workspaces() {

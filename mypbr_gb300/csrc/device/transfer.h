@@ -46,4 +46,12 @@ class Workspace {
 // Gives the current device's kept workspace back, if no call uses it.
 void release_workspaces();
 
+// cudaMalloc for everything but that workspace: where memory has run out the
+// workspace is given back and the allocation tried again.
+cudaError_t device_malloc_bytes(void** p, size_t bytes);
+template <typename T>
+cudaError_t device_malloc(T** p, size_t bytes) {
+    return device_malloc_bytes(reinterpret_cast<void**>(p), bytes);
+}
+
 }  // namespace mypbr_dev

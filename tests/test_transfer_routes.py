@@ -1,6 +1,8 @@
 """Which way frames go between host memory and the GPU, and what the copies do when a call fails: transfer.cu compiled
 against a CUDA runtime made of host memory (transfer_fakes.cpp), on the CPU."""
+import glob
 import os
+import re
 import subprocess
 
 import pytest
@@ -33,3 +35,16 @@ def test_a_frame_is_one_transfer(program, kind):
 @pytest.mark.parametrize("nbytes,offset", [(65536, 0), (65537, 8), (4 << 20, 70001), (20 << 20, 0), ((20 << 20) + 12345, 70001)])
 def test_the_pages_of_a_new_frame_are_made_first(program, nbytes, offset):
     holds(program, "new_frame", nbytes, offset)
+
+
+@pytest.mark.parametrize("scenario", ["out_of_memory", "large"])
+def test_kept_memory_makes_room(program, scenario):
+    holds(program, scenario)
+
+
+def test_every_allocation_can_have_the_kept_memory():
+    """cudaMalloc is called in transfer.cu alone; the other sources go through device_malloc, which gives kept memory back."""
+    for path in glob.glob(os.path.join(ROOT, "mypbr_gb300", "csrc", "**", "*.c*"), recursive=True):
+        if os.path.basename(path) != "transfer.cu":
+            with open(path) as f:
+                assert not re.search(r"\bcudaMalloc(Async|Managed)?\s*\(", f.read()), path

@@ -5,6 +5,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <string>
 #include <vector>
 
@@ -13,6 +14,8 @@
 namespace {
 
 struct Fake {
+    size_t left = SIZE_MAX;      // device memory, bytes
+    std::map<void*, size_t> held;
     int copies = 0;
     bool pages_made = false;     // when the transfer started
     const char* host = nullptr;  // the caller's memory and what the driver calls it
@@ -24,8 +27,19 @@ struct Fake {
 extern "C" {
 cudaError_t cudaGetDevice(int* d) { return *d = 0, cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
-cudaError_t cudaMalloc(void** p, size_t n) { return *p = std::malloc(n), cudaSuccess; }
-cudaError_t cudaFree(void* p) { return std::free(p), cudaSuccess; }
+cudaError_t cudaMalloc(void** p, size_t n) {
+    if (n > fake.left)
+        return cudaErrorMemoryAllocation;
+    fake.left -= n;
+    *p = std::malloc(n);
+    fake.held[*p] = n;
+    return cudaSuccess;
+}
+cudaError_t cudaFree(void* p) {
+    fake.left += fake.held[p];
+    fake.held.erase(p);
+    return std::free(p), cudaSuccess;
+}
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
     a->type = p == fake.host ? fake.kind : cudaMemoryTypeUnregistered;
@@ -42,7 +56,9 @@ cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cu
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind k) { return cudaMemcpyAsync(d, s, n, k, nullptr); }
 }
 
-int mypbr_dev::cuda_fail(cudaError_t, const char*) { return MYPBR_ERR_CUDA; }
+int mypbr_dev::cuda_fail(cudaError_t e, const char*) {
+    return e == cudaErrorMemoryAllocation ? MYPBR_ERR_OUT_OF_MEMORY : MYPBR_ERR_CUDA;
+}
 
 namespace {
 
@@ -99,6 +115,39 @@ void device_pointers_are_refused() {
     HOLDS(mypbr_dev::copy_to_host(bad, dev.data(), kBytes, nullptr) == MYPBR_ERR_CUDA);
 }
 
+// Memory that the kept workspace holds between calls is there for any allocation, and stays while a call uses it.
+void kept_memory_is_given_back() {
+    constexpr size_t MiB = size_t(1) << 20;
+    fake.left = 4 * MiB;
+    void* p = nullptr;
+    {
+        mypbr_dev::Workspace w;
+        HOLDS(w.reserve(3 * MiB) == MYPBR_OK);
+        HOLDS(mypbr_dev::device_malloc(&p, 2 * MiB) == cudaErrorMemoryAllocation && fake.left == 1 * MiB);
+        mypbr_dev::Workspace other;  // as a second thread's call: memory of its own
+        HOLDS(other.reserve(2 * MiB) == MYPBR_ERR_OUT_OF_MEMORY);
+        HOLDS(other.reserve(1 * MiB) == MYPBR_OK);
+    }
+    HOLDS(fake.left == 1 * MiB);
+    HOLDS(mypbr_dev::device_malloc(&p, 2 * MiB) == cudaSuccess && fake.left == 2 * MiB);
+    HOLDS(mypbr_dev::device_malloc(&p, 3 * MiB) == cudaErrorMemoryAllocation);
+}
+
+// More than is ever kept: the kept workspace makes room for it, and it is given back at once.
+void large_workspaces_are_not_kept() {
+    constexpr size_t GiB = size_t(1) << 30;
+    fake.left = 2 * GiB;
+    {
+        mypbr_dev::Workspace w;
+        HOLDS(w.reserve(GiB) == MYPBR_OK);
+    }
+    {
+        mypbr_dev::Workspace w;
+        HOLDS(w.reserve(GiB + GiB / 2) == MYPBR_OK && fake.left == GiB / 2);
+    }
+    HOLDS(fake.left == 2 * GiB);
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -113,6 +162,10 @@ int main(int argc, char** argv) {
         device_pointers_are_refused();
     else if (name == "new_frame")  // <bytes> <offset in the mapping>
         pages_are_made(std::strtoull(argv[2], nullptr, 10), std::strtoull(argv[3], nullptr, 10));
+    else if (name == "out_of_memory")
+        kept_memory_is_given_back();
+    else if (name == "large")
+        large_workspaces_are_not_kept();
     else
         return 2;
     return 0;
