@@ -717,6 +717,12 @@ int mypbr_env_distribution(const float* rgb, int32_t width, int32_t height, floa
 int mypbr_write_image(const char* path, const double* radiance, int32_t width, int32_t height,
                       const mypbr_display_opts* opts, int on_device);
 
+/* mypbr_gpu_denoise and mypbr_gpu_display keep the device memory they work in
+ * for their next call: one block on each device, as large as the largest call
+ * needed, 1 GiB at most. This gives it back (but not what another thread's
+ * call is using). Calls that run out of device memory do so by themselves. */
+int mypbr_gpu_release_memory(void);
+
 /* The failure path of the device's bounded waits, without a fault: one CTA
  * waits on an mbarrier phase that nothing completes, gives up after about a
  * second, and this returns MYPBR_ERR_DEVICE_TIMEOUT; the context stays

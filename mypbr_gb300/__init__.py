@@ -132,6 +132,7 @@ def lib():
     L.mypbr_ggx_albedo_table.argtypes = [dp]
     L.mypbr_gpu_denoise.argtypes = [vp, vp, vp, vp, ctypes.c_int32, ctypes.c_int32, vp, vp, ctypes.c_int]
     L.mypbr_env_distribution.argtypes = [vp, ctypes.c_int32, ctypes.c_int32, vp, vp, ctypes.c_int]
+    L.mypbr_gpu_release_memory.argtypes = []
     L.mypbr_gpu_test_wait_timeout.argtypes = []
     L.mypbr_gpu_test_device_error.argtypes = [vp, ctypes.c_int32]
     i32p = ctypes.POINTER(ctypes.c_int32)
@@ -533,6 +534,12 @@ def denoise(radiance, albedo, normal, variance, width, height, out, on_device=Fa
         return int(x) if on_device else x.ctypes.data
     check(lib().mypbr_gpu_denoise(addr(radiance), addr(albedo), addr(normal), addr(variance), int(width),
                                   int(height), None, addr(out), int(bool(on_device))))
+
+
+def release_memory():
+    """Gives back the device memory that denoise and display keep between
+    calls (mypbr_gpu_release_memory)."""
+    check(lib().mypbr_gpu_release_memory())
 
 
 def env_distribution(rgb, on_gpu=False):

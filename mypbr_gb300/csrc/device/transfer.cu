@@ -121,8 +121,10 @@ int Workspace::reserve(size_t bytes) {
             k.p = nullptr;
             k.bytes = 0;
             cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&k.p), bytes);
-            if (e != cudaSuccess)
+            if (e != cudaSuccess) {
+                cudaGetLastError();
                 return cuda_fail(e, "workspace");
+            }
             k.bytes = bytes;
         }
         base_ = k.p;
@@ -149,16 +151,29 @@ cudaError_t device_malloc_bytes(void** p, size_t bytes) {
     return e;
 }
 
-void release_workspaces() {
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || device >= kMaxDevices || !g_kept[device].busy.try_lock())
+namespace {
+// unless a call uses it
+void release(Kept& k) {
+    if (!k.busy.try_lock())
         return;
-    Kept& k = g_kept[device];
     if (k.p)
         cudaFree(k.p);
     k.p = nullptr;
     k.bytes = 0;
     k.busy.unlock();
 }
+}  // namespace
+
+void release_workspaces() {
+    int device = 0;
+    if (cudaGetDevice(&device) == cudaSuccess && device < kMaxDevices)
+        release(g_kept[device]);
+}
 
 }  // namespace mypbr_dev
+
+extern "C" int mypbr_gpu_release_memory(void) {
+    for (mypbr_dev::Kept& k : mypbr_dev::g_kept)
+        mypbr_dev::release(k);
+    return MYPBR_OK;
+}

@@ -133,6 +133,19 @@ void kept_memory_is_given_back() {
     HOLDS(mypbr_dev::device_malloc(&p, 3 * MiB) == cudaErrorMemoryAllocation);
 }
 
+// The public call gives back what no call is using.
+void released_on_request() {
+    fake.left = 1000;
+    {
+        mypbr_dev::Workspace w;
+        HOLDS(w.reserve(600) == MYPBR_OK);
+        HOLDS(mypbr_gpu_release_memory() == MYPBR_OK && fake.left == 400);
+    }
+    HOLDS(fake.left == 400);
+    HOLDS(mypbr_gpu_release_memory() == MYPBR_OK && fake.left == 1000);
+    HOLDS(mypbr_gpu_release_memory() == MYPBR_OK && fake.left == 1000);
+}
+
 // More than is ever kept: the kept workspace makes room for it, and it is given back at once.
 void large_workspaces_are_not_kept() {
     constexpr size_t GiB = size_t(1) << 30;
@@ -164,6 +177,8 @@ int main(int argc, char** argv) {
         pages_are_made(std::strtoull(argv[2], nullptr, 10), std::strtoull(argv[3], nullptr, 10));
     else if (name == "out_of_memory")
         kept_memory_is_given_back();
+    else if (name == "release")
+        released_on_request();
     else if (name == "large")
         large_workspaces_are_not_kept();
     else
