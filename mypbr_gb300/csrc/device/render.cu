@@ -2115,6 +2115,8 @@ extern "C" int mypbr_gpu_render_device(mypbr_gpu_scene* G, const mypbr_camera* c
 }
 
 namespace {
+constexpr size_t kFrameMost = size_t(1) << 30;
+
 struct DevBuf {
     double* p = nullptr;
     ~DevBuf() {
@@ -2142,6 +2144,17 @@ extern "C" int mypbr_gpu_render_ex(mypbr_gpu_scene* G, const mypbr_camera* cam, 
     size_t full = size_t(R.P.cam.width) * R.P.cam.height;
     size_t off = size_t(R.P.first_row) * R.P.cam.width, n = R.npix;
     const size_t need = full * size_t(3 + (feats ? 7 : 0) + (channel_variance ? 3 : 0));
+    // the planes stay with the handle for its next render, unless they are very large
+    struct Large {
+        mypbr_gpu_scene* G;
+        ~Large() {
+            if (G->frame_doubles * sizeof(double) > kFrameMost) {
+                cudaFree(G->frame);
+                G->frame = nullptr;
+                G->frame_doubles = 0;
+            }
+        }
+    } large{G};
     if (G->frame_doubles < need) {
         cudaFree(G->frame);
         G->frame = nullptr;
