@@ -773,6 +773,10 @@ int mypbr_guide_configure(mypbr_gpu_scene* scene, float alpha, int32_t depths, f
 int mypbr_guide_schedule(mypbr_gpu_scene* scene, int32_t steps_early, int32_t steps_late, int32_t max_steps,
                          int32_t use_after, float weight_cap);
 
+/* For tests, on the host: the training record slot of every path of a wave of
+ * `pixels` pixels and `passes` passes (out[pixel * passes + pass]), with
+ * `slots` slots; 0xffffffff for a path that records nothing. */
+int mypbr_guide_test_record_slots(int64_t pixels, int64_t passes, int64_t slots, uint32_t* out);
 /* the network's encoded inputs (n x 128, BF16 values as floats) of n
  * vertices given by their 7 scalars in [0, 1] (n x 7). */
 int mypbr_guide_test_encode(const float* scalars, int64_t n, float* out);

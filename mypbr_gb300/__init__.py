@@ -168,6 +168,7 @@ def lib():
     L.mypbr_guide_reset.argtypes = [vp]
     L.mypbr_guide_configure.argtypes = [vp, ctypes.c_float, i32, ctypes.c_float]
     L.mypbr_guide_schedule.argtypes = [vp, i32, i32, i32, i32, ctypes.c_float]
+    L.mypbr_guide_test_record_slots.argtypes = [i64, i64, i64, vp]
     L.mypbr_guide_test_encode.argtypes = [fp, i64, fp]
     L.mypbr_gpu_test_spawn.argtypes = [vp, fp, i64, ip]
     L.mypbr_guide_test_forward.argtypes = [ctypes.c_int, fp, fp, i64, fp]

@@ -1026,6 +1026,20 @@ int mypbr_guide_test_mixture(const float* raw, const float* u, const float* dirs
 
 }  // extern "C"
 
+extern "C" int mypbr_guide_test_record_slots(int64_t pixels, int64_t passes, int64_t slots, uint32_t* out) {
+    using namespace mypbr_dev;
+    if (pixels < 1 || passes < 0 || slots < 0 || pixels * passes >= (int64_t(1) << 31) || slots >= (int64_t(1) << 31) || !out) {
+        set_error_message("mypbr_guide_test_record_slots: bad argument");
+        return MYPBR_ERR_INVALID_ARGUMENT;
+    }
+    const GuideRecordSlots places = guide_record_slots(size_t(pixels), size_t(slots));
+    for (int64_t k = 0; k < pixels * passes; k++) {
+        uint32_t slot;
+        out[k] = places.find(uint32_t(k / passes), uint32_t(k % passes), slot) ? slot : 0xffffffffu;
+    }
+    return MYPBR_OK;
+}
+
 // The failure path of the bounded device waits, exercised without a fault:
 // a wait that nothing ends gives up, the host reads MYPBR_ERR_DEVICE_TIMEOUT,
 // and the context stays usable.

@@ -636,4 +636,19 @@ struct GuideRecords {
     uint32_t capacity;  // slots * depth
 };
 
+// Which paths of a wave record, and in which slot: passes in turn, pixels in
+// order, until the slots are used up. The whole passes among them lie pixel by
+// pixel, as the wave's paths do; what is left over is the first `rest` pixels'
+// next pass.
+struct GuideRecordSlots {
+    uint32_t pixels, passes, rest;
+    MYPBR_HD bool find(uint32_t pixel, uint32_t pass, uint32_t& slot) const {
+        slot = pass < passes ? pixel * passes + pass : pixels * passes + pixel;
+        return pass < passes || (pass == passes && pixel < rest);
+    }
+};
+inline GuideRecordSlots guide_record_slots(size_t pixels, size_t slots) {
+    return {uint32_t(pixels), uint32_t(slots / pixels), uint32_t(slots % pixels)};
+}
+
 }  // namespace mypbr_dev

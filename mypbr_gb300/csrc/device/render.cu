@@ -73,8 +73,8 @@ struct WaveParams {
     float guide_alpha_deep;    // the same at later bounces
     int guide_depths;          // bounces below this sample the mixture
     int record;                // write training records
-    GuideRecords rec;          // the first rec_passes paths of a pixel record their first rec.depth vertices
-    int rec_passes;
+    GuideRecords rec;          // paths that have a slot record their first rec.depth vertices
+    GuideRecordSlots rec_slots;
     GuidePacked* guide_mix;    // per queue entry
     float3 guide_lo, guide_inv;
 };
@@ -626,9 +626,8 @@ __device__ __forceinline__ void shade_body(const WaveParams& P, int depth) {
         int rec_at = -1;  // record written at this vertex (index), listed if the path goes on
         uint32_t rec_slot = 0;
         bool recorded = false;
-        if (GUIDED && P.record && path.band_pass < uint32_t(P.rec_passes)) {
+        if (GUIDED && P.record && P.rec_slots.find(path.band_pixel, path.band_pass, rec_slot)) {
             recorded = true;
-            rec_slot = path.band_pixel * uint32_t(P.rec_passes) + path.band_pass;
             if (depth >= 1 && depth - 1 < P.rec.depth) {
                 // what the previous vertex's record needs: radiance and throughput on arrival here
                 uint32_t r = rec_slot * uint32_t(P.rec.depth) + uint32_t(depth - 1);
@@ -855,8 +854,9 @@ MYPBR_DEV void shadow_end(const WaveParams& P, int2 wave, int depth, uint2 entry
     *to = make_float4(rad.x, rad.y, rad.z, 0.0f);
     if (P.record && ends) {
         const SlotPath sp = slot_path(P, wave, entry.y & ~kShadowEnds);
-        if (sp.band_pass < uint32_t(P.rec_passes))
-            P.rec.fin[sp.band_pixel * uint32_t(P.rec_passes) + sp.band_pass] = make_float4(rad.x, rad.y, rad.z, 0.0f);
+        uint32_t rec_slot;
+        if (P.rec_slots.find(sp.band_pixel, sp.band_pass, rec_slot))
+            P.rec.fin[rec_slot] = make_float4(rad.x, rad.y, rad.z, 0.0f);
     }
 }
 
@@ -1928,7 +1928,7 @@ int prepare(mypbr_gpu_scene* G, const mypbr_camera* cam, const mypbr_render_opts
             return s;
         GuideState& g = G->guide;
         P.rec = g.rec;
-        P.rec_passes = int(g.rec_slots / std::max<size_t>(R.npix, 1));
+        P.rec_slots = guide_record_slots(R.npix, g.rec_slots);
         P.guide_mix = reinterpret_cast<GuidePacked*>(g.packed);
         P.guide_lo = g.box_lo;
         P.guide_inv = g.box_inv;
