@@ -729,6 +729,11 @@ int mypbr_gpu_release_memory(void);
  * usable. For tests. */
 int mypbr_gpu_test_wait_timeout(void);
 
+/* Whether shadow rays test a scene's emitting surfaces one by one before they
+ * walk its tree (1) or look for their closest hit (0), by the number of both.
+ * For tests. */
+int mypbr_gpu_test_few_emitters(int64_t emitters, int64_t leaf_references);
+
 /* Writes the handle's device error word, as a kernel's own check would (1 and
  * 2: a BVH walk past its bounds; 3: a wait past its limit): the next call on
  * the handle reports it. For tests. */

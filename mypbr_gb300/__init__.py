@@ -134,6 +134,7 @@ def lib():
     L.mypbr_env_distribution.argtypes = [vp, ctypes.c_int32, ctypes.c_int32, vp, vp, ctypes.c_int]
     L.mypbr_gpu_release_memory.argtypes = []
     L.mypbr_gpu_test_wait_timeout.argtypes = []
+    L.mypbr_gpu_test_few_emitters.argtypes = [i64, i64]
     L.mypbr_gpu_test_device_error.argtypes = [vp, ctypes.c_int32]
     i32p = ctypes.POINTER(ctypes.c_int32)
     L.mypbr_image_read.argtypes = [ctypes.c_char_p, i32p, i32p, i32p, vp, ctypes.c_int64]

@@ -400,9 +400,10 @@ int create_scene(const mypbr_flat_scene* Fp, mypbr_gpu_scene** out) {
                                                               : -1;
             if (m >= 0 && emits(m)) {
                 glowing.push_back((uint32_t(p.kind) << kKindShift) | uint32_t(p.index));
-                few = glowing.size() <= kFewEmitters;
+                few = glowing.size() <= kMostEmitters;
             }
         }
+        few = few && few_emitters(glowing.size(), refs.size());
         D.emitter_count = few ? int(glowing.size()) : -1;
         if (!few)
             glowing.clear();
@@ -1095,6 +1096,10 @@ int check_device_error(mypbr_gpu_scene* G, cudaStream_t st) {
     return MYPBR_ERR_DEVICE_CHECK;
 }
 }  // namespace mypbr_dev
+
+extern "C" int mypbr_gpu_test_few_emitters(int64_t emitters, int64_t refs) {
+    return emitters >= 0 && refs >= 0 && mypbr_dev::few_emitters(size_t(emitters), size_t(refs));
+}
 
 extern "C" int mypbr_gpu_test_device_error(mypbr_gpu_scene* scene, int32_t code) {
     if (!scene || code < 1 || code > 3) {

@@ -95,3 +95,30 @@ def test_tied_lamps_light_the_room_as_the_oracle_says(lamps):
     sigma = np.sqrt(var.sum(axis=(0, 1)) + ref_var.sum(axis=(0, 1))) / n
     z = (rad.mean(axis=(0, 1)) - ref_rad.mean(axis=(0, 1))) / sigma
     assert np.all(np.abs(z) < 4), z
+
+
+# (lamps, leaf references) measured faster one way or the other
+@pytest.mark.parametrize("lamps,refs,few", [(1, 6, 1), (3, 8, 1), (4, 9, 0), (16, 21, 0), (12, 41, 0), (8, 109, 1), (12, 401, 1),
+                                            (16, 405, 0), (16, 1557, 1), (16, 300016, 1), (17, 300017, 0)])
+def test_which_scenes_look_for_emitters_first(lamps, refs, few):
+    assert mp.lib().mypbr_gpu_test_few_emitters(lamps, refs) == few
+
+
+# 1 to 16 lamps, with enough other surfaces that they are tested one by one, under skies that shine and do not
+@pytest.mark.gpu
+@pytest.mark.parametrize("sky", ["background 0 0 0", "background 0.3 0.4 0.5",
+                                 "background 0 0 0\nsun elevation 40 azimuth 30 intensity 3 angle 3"])
+@pytest.mark.parametrize("lamps", [1, 2, 5, 16])
+def test_every_path_has_the_light_of_its_closest_hit(lamps, sky):
+    rng = np.random.default_rng(lamps)
+    text = ROOM.replace("background 0 0 0\n", "")
+    for k in range(lamps):  # under the ceiling, facing down, up and sideways, some behind others
+        edges = ["0.5 0 0  0 0 0.5", "0 0 0.5  0.5 0 0", "0 0.5 0  0 0 0.5"][k % 3]
+        text += f"quad {-1.6 + 0.8 * (k % 5)} {1.9 - 0.05 * (k % 4)} {-3 + 1.5 * (k // 5)}  {edges}  {['red', 'blue'][k % 2]}\n"
+    for x, y, z, r in zip(*rng.uniform(-1.8, 1.8, (3, 170)), rng.uniform(0.02, 0.1, 170)):
+        text += f"box {x - r} {y - r} {z - r}  {x + r} {y + r} {z + r}  white\n"
+    scene = mp.parse_scene(text + sky + "\n")
+    assert mp.lib().mypbr_gpu_test_few_emitters(lamps, 19 + 6 * 170 + lamps) == 1
+    cam = scene.camera
+    cam.samples_per_pixel = 2
+    _same_light(mp.GpuScene(scene), cam)
