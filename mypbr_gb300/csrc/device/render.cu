@@ -1018,10 +1018,12 @@ __global__ void __maxnreg__(lane_registers(VOX, true)) k_shadow_lanes(WaveParams
                     emission = f3(0.0f);
                 else if (MODE == kShadowAny)
                     emission = unblocked<true>(S, W.h, W.o, W.d, rays[2 * size_t(entry.x) + 1].w);
-                if (MODE == kShadowEmitters && met && blocked_or_tied(W.h) == kTied)
+                // a tied ray brings its light later; ended here like the others, and not
+                // in a branch of its own, it costs them less (box of 12 quads, one
+                // lamp: shadow 1.94 ms against 2.03; 1.90 with ties taken for blocked)
+                shadow_end(P, wave, depth, entry, f3(1.0f), emission);
+                if (MODE == kShadowEmitters && blocked_or_tied(W.h) == kTied)
                     put_tie(rays, ties, k, entry);
-                else
-                    shadow_end(P, wave, depth, entry, f3(1.0f), emission);
             }
             const uint32_t next = take.take(sh_fetch_counter(P, depth), n, run, idle);
             if (idle) {
