@@ -725,6 +725,7 @@ int guide_ensure(mypbr_gpu_scene* G, int hidden, unsigned long long seed) {
     MYPBR_CUDA(cudaMemset(g.grad, 0, P * 4));
     k_guide_adam<<<64, 256>>>(g.master, g.m, g.v, nullptr, 0, g.w, g.wt, g.params, 0.0f, 0.0f, 0.0f);
     MYPBR_CUDA(cudaGetLastError());
+    MYPBR_CUDA(cudaStreamSynchronize(nullptr));  // renders run on streams that do not wait for the legacy one
     g.steps = 0;
     set_scene_box(G);
     return MYPBR_OK;
@@ -761,6 +762,7 @@ int guide_ensure_records(mypbr_gpu_scene* G, size_t mix_slots, size_t slots, int
     g.rec.capacity = uint32_t(n);
     g.rec_slots = slots;
     MYPBR_CUDA(cudaMemset(g.rec.count, 0, 4));
+    MYPBR_CUDA(cudaStreamSynchronize(nullptr));  // as above: the render counts on its own stream
     return MYPBR_OK;
 }
 
