@@ -381,23 +381,24 @@ def run_ours(args):
             peak_src = "measured"
         except Exception:
             peak, peak_src = 6800.0, "fallback"
+        lanes = args.traversal in (0, 1)  # k_extend_lanes, in blocks of 128 by default
         frame_ms = sum(kernel_ms.values())
         shares = {k: v / frame_ms for k, v in kernel_ms.items()}
         line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": total_ms / args.steps, "higher_is_better": True,
                 "scaling": "weak", "vs_baseline": None, "dtype": "fp32", "data": "synthetic",
                 "config": dict(WORKLOAD, spp=args.spp, parallelism=f"samples x{world}", traversal=args.traversal,
-                               block=args.block or 256, wave_paths=args.wave_paths or "default"),
+                               block=args.block or (128 if lanes else 256), wave_paths=args.wave_paths or "default"),
                 "gpu_launches": int(launches),
                 "rays": {"extension_per_path": totals["ext"] / (paths_per_step * args.steps),
                          "shadow_per_path": totals["sh"] / (paths_per_step * args.steps),
                          "mrays_per_s": world * (totals["ext"] + totals["sh"]) / (total_ms * 1e-3) / 1e6},
                 "kernel_time_share": shares,
                 "kernel_time_share_of": "one extra frame after the timed region, each kernel between CUDA events",
-                "roofline": {"bound": "hbm", "kernel": "k_extend", "achieved": achieved, "peak": peak,
+                "roofline": {"bound": "hbm", "kernel": "k_extend_lanes" if lanes else "k_extend", "achieved": achieved, "peak": peak,
                              "unit": "GB/s", "frac": achieved / peak if peak else None,
                              "traffic": EXTEND_DRAM_BYTES_PER_RAY * ext_per_launch,
-                             "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of k_extend on bounce "
+                             "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of k_extend_lanes on bounce "
                                                f"0 of a 4-spp frame ({EXTEND_PROFILE['dram_bytes'] / 1e6:.1f} MB for "
                                                f"{EXTEND_PROFILE['rays']} camera rays, {EXTEND_PROFILE['profile']}, captured at commit "
                                                f"{EXTEND_PROFILE['commit']}), "

@@ -149,9 +149,11 @@ __device__ void apply(const Display& D, double* c) {
 
 // The sRGB curve and 8 bits (color3.h:17-36). pow in FP64 took half the
 // compose kernel (an SM carries out two FP64 operations a clock), so the byte
-// comes from FP32 wherever its error cannot matter: 256 s in FP32 is within
-// 1e-3 of the FP64 value (s <= 1, relative error below 2e-6), and only values
-// closer than 1/128 to a whole number, some 1.6 %, are settled in FP64.
+// comes from FP32 wherever its error cannot matter: powf is __powf here
+// (--use_fast_math), by the programming guide's bounds on __log2f (2 ulps, or
+// 2^-22) and exp2f (2 ulps) within 2e-6 of the power for x above 0.0031, so 256
+// s in FP32 is within 1e-3 of the FP64 value, and only values closer than 1/128
+// to a whole number, some 1.6 %, are settled in FP64.
 __device__ unsigned char to_byte(double x) {
     if (x > 0.0031308 && x < 1.0) {
         const float b = 256.0f * (1.055f * powf(float(x), 1.0f / 2.4f) - 0.055f);

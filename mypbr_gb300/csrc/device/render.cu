@@ -9,7 +9,9 @@
 //           for non-specular vertices next-event estimation writes a shadow
 //           ray; the BSDF sample, Russian roulette, and the surviving path
 //           goes to the next extension queue;
-//   shadow  closest hit of every shadow ray; adds f L w / pdf to its path.
+//   shadow  what every shadow ray brings, by the cheapest question that tells
+//           (kShadowAny, kShadowEmitters, kShadowClosest); adds f L w / pdf to
+//           its path.
 // A path that ends leaves its radiance in its slot; once the wave is done one
 // kernel sums every pixel's slots into the FP64 film.
 // Path records move through the queues (RenderBuffers) and are appended with one
@@ -39,7 +41,8 @@ constexpr uint32_t kFlagSpecular = 1u;
 constexpr uint32_t kFlagSeen = 2u;
 
 // A shadow ray's light goes to an entry of the next extension queue, or, with
-// this bit, to the slot of a path that ended (a wave has at most 2^30 slots).
+// this bit, to the slot of a path that ended (a wave has at most 2^31 slots:
+// 2^30, or one pass of an image with more pixels).
 constexpr uint32_t kShadowEnds = 0x80000000u;
 
 // Shading classes: each has its own queue and kernel, so a warp shades one
@@ -296,7 +299,7 @@ __global__ void k_generate(WaveParams P, int gated) {
     if (!wave_starting(P, gated))
         return;
     const int2 wv = wave_of(P);
-    const uint32_t n = uint32_t(P.cam.width) * uint32_t(P.band_rows) * uint32_t(wv.y);  // at most 2^30
+    const uint32_t n = uint32_t(P.cam.width) * uint32_t(P.band_rows) * uint32_t(wv.y);  // at most 2^31
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += stride) {
         const SlotPath sp = slot_path(P, wv, t);
@@ -448,7 +451,7 @@ MYPBR_DEV uint32_t warp_run(uint32_t n) {
 // the Efficiency of Ray Traversal on GPUs", HPG 2009), on top of the postponed
 // leaves. Same hits as k_extend. The walk is bound by issue and by L1; what is
 // gained is lanes at work per instruction. Against postponed leaves alone
-// (extend ms, one box): guided voxel hall 89.4 -> 45.6 (rays through the slits
+// (extend ms): guided voxel hall 89.4 -> 45.6 (rays through the slits
 // cross the whole terrain, the others a room), plain hall 21.6 -> 19.1, sphere
 // field 32.3 -> 27.5 (binary walk 29.6), 300 k-triangle band 14.6 -> 14.2.
 // Registers: more resident warps against spills (extend ms at 80 / 72 / 64
@@ -812,8 +815,7 @@ __device__ __forceinline__ void shade_body(const WaveParams& P, int depth) {
     }
 }
 
-// The shading kernels. Resident blocks asked for, by class: measured on one
-// box, two blocks of 256 for the lambertian, metal and dielectric kernels
+// The shading kernels. Resident blocks asked for, by class: two blocks of 256 for the lambertian, metal and dielectric kernels
 // (sphere field at 64 spp: shading 22.2 ms against 24.9 with the compiler's
 // choice and 32.9 with one block), the compiler's choice for the principled
 // and generic ones, which spill less gainfully when bound (300 k-triangle
