@@ -720,7 +720,8 @@ int mypbr_write_image(const char* path, const double* radiance, int32_t width, i
 /* mypbr_gpu_denoise and mypbr_gpu_display keep the device memory they work in
  * for their next call: one block on each device, as large as the largest call
  * needed, 1 GiB at most. This gives it back (but not what another thread's
- * call is using). Calls that run out of device memory do so by themselves. */
+ * call is using), and 64 KiB of pinned memory once no scene handle is left.
+ * Calls that run out of device memory do so by themselves. */
 int mypbr_gpu_release_memory(void);
 
 /* The failure path of the device's bounded waits, without a fault: one CTA

@@ -92,6 +92,9 @@ struct mypbr_gpu_scene {
     int64_t material_count = 0;
     uint32_t shade_classes = 1u;  // bit c: paths can meet shading class c (0, a miss, always)
     mypbr_dev::RenderBuffers rb;
+    // The device's error word, in host memory: kernels write it in case of an
+    // error only, and a host that has waited for them reads it where it lies.
+    int* error = nullptr;
     unsigned long long* totals = nullptr;  // a render's ray totals (3)
     double* frame = nullptr;               // the planes of renders with host outputs, kept like the scratch
     size_t frame_doubles = 0;

@@ -316,6 +316,7 @@ int create_scene(const mypbr_flat_scene* Fp, mypbr_gpu_scene** out) {
         for (void* p : G.allocations)
             cudaFree(p);
         G.allocations.clear();
+        give_host_word(G.error);
         if (G.stream)
             cudaStreamDestroy(G.stream);
         G.stream = nullptr;
@@ -454,12 +455,12 @@ int create_scene(const mypbr_flat_scene* Fp, mypbr_gpu_scene** out) {
             D.bvh8_node_count = 0;
         }
     }
-    {
-        std::vector<int> zero(1, 0);
-        const int* err = nullptr;
-        PUT(zero, err);
-        D.error = const_cast<int*>(err);
+    if (!(G.error = take_host_word())) {
+        set_error_message("mypbr_gpu_scene_create: out of pinned host memory");
+        return fail_cleanup(MYPBR_ERR_OUT_OF_MEMORY);
     }
+    if (cudaError_t e = cudaHostGetDevicePointer(&D.error, G.error, 0); e != cudaSuccess)
+        return fail_cleanup(cuda_fail(e, "mypbr_gpu_scene_create"));
 
     // ---- primitives
     std::vector<float4> spheres;
@@ -1080,13 +1081,11 @@ extern "C" int mypbr_gpu_scene_create(const mypbr_flat_scene* scene, mypbr_gpu_s
 namespace mypbr_dev {
 // Reads and clears the sticky device error word after a synchronised call.
 int check_device_error(mypbr_gpu_scene* G, cudaStream_t st) {
-    int e = 0;
-    MYPBR_CUDA(cudaMemcpyAsync(&e, G->dev.error, sizeof e, cudaMemcpyDeviceToHost, st));
     MYPBR_CUDA(cudaStreamSynchronize(st));
+    const int e = *static_cast<volatile int*>(G->error);
     if (e == 0)
         return MYPBR_OK;
-    int zero = 0;
-    MYPBR_CUDA(cudaMemcpy(G->dev.error, &zero, sizeof zero, cudaMemcpyHostToDevice));
+    *G->error = 0;
     if (e == 3) {
         set_error_message("device wait: a tensor-core wait of the guiding network ran past its limit");
         return MYPBR_ERR_DEVICE_TIMEOUT;
@@ -1106,7 +1105,7 @@ extern "C" int mypbr_gpu_test_device_error(mypbr_gpu_scene* scene, int32_t code)
         mypbr_dev::set_error_message("mypbr_gpu_test_device_error: null scene, or a code that is none of the device's");
         return MYPBR_ERR_INVALID_ARGUMENT;
     }
-    MYPBR_CUDA(cudaMemcpy(scene->dev.error, &code, sizeof code, cudaMemcpyHostToDevice));
+    *scene->error = code;
     return MYPBR_OK;
 }
 
@@ -1120,7 +1119,10 @@ extern "C" void mypbr_gpu_scene_destroy(mypbr_gpu_scene* scene) {
     mypbr_dev::release_guide(scene->guide);
     for (void* p : scene->allocations)
         cudaFree(p);
-    if (scene->stream)
+    if (scene->stream) {
+        cudaStreamSynchronize(scene->stream);  // nothing may write the word once it is another handle's
         cudaStreamDestroy(scene->stream);
+    }
+    mypbr_dev::give_host_word(scene->error);
     delete scene;
 }

@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <mutex>
 #include <thread>
+#include <vector>
 
 #include "cuda_check.h"
 
@@ -152,6 +153,55 @@ cudaError_t device_malloc_bytes(void** p, size_t bytes) {
 }
 
 namespace {
+constexpr size_t kWordsInBlock = 16384;
+std::mutex g_words_mutex;
+std::vector<int*> g_word_blocks, g_free_words;  // the second has room for every word there is
+}  // namespace
+
+int* take_host_word() {
+    std::lock_guard<std::mutex> lock(g_words_mutex);
+    if (g_free_words.empty()) {
+        int* block = nullptr;
+        try {
+            g_word_blocks.reserve(g_word_blocks.size() + 1);
+            g_free_words.reserve((g_word_blocks.size() + 1) * kWordsInBlock);
+        } catch (...) {
+            return nullptr;
+        }
+        if (cudaHostAlloc(reinterpret_cast<void**>(&block), kWordsInBlock * sizeof(int),
+                          cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        g_word_blocks.push_back(block);
+        for (size_t k = kWordsInBlock; k-- > 0;)
+            g_free_words.push_back(block + k);
+    }
+    int* const word = g_free_words.back();
+    g_free_words.pop_back();
+    *word = 0;
+    return word;
+}
+
+void give_host_word(int* word) {
+    if (!word)
+        return;
+    std::lock_guard<std::mutex> lock(g_words_mutex);
+    g_free_words.push_back(word);
+}
+
+namespace {
+// once no word is taken
+void release_host_words() {
+    std::lock_guard<std::mutex> lock(g_words_mutex);
+    if (g_free_words.size() != g_word_blocks.size() * kWordsInBlock)
+        return;
+    for (int* block : g_word_blocks)
+        cudaFreeHost(block);
+    g_word_blocks.clear();
+    g_free_words.clear();
+}
+
 // unless a call uses it
 void release(Kept& k) {
     if (!k.busy.try_lock())
@@ -175,5 +225,6 @@ void release_workspaces() {
 extern "C" int mypbr_gpu_release_memory(void) {
     for (mypbr_dev::Kept& k : mypbr_dev::g_kept)
         mypbr_dev::release(k);
+    mypbr_dev::release_host_words();
     return MYPBR_OK;
 }

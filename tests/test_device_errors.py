@@ -32,3 +32,23 @@ def test_device_render_reports_its_own_error(code, status, null, stats):
     mp.check(mp.lib().mypbr_gpu_test_device_error(gpu.handle, code))
     assert render() == status
     assert render() == 0
+
+
+@pytest.mark.gpu
+def test_every_handle_has_an_error_word_of_its_own():
+    scene = mp.load_scene(scene_path("cornell_c1.scene"))
+    cam = scene.camera
+    cam.image_width, cam.samples_per_pixel, cam.max_depth = 16, 1, 2
+    gpus = [mp.GpuScene(scene) for _ in range(3)]
+    mp.check(mp.lib().mypbr_gpu_test_device_error(gpus[1].handle, 2))
+    cam.render(gpus[0])
+    cam.render(gpus[2])
+    gpus[1].close()  # its error goes with it
+    gpus[1] = mp.GpuScene(scene)
+    for gpu in gpus:
+        cam.render(gpu)
+    mp.release_memory()  # handles are alive: their words stay
+    mp.check(mp.lib().mypbr_gpu_test_device_error(gpus[0].handle, 2))
+    with pytest.raises(Exception):
+        cam.render(gpus[0])
+    cam.render(gpus[0])

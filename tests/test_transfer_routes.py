@@ -37,7 +37,7 @@ def test_the_pages_of_a_new_frame_are_made_first(program, nbytes, offset):
     holds(program, "new_frame", nbytes, offset)
 
 
-@pytest.mark.parametrize("scenario", ["out_of_memory", "release", "large"])
+@pytest.mark.parametrize("scenario", ["out_of_memory", "release", "large", "words"])
 def test_kept_memory_makes_room(program, scenario):
     holds(program, scenario)
 

@@ -6,6 +6,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -16,7 +17,8 @@ namespace {
 struct Fake {
     size_t left = SIZE_MAX;      // device memory, bytes
     std::map<void*, size_t> held;
-    int copies = 0;
+    int copies = 0, pinned = 0;  // transfers; pinned blocks
+    size_t pinned_left = SIZE_MAX;
     bool pages_made = false;     // when the transfer started
     const char* host = nullptr;  // the caller's memory and what the driver calls it
     cudaMemoryType kind = cudaMemoryTypeUnregistered;
@@ -38,6 +40,16 @@ cudaError_t cudaMalloc(void** p, size_t n) {
 cudaError_t cudaFree(void* p) {
     fake.left += fake.held[p];
     fake.held.erase(p);
+    return std::free(p), cudaSuccess;
+}
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
+    if (n > fake.pinned_left)
+        return cudaErrorMemoryAllocation;
+    fake.pinned++;
+    return *p = std::malloc(n), cudaSuccess;
+}
+cudaError_t cudaFreeHost(void* p) {
+    fake.pinned--;
     return std::free(p), cudaSuccess;
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
@@ -146,6 +158,33 @@ void released_on_request() {
     HOLDS(mypbr_gpu_release_memory() == MYPBR_OK && fake.left == 1000);
 }
 
+// Words of several blocks: each its own, zero when taken, the blocks freed on request once none is taken.
+void host_words() {
+    std::vector<int*> taken;
+    std::set<int*> different;
+    for (int k = 0; k < 40000; k++) {
+        taken.push_back(mypbr_dev::take_host_word());
+        HOLDS(taken.back() && *taken.back() == 0);
+        *taken.back() = k + 1;
+        different.insert(taken.back());
+    }
+    HOLDS(different.size() == taken.size() && fake.pinned == 3);
+    fake.pinned_left = 0;
+    while (int* word = mypbr_dev::take_host_word())
+        taken.push_back(word);
+    HOLDS(taken.size() == 3 * 16384);
+    mypbr_dev::give_host_word(taken.back());
+    taken.pop_back();
+    HOLDS(mypbr_gpu_release_memory() == MYPBR_OK && fake.pinned == 3);
+    for (int* word : taken)
+        mypbr_dev::give_host_word(word);
+    mypbr_dev::give_host_word(nullptr);
+    HOLDS(mypbr_gpu_release_memory() == MYPBR_OK && fake.pinned == 0);
+    HOLDS(!mypbr_dev::take_host_word());
+    fake.pinned_left = SIZE_MAX;
+    HOLDS(mypbr_dev::take_host_word() && fake.pinned == 1);
+}
+
 // More than is ever kept: the kept workspace makes room for it, and it is given back at once.
 void large_workspaces_are_not_kept() {
     constexpr size_t GiB = size_t(1) << 30;
@@ -179,6 +218,8 @@ int main(int argc, char** argv) {
         kept_memory_is_given_back();
     else if (name == "release")
         released_on_request();
+    else if (name == "words")
+        host_words();
     else if (name == "large")
         large_workspaces_are_not_kept();
     else
