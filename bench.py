@@ -410,7 +410,7 @@ def run_ours(args):
                              "issue": {"issue_active_frac": EXTEND_PROFILE["issue_active_frac"],
                                        "threads_per_instruction": EXTEND_PROFILE["threads_per_instruction"],
                                        "source": "ncu smsp__issue_active and smsp__thread_inst_executed_per_"
-                                                 "inst_executed of k_extend, bounces 0 and 1 of a 4-spp frame ("
+                                                 "inst_executed of k_extend_lanes, bounces 0 and 1 of a 4-spp frame ("
                                                  + EXTEND_PROFILE["profile"] + ", captured at commit "
                                                  + EXTEND_PROFILE["commit"] + ")"}},
                 "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": int(h2d),
