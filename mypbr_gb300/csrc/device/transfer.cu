@@ -154,17 +154,25 @@ cudaError_t device_malloc_bytes(void** p, size_t bytes) {
 
 namespace {
 constexpr size_t kWordsInBlock = 16384;
-std::mutex g_words_mutex;
-std::vector<int*> g_word_blocks, g_free_words;  // the second has room for every word there is
+struct HostWords {
+    std::mutex busy;
+    std::vector<int*> blocks, left;  // `left` has room for every word there is
+};
+// Never destroyed: a program's last handles may go after this library's objects.
+HostWords& host_words() {
+    static HostWords* const words = new HostWords;
+    return *words;
+}
 }  // namespace
 
 int* take_host_word() {
-    std::lock_guard<std::mutex> lock(g_words_mutex);
-    if (g_free_words.empty()) {
+    HostWords& w = host_words();
+    std::lock_guard<std::mutex> lock(w.busy);
+    if (w.left.empty()) {
         int* block = nullptr;
         try {
-            g_word_blocks.reserve(g_word_blocks.size() + 1);
-            g_free_words.reserve((g_word_blocks.size() + 1) * kWordsInBlock);
+            w.blocks.reserve(w.blocks.size() + 1);
+            w.left.reserve((w.blocks.size() + 1) * kWordsInBlock);
         } catch (...) {
             return nullptr;
         }
@@ -173,12 +181,12 @@ int* take_host_word() {
             cudaGetLastError();
             return nullptr;
         }
-        g_word_blocks.push_back(block);
+        w.blocks.push_back(block);
         for (size_t k = kWordsInBlock; k-- > 0;)
-            g_free_words.push_back(block + k);
+            w.left.push_back(block + k);
     }
-    int* const word = g_free_words.back();
-    g_free_words.pop_back();
+    int* const word = w.left.back();
+    w.left.pop_back();
     *word = 0;
     return word;
 }
@@ -186,20 +194,22 @@ int* take_host_word() {
 void give_host_word(int* word) {
     if (!word)
         return;
-    std::lock_guard<std::mutex> lock(g_words_mutex);
-    g_free_words.push_back(word);
+    HostWords& w = host_words();
+    std::lock_guard<std::mutex> lock(w.busy);
+    w.left.push_back(word);
 }
 
 namespace {
 // once no word is taken
 void release_host_words() {
-    std::lock_guard<std::mutex> lock(g_words_mutex);
-    if (g_free_words.size() != g_word_blocks.size() * kWordsInBlock)
+    HostWords& w = host_words();
+    std::lock_guard<std::mutex> lock(w.busy);
+    if (w.left.size() != w.blocks.size() * kWordsInBlock)
         return;
-    for (int* block : g_word_blocks)
+    for (int* block : w.blocks)
         cudaFreeHost(block);
-    g_word_blocks.clear();
-    g_free_words.clear();
+    w.blocks.clear();
+    w.left.clear();
 }
 
 // unless a call uses it
